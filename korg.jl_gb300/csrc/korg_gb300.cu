@@ -340,6 +340,7 @@ bool tile_geom(bool mixed, int Lp, int G, TileCfg c, TileGeom* g) {
     g->split = c.split ? 1 : 0;
     g->G = G;
     g->smem = 2 * region + size_t(g->threads) * (mixed ? sizeof(LineStage32) : sizeof(LineStage));
+    if (!mixed) g->smem += sizeof(double) * SL * (FAR_P + 1);  // Chebyshev coefficients of the far lines
     return g->smem <= 227 * 1024;
 }
 

@@ -1,0 +1,57 @@
+"""Far lines of the line tiles (evaluated at 16 Chebyshev nodes per tile and interpolated) against the
+FP64 oracle, at the sizes where the split can go wrong: tiles cut short by the grid's end, every
+layers-per-group template, other tile widths and a non-uniform grid with a
+gap."""
+import os
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+NT = os.cpu_count() or 1
+
+
+def _inputs(L, lo, hi, n, teff=5000.0):
+    from korg_gb300 import synthetic
+    w = synthetic.Workload("far", teff, 4.4, 0.0, L, (lo, hi), synthetic.synthetic_linelist(n, lo, hi, seed=n))
+    return synthetic.prepare(w)
+
+
+def _opacity(gpu_lib, oracle_lib, inp, wls, precision, tile=None):
+    from korg_gb300 import Wavelengths, line_absorption_
+    from korg_gb300.api import ContinuumInterpolant, _prec
+    from korg_gb300.data import default_partition_funcs
+    ctx = gpu_lib.Context(0)
+    if tile:
+        ctx.check(ctx.lib.korg_set_tile_config(ctx.h, len(inp.T), _prec(precision), *tile))
+    a0 = np.stack([np.interp(wls, inp.cntm_knots, v) for v in inp.cntm_vals], axis=1)
+    got, ref = a0.copy(), a0.copy()
+    n = line_absorption_(got, inp.linelist, Wavelengths.from_array(wls), inp.T, inp.ne, inp.number_densities,
+                         default_partition_funcs(), inp.xi, ContinuumInterpolant(inp.cntm_knots, inp.cntm_vals),
+                         precision=precision, ctx=ctx)
+    ctx.close()
+    n_ref = oracle_lib.line_absorption(ref, inp.linelist, wls, inp.T, inp.ne, inp.n_eff_vdW, inp.xi, inp.n_div_U,
+                                       inp.cntm_knots, inp.cntm_vals, cutoff=3e-4, nthreads=NT)
+    assert n == n_ref
+    return got, ref
+
+
+@pytest.mark.parametrize("L,tile", [(56, None), (56, (64, 0, 1)), (56, (96, 0, 0)), (80, None), (130, None)])
+@pytest.mark.parametrize("extra", [0, 1, 63, 64, 65, 127])
+def test_fp64_far_lines_match_oracle(gpu_lib, oracle_lib, L, tile, extra):
+    """The sum of a few hundred positive terms and the 16-node series both round at 1e-15 each: 1e-12."""
+    if (L != 56 or tile) and extra not in (1, 64):
+        pytest.skip("the remainders are covered at 56 layers")
+    inp = _inputs(L, 5000, 5010, 400)
+    wls = inp.wls.all_wls[:512 + extra] if extra else inp.wls.all_wls[:512]
+    got, ref = _opacity(gpu_lib, oracle_lib, inp, wls, "fp64", tile)
+    np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
+
+
+def test_fp64_far_lines_on_an_uneven_grid(gpu_lib, oracle_lib):
+    """Steps that grow along the grid, repeated wavelengths and a 20 A gap inside a tile."""
+    inp = _inputs(56, 5000, 5040, 800)
+    d = np.concatenate([np.full(300, 0.004), np.linspace(0.002, 0.03, 300), [0.0, 0.0, 20.0], np.full(300, 0.01)])
+    wls = (5002.0 + np.cumsum(d)) * 1e-8
+    got, ref = _opacity(gpu_lib, oracle_lib, inp, wls, "fp64")
+    np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
