@@ -283,6 +283,7 @@ TileArgs make_tile_args(const LineScratch& sc, double* alpha, const double* wls,
     ta.tier_ci = sc.tier_ci;
     ta.tier_start = sc.tier_meta;                 // [start: NTIER+1][unsorted][block counts]
     ta.unsorted = sc.tier_meta + NTIER + 1;
+    ta.far32 = 1;
     return ta;
 }
 
@@ -347,11 +348,20 @@ bool tile_geom(bool mixed, int Lp, int G, TileCfg c, TileGeom* g) {
 // Default tile shape: 128 wavelengths x one layer group (mixed: 64-line batches, FP64: 16).
 TileCfg default_tile(bool) { return TileCfg{TILE_TW, 0, 1}; }
 
+// far_lines: whether some tile can hold FAR_MIN_CAND32 candidates (mixed: line_far_kernel runs first).
 template <bool MIXED, int KMAX, int MAXT, int MINB>
-int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* q, cudaStream_t s) {
+int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* q, bool far_lines, cudaStream_t s) {
     ta.stage = g.stage;
     ta.region = g.region;
     ta.split = g.split;
+    if (MIXED && far_lines) {
+        if (q)
+            line_far_batch_kernel<KMAX><<<dim3(unsigned(q->nitems / q->groups), unsigned(q->groups)), FAR_THREADS, 0, s>>>(
+                q->spec, q->nspec, g.tw);
+        else
+            line_far_kernel<KMAX><<<dim3(unsigned((ta.nwl + g.tw - 1) / g.tw), unsigned(g.G)), FAR_THREADS, 0, s>>>(ta, g.tw);
+        KCUDA(cudaGetLastError());
+    }
     if (q) {
         auto kern = line_tile_queue_kernel<MIXED, KMAX, MAXT, MINB>;
         KCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
@@ -370,23 +380,26 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
 }
 
 template <bool MIXED>
-int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g, const TileQueue* q,
+int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g, const TileQueue* q, bool far_lines,
                   cudaStream_t s) {
     if constexpr (MIXED) {  // at most 256 threads (one layer group per CTA)
-        if (kmax == 14) return launch_tile<true, 14, 256, 3>(ctx, ta, g, q, s);
-        if (kmax == 16) return launch_tile<true, 16, 256, 2>(ctx, ta, g, q, s);
-        return launch_tile<true, 32, 256, 2>(ctx, ta, g, q, s);
+        if (kmax == 14) return launch_tile<true, 14, 256, 3>(ctx, ta, g, q, far_lines, s);
+        if (kmax == 16) return launch_tile<true, 16, 256, 2>(ctx, ta, g, q, far_lines, s);
+        return launch_tile<true, 32, 256, 2>(ctx, ta, g, q, far_lines, s);
     } else {
-        if (kmax == 14 && g.threads <= 256) return launch_tile<false, 14, 256, 2>(ctx, ta, g, q, s);
-        if (kmax == 14) return launch_tile<false, 14, 512, 1>(ctx, ta, g, q, s);
-        if (kmax == 16) return launch_tile<false, 16, 512, 1>(ctx, ta, g, q, s);
-        return launch_tile<false, 32, 512, 1>(ctx, ta, g, q, s);
+        if (kmax == 14 && g.threads <= 256) return launch_tile<false, 14, 256, 2>(ctx, ta, g, q, far_lines, s);
+        if (kmax == 14) return launch_tile<false, 14, 512, 1>(ctx, ta, g, q, far_lines, s);
+        if (kmax == 16) return launch_tile<false, 16, 512, 1>(ctx, ta, g, q, far_lines, s);
+        return launch_tile<false, 32, 512, 1>(ctx, ta, g, q, far_lines, s);
     }
 }
 
+// nlines: lines of the (largest) list.
 int run_tiles(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g, const TileQueue* q, bool mixed,
-              cudaStream_t s) {
-    return mixed ? dispatch_tile<true>(ctx, ta, kmax, g, q, s) : dispatch_tile<false>(ctx, ta, kmax, g, q, s);
+              int64_t nlines, cudaStream_t s) {
+    const bool far_lines = nlines >= FAR_MIN_CAND32 && (q || ta.far32);
+    return mixed ? dispatch_tile<true>(ctx, ta, kmax, g, q, far_lines, s)
+                 : dispatch_tile<false>(ctx, ta, kmax, g, q, far_lines, s);
 }
 
 // The tile shape for (L, precision): the autotuned one when there is one, else the default.
@@ -419,7 +432,7 @@ int autotune_tiles(korg_ctx* ctx, const TileArgs& ta0, int kmax, bool mixed, cud
             float t = 1e30f;
             for (int rep = 0; rep < 3; rep++) {
                 KCUDA(cudaEventRecord(ctx->ev[6], s));
-                KCHECK(run_tiles(ctx, ta, kmax, g, nullptr, mixed, s));
+                KCHECK(run_tiles(ctx, ta, kmax, g, nullptr, mixed, ta.n, s));
                 KCUDA(cudaEventRecord(ctx->ev[7], s));
                 KCUDA(cudaEventSynchronize(ctx->ev[7]));
                 float ms = 0;
@@ -438,7 +451,7 @@ bool worth_tuning(int64_t nwl, int64_t nlines) { return nwl >= 100000 && nlines 
 
 int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, const LinesDev& ln,
                         const LayersDev& lay, const CntmDev& cn, double cutoff, bool mixed,
-                        cudaStream_t s) {
+                        cudaStream_t s, bool far32 = true) {
     if (ln.n == 0) return KORG_OK;  // src/line_absorption.jl:35-37
     const int L = lay.L;
     int kmax = 0;
@@ -451,12 +464,13 @@ int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t
     line_scratch(static_cast<unsigned char*>(ctx->lines_scratch.p), ln.n, L, Lp, G, mixed, &sc);
     KCHECK(prep_lines(ctx, sc, wls, nwl, ln, lay, cn, cutoff, mixed, kmax, G, s));
     record(ctx, 2, s);
-    const TileArgs ta = make_tile_args(sc, alpha, wls, nwl, ln, L, Lp, G);
+    TileArgs ta = make_tile_args(sc, alpha, wls, nwl, ln, L, Lp, G);
+    ta.far32 = far32;
     if (ctx->autotune && !ctx->capturing && worth_tuning(nwl, ln.n)) KCHECK(autotune_tiles(ctx, ta, kmax, mixed, s));
     TileGeom g;
     if (!tile_geom(mixed, Lp, G, tile_cfg(ctx, L, mixed), &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
     ctx->stats_pending = true;
-    return run_tiles(ctx, ta, kmax, g, nullptr, mixed, s);
+    return run_tiles(ctx, ta, kmax, g, nullptr, mixed, ln.n, s);
 }
 
 // ------------------------------------------------------------------ hydrogen lines
@@ -692,7 +706,9 @@ int enqueue_batch(korg_ctx* ctx, const BatchPlan& p, int nspec, const korg_batch
         record(ctx, 2, s);
         const int groups = p.geom.split ? p.G : 1;
         const TileQueue q{d_targs + s0, s1 - s0, groups, int64_t(s1 - s0) * ntiles * groups, d_ctr + c};
-        KCHECK(run_tiles(ctx, TileArgs{}, p.kmax, p.geom, &q, mixed, s));
+        int64_t nlines = 0;
+        for (int i = s0; i < s1; i++) nlines = std::max(nlines, it[i].lines.n);
+        KCHECK(run_tiles(ctx, TileArgs{}, p.kmax, p.geom, &q, mixed, nlines, s));
         record(ctx, 5, s);
         for (int i = s0; i < s1; i++) {
             const korg_synth_inputs& in = it[i].in;
@@ -832,7 +848,9 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         KCHECK(run_line_absorption(ctx, aref, ref_wl_dev, 1, ln5, lay, cref, in->cutoff_threshold, false, s));
         if (in->hydrogen_lines)
             KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s));
-        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s));
+        // every line at every wavelength: the mixed line adjoint rounds the opacity cotangent to FP32,
+        // and single lines' log gf gradients would move by 3e-8 with the far lines' rounding
+        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s, false));
     }
     // the metal-line prologue: the batch's for this spectrum, else the context's line scratch (read
     // after step 1, which may have grown it)
@@ -2729,6 +2747,12 @@ int noalloc_tiles(const TileArgs& ta, int G, int kmax, bool mixed, cudaStream_t 
         return cudaGetLastError() == cudaSuccess ? KORG_OK : KORG_ECUDA;
     };
     if (mixed) {
+        if (ta.n >= FAR_MIN_CAND32) {
+            if (kmax == 14) line_far_kernel<14><<<grid, FAR_THREADS, 0, s>>>(t, g.tw);
+            else if (kmax == 16) line_far_kernel<16><<<grid, FAR_THREADS, 0, s>>>(t, g.tw);
+            else line_far_kernel<32><<<grid, FAR_THREADS, 0, s>>>(t, g.tw);
+            if (cudaGetLastError() != cudaSuccess) return KORG_ECUDA;
+        }
         if (kmax == 14) return go(line_tile_kernel<true, 14, 256, 3>);
         if (kmax == 16) return go(line_tile_kernel<true, 16, 256, 2>);
         return go(line_tile_kernel<true, 32, 256, 2>);
@@ -2821,5 +2845,6 @@ extern "C" KORG_API int korg_line_absorption_noalloc(double* alpha, const double
     ta.tier_ci = tl.ci;
     ta.tier_start = tl.start;
     ta.unsorted = tl.unsorted;
+    ta.far32 = 1;
     return noalloc_tiles(ta, G, kmax, mixed, s);
 }

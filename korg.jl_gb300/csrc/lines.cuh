@@ -80,11 +80,19 @@ struct PrepOut {
     int32_t Lp, K, G;
     unsigned long long* evals;   // running totals: evaluations, lines in window
     unsigned long long* nlines;
-    float4* params_w;        // [n][Lp] mixed, or null: wing cubic {A1, A2, A3, 0} in t' = cref / dl^2
-                             //   (cref = 2 sigma^2 of layer 0), valid beyond the layer's cubic boundary
+    float4* params_w;        // [n][G][wing_quads(K)] mixed, or null: wing cubics A1 t' + A2 t'^2 + A3 t'^3 in
+                             //   t' = cref / dl^2 (cref = 2 sigma^2 of layer 0), valid beyond the layer's cubic
+                             //   boundary; per group three planes A1, A2, A3 of K floats (K padded to 4)
     float* xcub;             // [n][G] mixed, or null: |wl - wl0| beyond which every layer of group g
                              //   is given by its wing cubic to FP32 rounding
 };
+
+// 16-byte pieces of one (line, layer group)'s wing cubics: three planes of K floats, K padded to 4.
+// Adjacent layers lie next to each other, so packed FP32 arithmetic (two FMAs an instruction) takes
+// its operands straight from 16-byte loads: 12 loads and 21 FMAs a line and warp instead of 14 and 42
+// (14 layers).  The tile kernel is bound by issue and the shared-memory pipe: full optical synthesis
+// 37.5 -> 34.3 ms, bit for bit the same.
+__host__ __device__ constexpr int wing_quads(int K) { return 3 * ((K + 3) / 4); }
 
 // Per-line quantities shared by every layer (line_absorption.jl:83,101,105,219).
 struct LineConst {
@@ -329,7 +337,8 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) line_prep_mixed_kernel(LinesD
         float dmax = -1.f, lmax = -1.f;
         int dl = 0, ll = 0;
         float4* dst = reinterpret_cast<float4*>(out.params) + i * Lp;
-        float4* dstw = out.params_w ? out.params_w + i * Lp : nullptr;
+        const int qb = wing_quads(out.K);
+        float* dstw = out.params_w ? reinterpret_cast<float*>(out.params_w + i * out.G * qb) : nullptr;
         float cref = 0.f;
         for (int l0 = 0; l0 < Lp; l0 += 32) {
             const int l = l0 + lane;
@@ -402,7 +411,11 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) line_prep_mixed_kernel(LinesD
                             pw.z = k0 * q * fmaf(fmaf(15.f, q2, -10.f), q2, 1.f) * kap * kap * kap;
                         }
                     }
-                    dstw[l] = pw;
+                    const int gl = l / out.K, plane = 4 * (qb / 3);
+                    float* w = dstw + gl * 4 * qb + (l - gl * out.K);
+                    w[0] = pw.x;
+                    w[plane] = pw.y;
+                    w[2 * plane] = pw.z;
                 }
             }
         }
@@ -544,6 +557,7 @@ struct TileArgs {
     const uint32_t* amask;
     const int32_t *lb, *ub;
     const int32_t *tier_idx, *tier_ci, *tier_start, *unsorted;
+    int32_t far32;            // mixed: line_far_kernel takes the far lines of tiles with FAR_MIN_CAND32 candidates
     const float4* params_w;   // mixed, or null: wing cubics (see PrepOut)
     const float* xcub;        // mixed, or null: cubic boundaries (see PrepOut)
 };
@@ -565,6 +579,21 @@ __device__ __forceinline__ int64_t upper_bound_i32(const int32_t* a, int64_t lo,
     return lo;
 }
 
+// Candidate run of width tier `t` for the tile [j0, jlast].
+__device__ __forceinline__ void tier_run(const TileArgs& a, int t, int64_t j0, int64_t jlast, int64_t (&run)[2]) {
+    const int64_t t0 = a.tier_start[t], t1 = a.tier_start[t + 1];
+    if (*a.unsorted) {
+        run[0] = t0;
+        run[1] = t1;
+    } else {
+        const int32_t w = c_tier_w[t] + 1;
+        const int32_t lo = int32_t(max(int64_t(j0) - w, int64_t(INT32_MIN / 2)));
+        const int32_t hi = int32_t(min(int64_t(jlast) + w, int64_t(INT32_MAX / 2)));
+        run[0] = lower_bound_i32(a.tier_ci, t0, t1, lo);
+        run[1] = upper_bound_i32(a.tier_ci, t0, t1, hi);
+    }
+}
+
 // A candidate line of the current chunk, as an FP64 tile sees it.
 struct LineStage {
     double wl;        // centre
@@ -580,6 +609,27 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src)
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+
+// Two FP32 values in one 64-bit register, and the packed FMA on them (each half rounds as fmaf does).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float part2(f32x2 v, int h) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    return h ? hi : lo;
+}
+__device__ __forceinline__ void set2(f32x2& v, int h, float x) {
+    v = h ? pack2(part2(v, 0), x) : pack2(x, part2(v, 1));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
 
 // Far-Lorentz branch of voigt_hjerting (line_absorption.jl:305-308) with r^2 = x^2/gamma^2.
 __device__ __forceinline__ float far_lorentz32(float4 p, float x2) {
@@ -602,14 +652,22 @@ __device__ __forceinline__ double far_lorentz64(const P64& p, double x2) {
 // FAR_P - 1.  The profiles' singularities are at the line centre (asymptotic and far-Lorentz series)
 // or beyond it (far-Lorentz: at wl0 +- i gamma), so with z = 2 kappa + 1 the series converges like
 // (z + sqrt(z^2 - 1))^-FAR_P.  Measured on 1/x^2 at the closest distance, 16 nodes, largest relative
-// error over the tile: kappa 2.5: at the rounding of FP64 (4e-15 in a plain FP64 evaluation of the
-// series; kappa 2: 8e-15).  16 nodes and not fewer: fewer would push kappa, and with it the lines
-// evaluated at every wavelength, up.  Measured: the 11 x 51 x 10,001 CO cross-section table 168.6 ->
-// 86.4 ms, line_absorption! of 2,000 lines on 10,001 points x 56 layers 6.3 -> 4.8 ms, same error
-// against 64 bits (FP64 pipe bound: the nodes do an eighth of the far evaluations).
+// error over the tile: kappa 0.75: 7e-10 (mixed; below the 6e-8 rounding of each FP32 evaluation),
+// kappa 2.5: at the rounding of FP64 (4e-15 in a plain FP64 evaluation of the series; kappa 2: 8e-15).
+// 16 nodes and not fewer: fewer would push kappa, and with it the lines evaluated at every wavelength, up.
+// Measured, FP64 (the nodes do an eighth of the far evaluations of a kernel bound by the FP64 pipe): the
+// 11 x 51 x 10,001 CO cross-section table 168.6 -> 86.4 ms, line_absorption! of 2,000 lines on 10,001
+// points x 56 layers 6.3 -> 4.8 ms, same error against 64 bits.
 constexpr int FAR_P = 16;
+constexpr float FAR_KAPPA32 = 0.75f;
 constexpr double FAR_KAPPA64 = 2.5;
 constexpr int FAR_MIN_POINTS = 64;  // shorter tiles: 16 nodes would save less than 3 of 4 evaluations
+// Mixed tiles with fewer candidates evaluate every line at every wavelength: there a few lines carry
+// the far opacity, and the FP32 rounding of their evaluations (1e-7 each, averaged differently at the
+// nodes) would move the flux by up to 6e-9 of itself (7e-11 and less above the limit), for a gain of
+// a tenth (full optical synthesis, 4,000 candidates a tile) or none (sparser lists).
+constexpr int64_t FAR_MIN_CAND32 = 8192;
+
 // cos(pi i / 32), i = 0..16; the other angles by symmetry
 __device__ __constant__ double c_cos32[17] = {
     1.0, 0.9951847266721969, 0.9807852804032304, 0.9569403357322088,
@@ -665,19 +723,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
 
     // candidate runs of the width tiers (threads 0..NTIER-1 search one tier each)
     __shared__ int64_t s_tier[NTIER][2];
-    if (tid < NTIER) {
-        const int64_t t0 = a.tier_start[tid], t1 = a.tier_start[tid + 1];
-        if (*a.unsorted) {
-            s_tier[tid][0] = t0;
-            s_tier[tid][1] = t1;
-        } else {
-            const int32_t w = c_tier_w[tid] + 1;
-            const int32_t lo = int32_t(max(int64_t(j0) - w, int64_t(INT32_MIN / 2)));
-            const int32_t hi = int32_t(min(int64_t(jlast) + w, int64_t(INT32_MAX / 2)));
-            s_tier[tid][0] = lower_bound_i32(a.tier_ci, t0, t1, lo);
-            s_tier[tid][1] = upper_bound_i32(a.tier_ci, t0, t1, hi);
-        }
-    }
+    if (tid < NTIER) tier_run(a, tid, j0, jlast, s_tier[tid]);
     __syncthreads();
 
     double acc[K];
@@ -882,6 +928,182 @@ struct LineStage32 {
 };
 static_assert(sizeof(LineStage32) == 32, "LineStage32 is two 16-byte loads");
 
+// Whether the mixed tile's far lines go to line_far_kernel (see FAR_MIN_CAND32).
+__device__ __forceinline__ bool far_tile32(const TileArgs& a, const int64_t (&run)[NTIER][2], int64_t npoints) {
+    if (!a.far32 || npoints < FAR_MIN_POINTS) return false;
+    int64_t n = 0;
+    for (int t = 0; t < NTIER; t++) n += max(run[t][1] - run[t][0], int64_t(0));
+    return n >= FAR_MIN_CAND32;
+}
+// Whether line i covers the tile [j0, jlast] from at least kspan away, in its cubic regime for group g.
+__device__ __forceinline__ bool far_line32(const TileArgs& a, int64_t i, int g, int32_t lb, int32_t ub, int64_t j0,
+                                           int64_t jlast, double wl_ref, float span32, float kspan) {
+    if (lb > j0 || ub < jlast) return false;
+    const float dh = float(a.wl[i] - wl_ref);
+    const float fdist = dh < 0.f ? -dh : (dh > span32 ? dh - span32 : 0.f);
+    return fdist >= kspan && fdist > a.xcub[i * a.G + g];
+}
+
+// Far lines of a mixed tile of tw wavelengths x the K layers of group g, added to alpha.  Lanes of a
+// half-warp hold layers (K = 32: of a warp), each with its wing cubic in registers, and walk the
+// FAR_P nodes: a line's constants are one coalesced load, fetched a step ahead, and the nodes' t' are
+// shared through shared memory, so there is neither staging nor a block barrier per chunk (the tile
+// kernel spends most of its time on both when most of its lines are far).  Packed FP32 sums over at
+// most FAR_FLUSH lines, then FP64 sums in shared memory; line order within each half-warp is the
+// list's, so results are reproducible.  Whole passes: 80 layers, 286,000 lines, 200,001 points 27.9 ->
+// 22.2 ms; 8 infrared spectra of 5,000-50,000 lines on 100,001 points 64.8 -> 48.1 ms.
+constexpr int FAR_THREADS = 128, FAR_WARPS = FAR_THREADS / 32, FAR_FLUSH = 64;
+template <int K>
+struct FarShared {
+    double node[FAR_WARPS][FAR_P][K];       // FP64 node sums of each warp
+    double v[K][FAR_P], cf[K][FAR_P + 1];
+    float tp[FAR_WARPS][2][FAR_P];          // t' of the line(s) at hand
+    int64_t tier[NTIER][2];
+    double stage[32][K + 1];                // alpha of 32 wavelengths
+};
+template <int K>
+__device__ __forceinline__ void line_far_body(const TileArgs& a, int64_t tile, int tw, int g, FarShared<K>& sh) {
+    constexpr int LPW = K <= 16 ? 2 : 1;    // lines a warp works on at a time
+    constexpr int HL = 32 / LPW;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = lane / HL, k = lane % HL;
+    const int64_t j0 = tile * tw, jlast = min(j0 + tw, a.nwl) - 1;
+    const double wl_ref = a.wls[j0], span = a.wls[jlast] - wl_ref;
+    const float span32 = float(span);
+    if (tid < NTIER) tier_run(a, tid, j0, jlast, sh.tier[tid]);
+    __syncthreads();
+    if (!far_tile32(a, sh.tier, jlast - j0 + 1)) return;  // uniform
+    const float kspan = FAR_KAPPA32 * span32;
+    for (int e = tid; e < FAR_WARPS * FAR_P * K; e += FAR_THREADS) (&sh.node[0][0][0])[e] = 0.0;
+    __syncthreads();
+    const double hw = 0.5 * span, dn = hw + hw * cos_pi32(2 * (lane % FAR_P) + 1);
+    const float nh = float(dn), nlo = float(dn - double(nh));
+    constexpr int plane = 4 * (wing_quads(K) / 3);
+    const float* wing = reinterpret_cast<const float*>(a.params_w) + size_t(g) * 3 * plane + min(k, K - 1);
+    f32x2 part[FAR_P / 2];
+#pragma unroll
+    for (int n = 0; n < FAR_P / 2; n++) part[n] = 0ull;
+    int pending = 0;
+    auto flush = [&]() {
+#pragma unroll
+        for (int n = 0; n < FAR_P; n++) {
+            float v = part2(part[n / 2], n % 2);
+            double d = double(v);
+            if (LPW == 2) d += double(__shfl_xor_sync(0xffffffffu, v, 16));
+            if (half == 0 && k < K) sh.node[warp][n][k] += d;
+        }
+#pragma unroll
+        for (int n = 0; n < FAR_P / 2; n++) part[n] = 0ull;
+        pending = 0;
+    };
+    for (int tier = 0; tier < NTIER; tier++)
+        for (int64_t base = sh.tier[tier][0] + 32 * warp; base < sh.tier[tier][1]; base += FAR_THREADS) {
+            int32_t li = 0;
+            bool far = false;
+            float dhi = 0.f, dlo = 0.f, cref = 0.f;
+            if (base + lane < sh.tier[tier][1]) {
+                li = a.tier_idx[base + lane];
+                far = far_line32(a, li, g, a.lb[li], a.ub[li], j0, jlast, wl_ref, span32, kspan);
+                if (far) {
+                    const double d = a.wl[li] - wl_ref;
+                    dhi = float(d);
+                    dlo = float(d - double(dhi));
+                    cref = reinterpret_cast<const float4*>(a.params)[int64_t(li) * a.Lp].x;
+                }
+            }
+            unsigned m = __ballot_sync(0xffffffffu, far);
+            // the next line of this half-warp (32: none), and its constants
+            auto next = [&]() {
+                int src = 32;
+#pragma unroll
+                for (int h = 0; h < LPW; h++) {
+                    const int b = m ? __ffs(m) - 1 : 32;
+                    if (h == half) src = b;
+                    m &= m - 1;
+                }
+                return src;
+            };
+            auto load = [&](int src, float (&c)[3]) {
+                const int32_t i = __shfl_sync(0xffffffffu, li, src & 31);
+                const float* w = wing + size_t(i) * a.G * 3 * plane;
+                c[0] = src < 32 ? w[0] : 0.f;
+                c[1] = src < 32 ? w[plane] : 0.f;
+                c[2] = src < 32 ? w[2 * plane] : 0.f;
+            };
+            float c[3], cn[3];
+            const int n_lines = __popc(m);
+            int src = next();
+            load(src, c);
+            for (int r = 0; r < n_lines; r += LPW) {
+                const int src_n = next();
+                load(src_n, cn);
+                const float lh = __shfl_sync(0xffffffffu, dhi, src & 31), ll = __shfl_sync(0xffffffffu, dlo, src & 31),
+                            lc = __shfl_sync(0xffffffffu, cref, src & 31);
+                const float x = (nh - lh) + (nlo - ll);
+                __syncwarp();
+                if (src < 32) sh.tp[warp][half][lane % FAR_P] = __fdividef(lc, x * x);
+                __syncwarp();
+                if (src < 32) {
+                    const f32x2 a1 = pack2(c[0], c[0]), a2 = pack2(c[1], c[1]), a3 = pack2(c[2], c[2]);
+                    const ulonglong2* tp = reinterpret_cast<const ulonglong2*>(sh.tp[warp][half]);
+#pragma unroll
+                    for (int n = 0; n < FAR_P / 4; n++) {
+                        const ulonglong2 t = tp[n];
+                        part[2 * n] = fma2(t.x, fma2(t.x, fma2(t.x, a3, a2), a1), part[2 * n]);
+                        part[2 * n + 1] = fma2(t.y, fma2(t.y, fma2(t.y, a3, a2), a1), part[2 * n + 1]);
+                    }
+                }
+                src = src_n;
+                c[0] = cn[0];
+                c[1] = cn[1];
+                c[2] = cn[2];
+            }
+            pending += (n_lines + LPW - 1) / LPW;
+            if (pending >= FAR_FLUSH) flush();
+        }
+    flush();
+    __syncthreads();
+    for (int e = tid; e < K * FAR_P; e += FAR_THREADS) {
+        double v = 0.0;
+        for (int w = 0; w < FAR_WARPS; w++) v += sh.node[w][e % FAR_P][e / FAR_P];
+        sh.v[e / FAR_P][e % FAR_P] = v;
+    }
+    __syncthreads();
+    for (int e = tid; e < K * FAR_P; e += FAR_THREADS)
+        sh.cf[e / FAR_P][e % FAR_P] = far_coef(sh.v[e / FAR_P], 1, e % FAR_P);
+    __syncthreads();
+    // the series at every wavelength: the mean in FP64, the variation over the tile in FP32; each warp's
+    // lanes take 32 wavelengths in turn, for a quarter of the layers
+    const int l0 = g * K, nk = min(K, a.L - l0);
+    for (int64_t jb = j0; jb <= jlast; jb += 32) {
+        const int64_t j = jb + lane;
+        const float u = hw > 0 ? fminf(fmaxf(float(((a.wls[min(j, jlast)] - wl_ref) - hw) / hw), -1.f), 1.f) : 0.f;
+        for (int q = warp; q < K; q += FAR_WARPS) {
+            float t0 = 1.f, t1 = u, var = 0.f;
+#pragma unroll
+            for (int n = 1; n < FAR_P; n++) {
+                var = fmaf(float(sh.cf[q][n]), t1, var);
+                const float t2 = fmaf(2.f * u, t1, -t0);
+                t0 = t1;
+                t1 = t2;
+            }
+            sh.stage[lane][q] = sh.cf[q][0] + double(var);
+        }
+        __syncthreads();
+        const int nj = int(min(int64_t(32), jlast - jb + 1));
+        for (int e = tid; e < nj * nk; e += FAR_THREADS) {
+            const int jj = e / nk, q = e - jj * nk;
+            a.alpha[(jb + jj) * a.L + l0 + q] += sh.stage[jj][q];
+        }
+        __syncthreads();
+    }
+}
+
+template <int K>
+__global__ void __launch_bounds__(FAR_THREADS) line_far_kernel(TileArgs a, int tw) {
+    __shared__ FarShared<K> sh;
+    line_far_body<K>(a, blockIdx.x, tw, int(blockIdx.y), sh);
+}
+
 // Mixed-precision tile: TW = blockDim.x wavelengths x the K layers of group g.  Thread t owns
 // wavelength j0 + t and all K layers.  Per staged line:
 //   * lines whose layers are all in their cubic regime over the tile (most evaluations: far
@@ -915,28 +1137,20 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
     const int32_t jm = int32_t(j0 + tid);
     const double dj = (j0 + tid < a.nwl ? a.wls[j0 + tid] : wl_ref) - wl_ref;
     const float xh = float(dj), xl = float(dj - double(xh));
-    if (tid < NTIER) {  // candidate runs of the width tiers
-        const int64_t t0 = a.tier_start[tid], t1 = a.tier_start[tid + 1];
-        if (*a.unsorted) {
-            s_tier[tid][0] = t0;
-            s_tier[tid][1] = t1;
-        } else {
-            const int32_t w = c_tier_w[tid] + 1;
-            const int32_t lo = int32_t(max(int64_t(j0) - w, int64_t(INT32_MIN / 2)));
-            const int32_t hi = int32_t(min(int64_t(jlast) + w, int64_t(INT32_MAX / 2)));
-            s_tier[tid][0] = lower_bound_i32(a.tier_ci, t0, t1, lo);
-            s_tier[tid][1] = upper_bound_i32(a.tier_ci, t0, t1, hi);
-        }
-    }
+    if (tid < NTIER) tier_run(a, tid, j0, jlast, s_tier[tid]);  // candidate runs of the width tiers
     __syncthreads();
 
+    const float kspan = far_tile32(a, s_tier, jlast - j0 + 1) ? FAR_KAPPA32 * span32 : INFINITY;
+    // accumulators of layer pairs (packed FP32 arithmetic on the wing cubics)
+    constexpr int KP = K / 2, QB = wing_quads(K);
     float acc[K], comp[K];
 #pragma unroll
     for (int k = 0; k < K; k++) { acc[k] = 0.f; comp[k] = 0.f; }
 
     const int64_t src0 = int64_t(g) * K;  // the group's first float4 within a line's Lp constants
-    const int cb0 = tid / K, cr0 = tid - cb0 * K;      // this thread's first staged (line, layer)
-    const int cdb = nthr / K, cdr = nthr - cdb * K;    // and the step between its pieces
+    constexpr int PC = K;                                // 16-byte pieces of a staged line (QB <= K)
+    const int cb0 = tid / PC, cr0 = tid - cb0 * PC;      // this thread's first staged (line, piece)
+    const int cdb = nthr / PC, cdr = nthr - cdb * PC;    // and the step between its pieces
     for (int tier = 0; tier < NTIER; tier++)
     for (int64_t base = s_tier[tier][0]; base < s_tier[tier][1]; base += nthr) {
         const int64_t pidx = base + tid;
@@ -948,6 +1162,7 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
             lbi = a.lb[i];
             ubi = a.ub[i];
             take = lbi <= jlast && ubi >= j0;
+            if (take && kspan < INFINITY) take = !far_line32(a, i, g, lbi, ubi, j0, jlast, wl_ref, span32, kspan);
         }
         const unsigned msk = __ballot_sync(0xffffffffu, take);
         if (lane == 0) s_warp[warp] = __popc(msk);
@@ -985,15 +1200,18 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
             if (q < nq) {
                 const int b0 = q * B, nb = min(B, cnt - b0);
                 unsigned char* buf = smem + size_t(q & 1) * a.region;
-                int b = cb0, r = cr0;  // piece e = tid + k nthr is (line b, layer r), stepped without a division
-                for (int e = tid; e < nb * K; e += nthr) {
+                int b = cb0, r = cr0;  // piece e = tid + k nthr is (line b, 16-byte piece r), stepped without a division
+                for (int e = tid; e < nb * PC; e += nthr) {
                     const LineStage32& sl = s_ln[b0 + b];
-                    const float4* src = sl.cubic ? a.params_w : reinterpret_cast<const float4*>(a.params);
-                    cp_async16(buf + (size_t(b) * K + r) * 16, src + (int64_t(sl.li) * Lp + src0 + r));
+                    if (!sl.cubic)
+                        cp_async16(buf + (size_t(b) * PC + r) * 16,
+                                   reinterpret_cast<const float4*>(a.params) + (int64_t(sl.li) * Lp + src0 + r));
+                    else if (r < QB)
+                        cp_async16(buf + (size_t(b) * PC + r) * 16, a.params_w + ((int64_t(sl.li) * G + g) * QB + r));
                     b += cdb;
                     r += cdr;
-                    if (r >= K) {
-                        r -= K;
+                    if (r >= PC) {
+                        r -= PC;
                         b++;
                     }
                 }
@@ -1007,9 +1225,9 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
             __syncthreads();    // ... and everybody else's
             const int b0 = q * B, nb = min(B, cnt - b0);
             const float4* s_par = reinterpret_cast<const float4*>(smem + size_t(q & 1) * a.region);
-            float part[K];
+            f32x2 part[KP];
 #pragma unroll
-            for (int k = 0; k < K; k++) part[k] = 0.f;
+            for (int k = 0; k < KP; k++) part[k] = 0ull;
             for (int b = 0; b < nb; b++) {
                 const LineStage32 st = s_ln[b0 + b];
                 const float4* pr = s_par + b * K;
@@ -1017,10 +1235,15 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
                 const float x = fabsf((xh - st.dhi) + (xl - st.dlo));
                 if (st.cubic) {
                     const float tp = in ? __fdividef(st.cref, x * x) : 0.f;
+                    const f32x2 t2 = pack2(tp, tp);
+                    // planes A1, A2, A3 of K layers (padded to 4): two layer pairs per 16-byte load
 #pragma unroll
-                    for (int k = 0; k < K; k++) {
-                        const float4 p = pr[k];
-                        part[k] = fmaf(tp, fmaf(tp, fmaf(tp, p.z, p.y), p.x), part[k]);
+                    for (int q = 0; q < QB / 3; q++) {
+                        const ulonglong2 a1 = reinterpret_cast<const ulonglong2*>(pr)[q],
+                                         a2 = reinterpret_cast<const ulonglong2*>(pr)[QB / 3 + q],
+                                         a3 = reinterpret_cast<const ulonglong2*>(pr)[2 * (QB / 3) + q];
+                        part[2 * q] = fma2(t2, fma2(t2, fma2(t2, a3.x, a2.x), a1.x), part[2 * q]);
+                        if (2 * q + 1 < KP) part[2 * q + 1] = fma2(t2, fma2(t2, fma2(t2, a3.y, a2.y), a1.y), part[2 * q + 1]);
                     }
                 } else if (__all_sync(0xffffffffu, !in || x > st.xfar)) {
                     // every in-window wavelength of the warp in a closed-form wing branch, chosen
@@ -1030,24 +1253,27 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
 #pragma unroll
                         for (int k = 0; k < K; k++) {
                             const float4 p = pr[k];
+                            float v = part2(part[k / 2], k % 2);
                             if (p.y <= 0.2f) {
                                 const float iv = t * p.x;
-                                part[k] = fmaf(p.z * iv, fmaf(fmaf(3.75f, iv, 1.5f), iv, 1.f), part[k]);
+                                v = fmaf(p.z * iv, fmaf(fmaf(3.75f, iv, 1.5f), iv, 1.f), v);
                             } else {
-                                part[k] += far_lorentz32(p, x2);
+                                v += far_lorentz32(p, x2);
                             }
+                            set2(part[k / 2], k % 2, v);
                         }
                     }
                 } else if (in) {
                     const float t = __fdividef(1.f, x * x);
 #pragma unroll
-                    for (int k = 0; k < K; k++) part[k] += profile32x(pr[k], x, t);
+                    for (int k = 0; k < K; k++)
+                        set2(part[k / 2], k % 2, part2(part[k / 2], k % 2) + profile32x(pr[k], x, t));
                 }
             }
             // batch partial sums enter the accumulators with Kahan compensation
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                const float y = part[k] - comp[k];
+                const float y = part2(part[k / 2], k % 2) - comp[k];
                 const float tt = acc[k] + y;
                 comp[k] = (tt - acc[k]) - y;
                 acc[k] = tt;
@@ -1113,6 +1339,17 @@ __global__ void __launch_bounds__(MAXT, MINB) line_tile_queue_kernel(TileQueue q
             line_tile_body64<K>(s_a, r / q.groups, q.groups > 1 ? int(r % q.groups) : -1, smem);
         __syncthreads();  // s_a and s_item are rewritten for the next item
     }
+}
+
+
+// The far lines of a batch: one CTA per (spectrum, tile, group), spectra interleaved as in the queue.
+template <int K>
+__global__ void __launch_bounds__(FAR_THREADS) line_far_batch_kernel(const TileArgs* spec, int32_t nspec, int tw) {
+    __shared__ FarShared<K> sh;
+    __shared__ TileArgs s_a;
+    if (threadIdx.x == 0) s_a = spec[blockIdx.x % nspec];
+    __syncthreads();
+    line_far_body<K>(s_a, blockIdx.x / nspec, tw, int(blockIdx.y), sh);
 }
 
 }  // namespace korg

@@ -1,7 +1,7 @@
 """Far lines of the line tiles (evaluated at 16 Chebyshev nodes per tile and interpolated) against the
 FP64 oracle, at the sizes where the split can go wrong: tiles cut short by the grid's end, every
-layers-per-group template, other tile widths and a non-uniform grid with a
-gap."""
+layers-per-group template, other tile widths, a non-uniform grid with a gap, and mixed tiles above the
+candidate limit."""
 import os
 
 import numpy as np
@@ -55,3 +55,14 @@ def test_fp64_far_lines_on_an_uneven_grid(gpu_lib, oracle_lib):
     wls = (5002.0 + np.cumsum(d)) * 1e-8
     got, ref = _opacity(gpu_lib, oracle_lib, inp, wls, "fp64")
     np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("L", [56, 80, 130])
+def test_mixed_far_lines_match_oracle(gpu_lib, oracle_lib, L):
+    """FP32 evaluations (a few 1e-7 each) of lines whose sum is dominated by no single one; the seams
+    of the Hjerting branches are the exceptions."""
+    inp = _inputs(L, 5000, 5020, 20000, teff=4500.0)
+    wls = inp.wls.all_wls[:1000 + 65]
+    got, ref = _opacity(gpu_lib, oracle_lib, inp, wls, "mixed")
+    rel = np.abs(got / ref - 1)
+    assert np.percentile(rel, 99.9) <= 2e-6 and rel.max() <= 1e-3
