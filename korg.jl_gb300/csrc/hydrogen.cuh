@@ -213,24 +213,85 @@ __device__ __forceinline__ double brackett_oscillator_strength(int n, int m) {
     return FK * (1 - WT * GINF - (0.222 + GCA / m) * (1 - WT));
 }
 
-// One CTA per (m, layer): the Brackett line m profile (:147-162, :211-251, :272-369).
-template <bool MIXED>
-__global__ void __launch_bounds__(256) brackett_prep_kernel(HLayers hl, int ntrans, int n_max, const double* wls,
-                                                            int64_t nwl, int use_MHD, HOut out, double* Qbase) {
-    __shared__ double s_grid[BR_NP], s_imp[BR_NP], s_qs[BR_NP], s_tmp[BR_NP];
-    __shared__ int s_red;
-    const int n = 4, m = 5 + blockIdx.x, l = blockIdx.y, L = hl.L, k = threadIdx.x;
-    const int slot = ntrans + blockIdx.x;
-    const double T = hl.T[l], ne = hl.ne[l];
+// src/line_absorption.jl:169-182 with the table-driven exp and log (expint1_64)
+__device__ __forceinline__ double expint1_t(double x, const MathTables& mt) {
+    if (x < 0) return 0.0;
+    if (x <= 0.01) return -flog64(x, mt) - 0.577215 + x;
+    if (x <= 1.0)
+        return -flog64(x, mt) - 0.57721566 +
+               x * (0.99999193 + x * (-0.24991055 + x * (0.05519968 + x * (-0.00976004 + x * 0.00107857))));
+    if (x <= 30.0)
+        return (x * (x + 2.334733) + 0.25062) / ((x * (x + 3.330657) + 1.681534) * x) * fexp64(-x, mt);
+    return 0.0;
+}
+
+// Per-(line, layer) scalars of brackett_line_stark_profiles (:272-369), computed by one warp: a few
+// pow and divisions each, which every thread of the block repeated before (half the kernel's FP64 work).
+struct BrackettConst {
+    double wl0, window, wstart, wend, step, nu0, sdop, stark_width;
+    double C1, C2, G1, GCON1, GCON2, Pp, dbdl, thin;  // thin: the width where y1, y2 are tiny
+    double inv_nu0_kT;                                // h / (k T)
+};
+__device__ BrackettConst brackett_const(int n, int m, double T, double ne, double xi, double wlmin, double wlmax) {
+    BrackettConst q;
     const double E = RYDBERGH_EV * (1.0 / (n * n) - 1.0 / (m * m));
     const double wl0 = HPLANCK_EV * C_CGS / E;
     const double F0 = 1.25e-9 * pow(ne, 2.0 / 3.0);
     const double Knm = greim_1960_Knm(n, m);
-    const double stark_width = 1.6678E-18 * Knm * F0 * C_CGS;
-    const double sdop = doppler_width(wl0, T, 1.008 * AMU_CGS, hl.xi[l]);
-    const double window = 5 * fmax(sdop, stark_width);
+    q.wl0 = wl0;
+    q.stark_width = 1.6678E-18 * Knm * F0 * C_CGS;
+    q.sdop = doppler_width(wl0, T, 1.008 * AMU_CGS, xi);
+    q.window = 5 * fmax(q.sdop, q.stark_width);
+    q.wstart = fmax(wlmin, wl0 - q.window);
+    q.wend = fmin(wl0 + q.window, wlmax);
+    q.step = (q.wend - q.wstart) / (BR_NP - 1);
+    q.nu0 = C_CGS / wl0;
+    const double ne_1_6 = pow(ne, 1.0 / 6.0);
+    q.GCON1 = 0.2 + 0.09 * sqrt(T / 10000) / (1 + ne / 1.E13);
+    q.GCON2 = 0.2 / (1 + ne / 1.E15);
+    const double Y1WHT = (m - n <= 3) ? 1e14 : 1e13;
+    const double WTY1 = 1 / (1 + ne / Y1WHT);
+    const double Y1B = 2 / (1 + 0.012 / T * sqrt(ne / T));
+    const double mm_nn = double(m * m - n * n);
+    const double C1CON = Knm / wl0 * (mm_nn * mm_nn) / double(n * n * m * m) * 1e-8;
+    const double Y1SCAL = 320 * (pow(T / 10000, 0.3) / ne_1_6) * WTY1 + Y1B * (1 - WTY1);
+    q.C1 = F0 * 78940 / T * C1CON * Y1SCAL;
+    const double kl = Knm / wl0;
+    q.C2 = (F0 * F0) / (5.96E-23 * ne) * (kl * kl) * 1e-16;
+    q.G1 = 6.77 * sqrt(q.C1);
+    q.Pp = ne_1_6 * 0.08989 / sqrt(T);
+    q.dbdl = 1e8 / (Knm * F0);
+    q.thin = q.G1 * fmax(0.0, 0.2114 + log(sqrt(q.C2) / q.C1)) * (1 - q.GCON1 - q.GCON2);
+    q.inv_nu0_kT = HPLANCK_CGS / KBOLTZ_CGS / T;
+    return q;
+}
+
+// One CTA per (m, layer): the Brackett line m profile (:147-162, :211-251, :272-369).  Bound by the
+// FP64 pipe: ~200 operations per profile point, then up to two direct convolutions of 201 points.
+// 26 lines x 56 layers: 235 -> 129 us (window at 5100 A), 465 -> 236 us (15,000 A, both convolutions).
+template <bool MIXED>
+__global__ void __launch_bounds__(256) brackett_prep_kernel(HLayers hl, int ntrans, int n_max, const double* wls,
+                                                            int64_t nwl, int use_MHD, HOut out, double* Qbase,
+                                                            const MathTables* math) {
+    __shared__ double s_grid[BR_NP], s_imp[BR_NP], s_qs[BR_NP], s_tmp[BR_NP];
+    __shared__ MathTables s_math;
+    __shared__ BrackettConst s_c;
+    __shared__ int s_red;
+    const int n = 4, m = 5 + blockIdx.x, l = blockIdx.y, L = hl.L, k = threadIdx.x;
+    const int slot = ntrans + blockIdx.x;
+    const double T = hl.T[l], ne = hl.ne[l];
     const double wlmin = wls[0], wlmax = wls[nwl - 1];
-    const double wstart = fmax(wlmin, wl0 - window), wend = fmin(wl0 + window, wlmax);
+    load_math_tables(s_math, math);
+    if (k < 32) {
+        const BrackettConst c = brackett_const(n, m, T, ne, hl.xi[l], wlmin, wlmax);
+        if (k == 0) {
+            s_c = c;
+            s_red = -1;
+        }
+    }
+    __syncthreads();
+    const double wl0 = s_c.wl0, step = s_c.step, sdop = s_c.sdop, stark_width = s_c.stark_width, nu0 = s_c.nu0;
+    const double window = s_c.window, wstart = s_c.wstart, wend = s_c.wend;
     HRec r = {};
     r.kind = HK_OFF;
     r.lb = 0;
@@ -240,65 +301,43 @@ __global__ void __launch_bounds__(256) brackett_prep_kernel(HLayers hl, int ntra
         if (k == 0) out.rec[int64_t(slot) * L + l] = r;
         return;
     }
-    const double step = (wend - wstart) / (BR_NP - 1);
-    const double nu0 = C_CGS / wl0;
-    if (k < BR_NP) s_grid[k] = (k == BR_NP - 1) ? wend : wstart + k * step;
-    if (k == 0) s_red = -1;
-    __syncthreads();
-    // brackett_line_stark_profiles (:272-369)
-    const double ne_1_6 = pow(ne, 1.0 / 6.0);
-    const double GCON1 = 0.2 + 0.09 * sqrt(T / 10000) / (1 + ne / 1.E13);
-    const double GCON2 = 0.2 / (1 + ne / 1.E15);
-    const double Y1WHT = (m - n <= 3) ? 1e14 : 1e13;
-    const double WTY1 = 1 / (1 + ne / Y1WHT);
-    const double Y1B = 2 / (1 + 0.012 / T * sqrt(ne / T));
-    const double mm_nn = double(m * m - n * n);
-    const double C1CON = Knm / wl0 * (mm_nn * mm_nn) / double(n * n * m * m) * 1e-8;
-    const double Y1SCAL = 320 * (pow(T / 10000, 0.3) / ne_1_6) * WTY1 + Y1B * (1 - WTY1);
-    const double C1 = F0 * 78940 / T * C1CON * Y1SCAL;
-    const double kl = Knm / wl0;
-    const double C2 = (F0 * F0) / (5.96E-23 * ne) * (kl * kl) * 1e-16;
-    const double G1 = 6.77 * sqrt(C1);
-    const double Pp = ne_1_6 * 0.08989 / sqrt(T);
-    const double dbdl = 1e8 / (Knm * F0);
+    double nu = 0.0;
     if (k < BR_NP) {
-        const double wl = s_grid[k];
-        if (C_CGS / wl < nu0) atomicMax(&s_red, k);
-        const double beta = fabs(wl - wl0) / F0 / Knm * 1e8;
-        const double y1 = C1 * beta, y2 = C2 * (beta * beta);
+        const double wl = (k == BR_NP - 1) ? wend : wstart + k * step;
+        s_grid[k] = wl;
+        nu = C_CGS / wl;
+        if (nu < nu0) atomicMax(&s_red, k);
+        // brackett_line_stark_profiles (:272-369)
+        const double beta = fabs(wl - wl0) * s_c.dbdl;
+        const double y1 = s_c.C1 * beta, y2 = s_c.C2 * (beta * beta);
         double width;
         if ((y2 <= 1e-4) && (y1 <= 1e-5)) {
-            width = G1 * fmax(0.0, 0.2114 + log(sqrt(C2) / C1)) * (1 - GCON1 - GCON2);
+            width = s_c.thin;
         } else {
             const double t90 = 90 * y1;
-            const double GAM = (G1 * (0.5 * exp(-fmin(80.0, y1)) + expint1_64(y1) - 0.5 * expint1_64(y2)) *
-                                (1 - GCON1 / (1 + t90 * t90 * t90) - GCON2 / (1 + 2000 * y1)));
+            const double GAM = (s_c.G1 * (0.5 * fexp64(-fmin(80.0, y1), s_math) + expint1_t(y1, s_math) -
+                                          0.5 * expint1_t(y2, s_math)) *
+                                (1 - s_c.GCON1 / (1 + t90 * t90 * t90) - s_c.GCON2 / (1 + 2000 * y1)));
             width = GAM <= 1e-20 ? 0.0 : GAM;
         }
         s_imp[k] = width > 0 ? width / (PI * (width * width + beta * beta)) : 0.0;
         const double ps = (0.9 * y1) * (0.9 * y1);
         double qe = (ps + 0.03 * sqrt(y1)) / (ps + 1.0);
-        s_qs[k] = holtsmark_profile(beta, Pp) * (1 + qe);
+        s_qs[k] = holtsmark_profile(beta, s_c.Pp) * (1 + qe);
     }
     __syncthreads();
     if (k < BR_NP) {
-        const double wl = s_grid[k];
-        const double f = sqrt(wl / wl0);
-        double a = s_imp[k] * f, b = s_qs[k] * f;
-        if (k <= s_red) {
-            const double bz = exp((HPLANCK_CGS * (C_CGS / wl - nu0)) / KBOLTZ_CGS / T);
-            a = a * bz;
-            b = b * bz;
-        }
-        s_imp[k] = a * dbdl;
-        s_qs[k] = b * dbdl;
+        const double f = sqrt(s_grid[k] / wl0) * s_c.dbdl;
+        const double g = k <= s_red ? f * fexp64(s_c.inv_nu0_kT * (nu - nu0), s_math) : f;
+        s_imp[k] *= g;
+        s_qs[k] *= g;
     }
     __syncthreads();
     const int start = (BR_NP + 1) / 2 - 1;
     if (sdop / stark_width > 0.25) {  // :240-244 Doppler convolution of the quasistatic part
         if (k < BR_NP) {
             const double d = s_grid[k] - wl0;
-            s_tmp[k] = exp(-0.5 * (d * d) / (sdop * sdop)) / SQRT_2PI / sdop;
+            s_tmp[k] = fexp64(-0.5 * (d * d) / (sdop * sdop), s_math) / SQRT_2PI / sdop;
         }
         __syncthreads();
         double s = 0;
@@ -323,6 +362,7 @@ __global__ void __launch_bounds__(256) brackett_prep_kernel(HLayers hl, int ntra
         const double beta = 1 / (KBOLTZ_EV * T);
         const double E_low = RYDBERGH_EV * (1 - 1.0 / (n * n));
         const double w = use_MHD ? hummer_mihalas_w(double(m), hl.nH[l], hl.nHe[l], ne) : 1.0;
+        const double E = RYDBERGH_EV * (1.0 / (n * n) - 1.0 / (m * m));
         const double levels = w * exp(-beta * E_low) * (1 - exp(-beta * E)) / hl.UH[l];
         const double gf = 2 * (n * n) * brackett_oscillator_strength(n, m);
         r.amp = gf * hl.nH[l] * sigma_line(wl0) * levels;
@@ -345,7 +385,7 @@ struct HTileArgs {
     double* alpha;
     const double* wls;
     int64_t nwl;
-    int32_t L, G, ntrans, ntot;
+    int32_t L, TW, ntrans, ntot;
     const HRec* rec;
     const double* Q;       // Stehle tables then Brackett profiles
     const float* Q32;
@@ -355,12 +395,18 @@ struct HTileArgs {
     const float* logdnu32;
 };
 
+// A block takes TW wavelengths; its thread groups and the grid's second dimension share the layers
+// (layer l = slice + slices k).  Long grids: 128 wavelengths x 4 groups (64 x 8 above 64 layers: at 56
+// layers the same time in the infrared, a fifth more in the optical).  Short grids (at most HT_SHORT
+// wavelengths): 32 x 4 and two blocks in y, so that they reach all SMs.  In the infrared the
+// Brackett interpolation's FP64 operations bound it, elsewhere latency.  100,001 points of the H band:
+// 809 -> 740 us; 2,001 points at 5100 A: 139 -> 81 us.
+constexpr int64_t HT_SHORT = 32768;
 template <bool MIXED, int KMAX>
 __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile_kernel(HTileArgs a) {
     const int tid = threadIdx.x;
-    const int L = a.L, G = a.G;
-    const int TW = blockDim.x / G;
-    const int jl = tid % TW, g = tid / TW;
+    const int L = a.L, TW = a.TW, G = (blockDim.x / TW) * gridDim.y;  // layer slices
+    const int jl = tid % TW, g = tid / TW + (blockDim.x / TW) * blockIdx.y;
     const int64_t j0 = int64_t(blockIdx.x) * TW, jg = j0 + jl;
     const int64_t jlast = min(j0 + TW, a.nwl) - 1;
     const bool live = jg < a.nwl;
@@ -385,16 +431,25 @@ __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile
             const int l = g + G * k;
             if (l >= L) continue;
             const HRec& r = a.rec[int64_t(t) * L + l];
-            if (r.kind == HK_OFF || jg < r.lb || jg > r.ub) continue;
-            if (r.kind == HK_BRACKETT) {
+            const int4 w = *reinterpret_cast<const int4*>(&r.lb);  // lb, ub, kind, nD
+            const int kind = w.z;
+            if (kind == HK_OFF || jg < w.x || jg > w.y) continue;
+            if (kind == HK_BRACKETT) {
                 // linear_interpolation over the 201-point range grid (:249, :160); the position on
-                // the grid by the reciprocal step (one rounding more than a division, no FP64 divide)
+                // the grid by the reciprocal step, its interval by adding 1.5 2^52 (round to nearest
+                // of u - 1/2; at a grid point either interval gives the same value)
                 const double u = (wl - r.wl0) * r.a;
-                int i = int(floor(u));
-                i = i < 0 ? 0 : (i > BR_NP - 2 ? BR_NP - 2 : i);
-                const double d = u - i;
-                const double* q = a.Q + brQ + (int64_t(t - a.ntrans) * L + l) * BR_NP;
-                const double term = (q[i] * (1 - d) + q[i + 1] * d) * r.amp;
+                const double MAGIC = 6755399441055744.0;
+                double kd = (u - 0.5) + MAGIC;
+                int i = __double2loint(kd);
+                kd -= MAGIC;
+                if (unsigned(i) > unsigned(BR_NP - 2)) {
+                    i = i < 0 ? 0 : BR_NP - 2;
+                    kd = i;
+                }
+                const double* q = a.Q + brQ + (int64_t(t - a.ntrans) * L + l) * BR_NP + i;
+                const double q0 = q[0];
+                const double term = fma(u - kd, q[1] - q0, q0) * r.amp;
                 if (MIXED) {
                     const float y = float(term) - float(comp[k]), tt = float(acc[k]) + y;
                     comp[k] = Acc((tt - float(acc[k])) - y);
@@ -404,10 +459,10 @@ __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile
                 }
                 continue;
             }
-            const int nDt = r.nD;
+            const int nDt = w.w;
             if (MIXED) {
                 float v32 = 0.f;
-                if (r.kind == HK_STARK_ABO) {  // :136
+                if (kind == HK_STARK_ABO) {  // :136
                     const float x = float(fabs(wl - r.wl0));
                     v32 = profile32x(r.abo32, x, __fdividef(1.f, x * x));
                 }
@@ -448,7 +503,7 @@ __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile
                 comp[k] = Acc((tt - float(acc[k])) - y);
                 acc[k] = Acc(tt);
             } else {
-                if (r.kind == HK_STARK_ABO) acc[k] += Acc(voigt64(r.a, fabs(wl - r.wl0) * r.inv_s) * r.scale);  // :136
+                if (kind == HK_STARK_ABO) acc[k] += Acc(voigt64(r.a, fabs(wl - r.wl0) * r.inv_s) * r.scale);  // :136
                 double sd = fabs(nu - r.nu0) / r.F0;  // :141
                 sd = sd + (sd == 0) * 2.2250738585072014e-308;  // _zero2epsilon
                 const double x = log(sd);

@@ -56,7 +56,7 @@ struct korg_ctx {
     cudaStream_t stream = nullptr;  // used by the host-pointer calls and for graph capture
     std::string err;
     // scratch arena: grown on demand, never shrunk, freed by korg_destroy
-    DevBuf lines_scratch, counters, tune_alpha;
+    DevBuf lines_scratch, ref_part, counters, tune_alpha;
     DevBuf hrec, hQ, hQ32, hulb, huub;
     DevBuf stage_dev, aref, alpha, flux, cntm, math;
     DevBuf vjp_g, vjp_dpar, vjp_small, vjp_hder, vjp_hdq;  // reverse mode
@@ -293,16 +293,16 @@ int prep_lines(korg_ctx* ctx, const LineScratch& sc, const double* wls, int64_t 
                cudaStream_t s) {
     const int L = lay.L, Lp = G * kmax;
     auto* ctr = static_cast<unsigned long long*>(ctx->counters.p);
-    layer_const_kernel<<<(L + 127) / 128, 128, 0, s>>>(lay, sc.lc);
+    layer_const_kernel<<<(L + 31) / 32, 32, 0, s>>>(lay, sc.lc);
     PrepOut po{sc.params, sc.lb, sc.ub, sc.ci, sc.xfar, sc.amask, Lp, kmax, G, ctr, ctr + 1, sc.params_w, sc.xcub};
-    const size_t prep_smem = size_t(256 / 32) * Lp * (sizeof(float) + sizeof(int));
-    const unsigned pblocks = unsigned((ln.n * 32 + 255) / 256);
+    const PrepGeom pg = prep_geom(ln.n, mixed);
     auto* math = static_cast<MathTables*>(ctx->math.p);
     if (mixed)
-        line_prep_mixed_kernel<<<prep_mixed_blocks(ln.n), 32 * PREP_WARPS, prep_mixed_smem(Lp), s>>>(
-            ln, lay, sc.lc, cn, wls, nwl, cutoff, po, math);
+        line_prep_mixed_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, true), s>>>(
+            ln, lay, sc.lc, cn, wls, nwl, cutoff, po, math, pg.lpw);
     else
-        line_prep64_kernel<<<pblocks, 256, prep_smem, s>>>(ln, lay, sc.lc, cn, wls, nwl, cutoff, po, math);
+        line_prep64_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, false), s>>>(ln, lay, sc.lc, cn, wls, nwl,
+                                                                                      cutoff, po, math);
     KCUDA(cudaGetLastError());
     const int nblk = part_blocks(ln.n);
     TierLists tl{sc.tier_idx, sc.tier_ci, sc.tier_meta, sc.tier_meta + NTIER + 1};
@@ -473,6 +473,24 @@ int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t
     return run_tiles(ctx, ta, kmax, g, nullptr, mixed, ln.n, s);
 }
 
+// alpha_ref[l] += the reference list's opacity at the reference wavelength, FP64 (src/synthesize.jl:265-283).
+int run_ref_lines(korg_ctx* ctx, double* aref, const double* ref_wl, const LinesDev& ln, const LayersDev& lay,
+                  const CntmDev& cn, double cutoff, cudaStream_t s) {
+    if (ln.n == 0) return KORG_OK;
+    if (lay.L > 256) return set_err(ctx, KORG_EINVAL, "at most 256 layers are supported (got %d)", lay.L);
+    if (ln.n > INT32_MAX) return set_err(ctx, KORG_EINVAL, "sizes exceed int32 indexing");
+    KCHECK(ensure(ctx, ctx->ref_part, sizeof(double) * size_t(ln.n) * lay.L));
+    double* part = static_cast<double*>(ctx->ref_part.p);
+    auto* ctr = static_cast<unsigned long long*>(ctx->counters.p);
+    const int warps = prep_block_warps(ln.n);
+    line_point_kernel<<<unsigned((ln.n + warps - 1) / warps), 32 * warps, 0, s>>>(
+        ln, lay, cn, ref_wl, cutoff, part, ctr, ctr + 1, static_cast<MathTables*>(ctx->math.p));
+    line_point_sum_kernel<<<lay.L, 128, 0, s>>>(part, ln.n, lay.L, aref);
+    KCUDA(cudaGetLastError());
+    ctx->stats_pending = true;
+    return KORG_OK;
+}
+
 // ------------------------------------------------------------------ hydrogen lines
 // The per-(transition, layer) records and profile tables of the hydrogen lines (the prep kernels).
 int run_hydrogen_prep(korg_ctx* ctx, const double* wls, int64_t nwl, const HLayers& hl, double window, int use_MHD,
@@ -493,16 +511,18 @@ int run_hydrogen_prep(korg_ctx* ctx, const double* wls, int64_t nwl, const HLaye
             static_cast<int32_t*>(ctx->hulb.p), static_cast<int32_t*>(ctx->huub.p)};
     const int n = ntrans * L;
     if (mixed)
-        hline_prep_kernel<true><<<(n + 127) / 128, 128, 0, s>>>(ctx->stark, hl, wls, nwl, window, use_MHD, ho, ho.Q);
+        hline_prep_kernel<true><<<(n + 31) / 32, 32, 0, s>>>(ctx->stark, hl, wls, nwl, window, use_MHD, ho, ho.Q);
     else
-        hline_prep_kernel<false><<<(n + 127) / 128, 128, 0, s>>>(ctx->stark, hl, wls, nwl, window, use_MHD, ho, ho.Q);
+        hline_prep_kernel<false><<<(n + 31) / 32, 32, 0, s>>>(ctx->stark, hl, wls, nwl, window, use_MHD, ho, ho.Q);
     KCUDA(cudaGetLastError());
     double* brQ = ho.Q + size_t(ntrans) * L * HND_MAX;
     if (nbr > 0) {
         if (mixed)
-            brackett_prep_kernel<true><<<dim3(nbr, L), 256, 0, s>>>(hl, ntrans, ctx->n_max, wls, nwl, use_MHD, ho, brQ);
+            brackett_prep_kernel<true><<<dim3(nbr, L), 256, 0, s>>>(hl, ntrans, ctx->n_max, wls, nwl, use_MHD, ho, brQ,
+                                                                      static_cast<MathTables*>(ctx->math.p));
         else
-            brackett_prep_kernel<false><<<dim3(nbr, L), 256, 0, s>>>(hl, ntrans, ctx->n_max, wls, nwl, use_MHD, ho, brQ);
+            brackett_prep_kernel<false><<<dim3(nbr, L), 256, 0, s>>>(hl, ntrans, ctx->n_max, wls, nwl, use_MHD, ho, brQ,
+                                                                      static_cast<MathTables*>(ctx->math.p));
         KCUDA(cudaGetLastError());
     }
     ctx->hyd_prep = mixed ? 1 : 0;
@@ -513,10 +533,11 @@ int run_hydrogen_prep(korg_ctx* ctx, const double* wls, int64_t nwl, const HLaye
 int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, const HLayers& hl, double window,
                  int use_MHD, bool mixed, cudaStream_t s) {
     const int L = hl.L;
-    // the hydrogen tile kernel interleaves layers: thread group g owns layers g, g+G, ...
-    int kmax = 16, G = (L + 15) / 16;
-    if (G > 8) { kmax = 32; G = (L + 31) / 32; }
-    if (G > 8) return set_err(ctx, KORG_EINVAL, "at most 256 layers are supported (got %d)", L);
+    if (L > 256) return set_err(ctx, KORG_EINVAL, "at most 256 layers are supported (got %d)", L);
+    // layer slices (slice g owns layers g, g + slices, ...): thread groups of a block x blocks in y
+    const bool shrt = nwl <= HT_SHORT;
+    const int TW = shrt ? 32 : (L <= 64 ? 128 : 64), groups = shrt || L <= 64 ? 4 : 8, gy = shrt ? 2 : 1;
+    const int kmax = (L + groups * gy - 1) / (groups * gy);  // layers per thread
     HOut ho;
     KCHECK(run_hydrogen_prep(ctx, wls, nwl, hl, window, use_MHD, mixed, s, &ho));
     const int ntrans = ctx->stark.ntrans;
@@ -526,7 +547,7 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
     ha.wls = wls;
     ha.nwl = nwl;
     ha.L = L;
-    ha.G = G;
+    ha.TW = TW;
     ha.ntrans = ntrans;
     ha.ntot = ntot;
     ha.rec = ho.rec;
@@ -537,15 +558,18 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
     ha.d_off = ctx->stark.d_off;
     ha.logdnu = ctx->stark.logdnu;
     ha.logdnu32 = ctx->stark.logdnu32;
-    const int TW = G <= 4 ? 128 : 64;
-    const unsigned tiles = unsigned((nwl + TW - 1) / TW);
-    const int threads = TW * G;
-    if (mixed) {
-        if (kmax == 16) hline_tile_kernel<true, 16><<<tiles, threads, 0, s>>>(ha);
-        else hline_tile_kernel<true, 32><<<tiles, threads, 0, s>>>(ha);
+    const dim3 grid(unsigned((nwl + TW - 1) / TW), unsigned(gy));
+    const int threads = TW * groups;
+    auto go = [&](auto kern) { kern<<<grid, threads, 0, s>>>(ha); };
+    if (kmax <= 8) {
+        if (mixed) go(hline_tile_kernel<true, 8>);
+        else go(hline_tile_kernel<false, 8>);
+    } else if (kmax <= 16) {
+        if (mixed) go(hline_tile_kernel<true, 16>);
+        else go(hline_tile_kernel<false, 16>);
     } else {
-        if (kmax == 16) hline_tile_kernel<false, 16><<<tiles, threads, 0, s>>>(ha);
-        else hline_tile_kernel<false, 32><<<tiles, threads, 0, s>>>(ha);
+        if (mixed) go(hline_tile_kernel<true, 32>);
+        else go(hline_tile_kernel<false, 32>);
     }
     KCUDA(cudaGetLastError());
     return KORG_OK;
@@ -579,7 +603,7 @@ int run_synthesize(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& l
     KCUDA(cudaMemcpyAsync(aref, in->alpha_ref_cntm, sizeof(double) * L, cudaMemcpyDeviceToDevice, s));
     const CntmDev cref{1, nullptr, in->alpha_ref_cntm};
     record(ctx, 1, s);
-    KCHECK(run_line_absorption(ctx, aref, ref_wl_dev, 1, ln5, lay, cref, in->cutoff_threshold, false, s));
+    KCHECK(run_ref_lines(ctx, aref, ref_wl_dev, ln5, lay, cref, in->cutoff_threshold, s));
     // :293-303 hydrogen lines
     record(ctx, 3, s);
     if (in->hydrogen_lines) {
@@ -689,8 +713,7 @@ int enqueue_batch(korg_ctx* ctx, const BatchPlan& p, int nspec, const korg_batch
             KCUDA(cudaGetLastError());
             KCUDA(cudaMemcpyAsync(aref, in.alpha_ref_cntm, sizeof(double) * L, cudaMemcpyDeviceToDevice, s));
             const CntmDev cref{1, nullptr, in.alpha_ref_cntm};
-            KCHECK(run_line_absorption(ctx, aref, d_refwl + i, 1, lines_dev(&it[i].lines5), lay, cref,
-                                       in.cutoff_threshold, false, s));
+            KCHECK(run_ref_lines(ctx, aref, d_refwl + i, lines_dev(&it[i].lines5), lay, cref, in.cutoff_threshold, s));
             if (in.hydrogen_lines) {
                 const HLayers hl{L, lay.T, lay.ne, in.nH_I, in.nHe_I, in.UH_I, lay.xi};
                 KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in.hydrogen_window, in.use_MHD, mixed, s));
@@ -845,7 +868,7 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         alpha_init_kernel<<<unsigned((nwl + 63) / 64), 256, 0, s>>>(alpha, wls, nwl, L, cn);
         KCUDA(cudaGetLastError());
         KCUDA(cudaMemcpyAsync(aref, in->alpha_ref_cntm, sizeof(double) * L, cudaMemcpyDeviceToDevice, s));
-        KCHECK(run_line_absorption(ctx, aref, ref_wl_dev, 1, ln5, lay, cref, in->cutoff_threshold, false, s));
+        KCHECK(run_ref_lines(ctx, aref, ref_wl_dev, ln5, lay, cref, in->cutoff_threshold, s));
         if (in->hydrogen_lines)
             KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s));
         // every line at every wavelength: the mixed line adjoint rounds the opacity cotangent to FP32,
@@ -1259,7 +1282,7 @@ KORG_API void korg_destroy(korg_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     drop_graph(ctx);
-    DevBuf* bufs[] = {&ctx->lines_scratch, &ctx->counters, &ctx->tune_alpha, &ctx->hrec, &ctx->hQ, &ctx->hQ32,
+    DevBuf* bufs[] = {&ctx->lines_scratch, &ctx->ref_part, &ctx->counters, &ctx->tune_alpha, &ctx->hrec, &ctx->hQ, &ctx->hQ32,
                       &ctx->hulb, &ctx->huub, &ctx->stage_dev, &ctx->aref, &ctx->alpha, &ctx->flux, &ctx->cntm,
                       &ctx->math, &ctx->b_alpha, &ctx->b_lines, &ctx->b_meta, &ctx->vjp_g, &ctx->vjp_dpar,
                       &ctx->vjp_small, &ctx->vjp_hder, &ctx->vjp_hdq, &ctx->mx_layers};
@@ -2808,19 +2831,19 @@ extern "C" KORG_API int korg_line_absorption_noalloc(double* alpha, const double
     const CntmDev cn{cntm->nk, cntm->knots, cntm->vals};
     auto* lc = reinterpret_cast<LayerConst*>(sp + o_lc);
     auto* math = reinterpret_cast<MathTables*>(sp + o_math);
-    layer_const_kernel<<<(L + 127) / 128, 128, 0, s>>>(lay, lc);
+    layer_const_kernel<<<(L + 31) / 32, 32, 0, s>>>(lay, lc);
     PrepOut po{sp + o_par, reinterpret_cast<int32_t*>(sp + o_lb), reinterpret_cast<int32_t*>(sp + o_ub),
                reinterpret_cast<int32_t*>(sp + o_ci), reinterpret_cast<float*>(sp + o_xfar),
                reinterpret_cast<uint32_t*>(sp + o_am), Lp, kmax, G, ctr, ctr + 1,
                mixed ? reinterpret_cast<float4*>(sp + o_par) + size_t(n) * Lp : nullptr,
                mixed ? reinterpret_cast<float*>(sp + o_xfar) + size_t(n) * G : nullptr};
-    const size_t prep_smem = size_t(256 / 32) * Lp * (sizeof(float) + sizeof(int));
-    const unsigned pblocks = unsigned((n * 32 + 255) / 256);
+    const PrepGeom pg = prep_geom(n, mixed);
     if (mixed)
-        line_prep_mixed_kernel<<<prep_mixed_blocks(n), 32 * PREP_WARPS, prep_mixed_smem(Lp), s>>>(
-            ln, lay, lc, cn, wls, nwl, cutoff, po, math);
+        line_prep_mixed_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, true), s>>>(ln, lay, lc, cn, wls, nwl,
+                                                                                         cutoff, po, math, pg.lpw);
     else
-        line_prep64_kernel<<<pblocks, 256, prep_smem, s>>>(ln, lay, lc, cn, wls, nwl, cutoff, po, math);
+        line_prep64_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, false), s>>>(ln, lay, lc, cn, wls, nwl,
+                                                                                      cutoff, po, math);
     TierLists tl{reinterpret_cast<int32_t*>(sp + o_ti), reinterpret_cast<int32_t*>(sp + o_tc), meta, meta + NTIER + 1};
     int32_t* bcnt = meta + NTIER + 2;
     tier_count_kernel<<<nblk, PART_THREADS, 0, s>>>(po.lb, po.ub, po.ci, n, bcnt, tl.unsorted);

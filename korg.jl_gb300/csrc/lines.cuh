@@ -15,6 +15,8 @@
 //          candidates is compacted with warp ballots, and the constants of each batch of lines
 //          are copied to shared memory with cp.async, double buffered.
 #pragma once
+#include <algorithm>
+
 #include "physics.cuh"
 
 namespace korg {
@@ -52,9 +54,7 @@ struct LayerConst {
     float T32, xi32, ne32, nv32, stark6_32, vdw3_32;
 };
 
-__global__ void layer_const_kernel(LayersDev lay, LayerConst* out) {
-    int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= lay.L) return;
+__device__ __forceinline__ LayerConst layer_const(const LayersDev& lay, int l) {
     double T = lay.T[l];
     LayerConst c;
     c.beta = 1 / (KBOLTZ_EV * T);
@@ -66,7 +66,12 @@ __global__ void layer_const_kernel(LayersDev lay, LayerConst* out) {
     c.nv32 = float(lay.n_eff_vdW[l]);
     c.stark6_32 = float(c.stark6);
     c.vdw3_32 = float(c.vdw3);
-    out[l] = c;
+    return c;
+}
+
+__global__ void layer_const_kernel(LayersDev lay, LayerConst* out) {
+    int l = blockIdx.x * blockDim.x + threadIdx.x;
+    if (l < lay.L) out[l] = layer_const(lay, l);
 }
 
 struct PrepOut {
@@ -233,6 +238,65 @@ __global__ void __launch_bounds__(256) line_prep64_kernel(LinesDev ln, LayersDev
     if (lane == 0) store_window(out, i, lwin, dwin, q.wl, wls, nwl, L);
 }
 
+// Lines at one wavelength `*wl_at` (the reference wavelength, src/synthesize.jl:265-283), in FP64: one
+// warp per line, lanes over layers, every layer's contribution written to part[i][L] (0 outside the
+// line's window); line_point_sum_kernel adds them up.  The tile path (prologue, candidate lists, one
+// thread at work per layer group) took 62 + 124 us for 409 lines x 56 layers (80 + 1233 us for 80 layers of
+// a cool giant), these two 50 + 6 (66 + 6).
+__global__ void __launch_bounds__(256) line_point_kernel(LinesDev ln, LayersDev lay, CntmDev cn, const double* wl_at,
+                                                         double cutoff, double* part, unsigned long long* evals,
+                                                         unsigned long long* nlines, const MathTables* math) {
+    __shared__ MathTables s_math;
+    load_math_tables(s_math, math);
+    __syncthreads();
+    const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= ln.n) return;
+    const int L = lay.L;
+    const LineConst q = line_const(ln, i);
+    const KnotPos kp = knot_pos(cn.knots, cn.nk, q.wl);
+    const double wl = *wl_at, x = fabs(wl - q.wl);
+    double dwin = 0.0, lwin = 0.0;
+    double* dst = part + i * L;
+    for (int l = lane; l < L; l += 32) {
+        const LayerConst c = layer_const(lay, l);
+        const LineLayer64 r = line_layer64(q, lay, c, cn, kp, cutoff, l, s_math);
+        dwin = fmax(dwin, r.dw);
+        lwin = fmax(lwin, r.lw);
+        const double inv_s = 1 / (r.sigma * SQRT_2);  // :246-248
+        dst[l] = voigt64(r.gamma * inv_s, x * inv_s) * (inv_s / SQRT_PI * r.amp);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        dwin = fmax(dwin, __shfl_xor_sync(0xffffffffu, dwin, o));
+        lwin = fmax(lwin, __shfl_xor_sync(0xffffffffu, lwin, o));
+    }
+    const double window = sqrt(lwin * lwin + dwin * dwin);    // :113
+    if (wl >= q.wl - window && wl <= q.wl + window) {         // :114-115 on a grid of one point
+        if (lane == 0) {
+            atomicAdd(evals, (unsigned long long)L);
+            atomicAdd(nlines, 1ull);
+        }
+    } else {
+        for (int l = lane; l < L; l += 32) dst[l] = 0.0;
+    }
+}
+
+// alpha[l] += sum over the lines of part[i][l]: one block per layer, a fixed tree (reproducible)
+__global__ void __launch_bounds__(128) line_point_sum_kernel(const double* part, int64_t n, int L, double* alpha) {
+    __shared__ double s_sum[128];
+    const int l = blockIdx.x, t = threadIdx.x;
+    double v = 0.0;
+    for (int64_t i = t; i < n; i += 128) v += part[i * L + l];
+    s_sum[t] = v;
+    __syncthreads();
+    for (int o = 64; o > 0; o >>= 1) {
+        if (t < o) s_sum[t] += s_sum[t + o];
+        __syncthreads();
+    }
+    if (t == 0) alpha[l] += s_sum[0];
+}
+
 // FP32 forms of line_absorption.jl:140-161 (used to locate the widest layers)
 __device__ __forceinline__ float inverse_gaussian32(float rho, float sigma) {
     if (rho > 1.f / (2.5066282746f * sigma)) return 0.f;
@@ -282,26 +346,29 @@ struct LinePrep32 {
     float wlc, k_m, wl2c, grad, gstark, v1, abo_pre, vexp, invmu, t32;
     int32_t flags, sp, ki;     // flags: 1 molecule, 2 ABO broadening; ki: continuum knot interval
 };
-constexpr int PREP_WARPS = 8;
+constexpr int PREP_WARPS = 8;  // warps per block, at most
 
+// `lpw` lines per warp (at most 32): 32 lanes of per-line FP64 work where there are lines enough, fewer
+// for short lists, whose warps then spread over the SMs (one FP64 warp instruction takes 16 cycles of
+// an SM's pipe however few lanes are active, and phase B walks the warp's lines one by one).
 __global__ void __launch_bounds__(32 * PREP_WARPS) line_prep_mixed_kernel(LinesDev ln, LayersDev lay,
                                                                           const LayerConst* lc, CntmDev cn,
                                                                           const double* wls, int64_t nwl,
                                                                           double cutoff, PrepOut out,
-                                                                          const MathTables* math) {
+                                                                          const MathTables* math, int lpw) {
     __shared__ MathTables s_math;
     __shared__ LinePrep32 s_line[PREP_WARPS][32];
     extern __shared__ float s_dyn[];  // [warps][Lp] boundaries, [warps][Lp] class flags, [warps][Lp] cubic boundaries
     load_math_tables(s_math, math);
     __syncthreads();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int64_t base = (int64_t(blockIdx.x) * PREP_WARPS + wib) * 32;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int64_t base = (int64_t(blockIdx.x) * nwarps + wib) * lpw;
     if (base >= ln.n) return;
-    const int nl = int(min(int64_t(32), ln.n - base));
+    const int nl = int(min(int64_t(lpw), ln.n - base));
     const int L = lay.L, Lp = out.Lp;
     float* s_bnd = s_dyn + wib * Lp;
-    int* s_cls = reinterpret_cast<int*>(s_dyn + PREP_WARPS * Lp) + wib * Lp;
-    float* s_cub = s_dyn + 2 * PREP_WARPS * Lp + wib * Lp;
+    int* s_cls = reinterpret_cast<int*>(s_dyn + nwarps * Lp) + wib * Lp;
+    float* s_cub = s_dyn + 2 * nwarps * Lp + wib * Lp;
     // phase A: one lane per line
     KnotPos kp_mine{0, 0.0};
     if (lane < nl) {
@@ -441,9 +508,29 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) line_prep_mixed_kernel(LinesD
     }
 }
 
-// Launch geometry of line_prep_mixed_kernel for n lines.
-inline unsigned prep_mixed_blocks(int64_t n) { return unsigned((n + 32 * PREP_WARPS - 1) / (32 * PREP_WARPS)); }
-inline size_t prep_mixed_smem(int Lp) { return size_t(PREP_WARPS) * Lp * (2 * sizeof(float) + sizeof(int)); }
+// Launch geometry of the prologue kernels.  Up to about two warps per SM the FP64 work of a short list
+// is spread thin: fewer lines per warp (mixed), then fewer warps per block.  300 lines, mixed: 196 -> 55 us; lists
+// of 10,000 lines and more launch as before.
+constexpr int64_t PREP_SPREAD_WARPS = 304;
+inline int prep_block_warps(int64_t warps) {
+    return int(std::min<int64_t>(std::max<int64_t>(warps / PREP_SPREAD_WARPS, 1), PREP_WARPS));
+}
+struct PrepGeom {
+    int lpw, warps;  // lines per warp, warps per block
+    unsigned blocks;
+};
+inline PrepGeom prep_geom(int64_t n, bool mixed) {
+    PrepGeom g{mixed ? 4 : 1, 1, 0};
+    while (mixed && g.lpw < 32 && n > g.lpw * PREP_SPREAD_WARPS) g.lpw *= 2;
+    const int64_t w = (n + g.lpw - 1) / g.lpw;
+    g.warps = prep_block_warps(w);
+    g.blocks = unsigned((w + g.warps - 1) / g.warps);
+    return g;
+}
+// bytes of dynamic shared memory: boundaries and class flags, mixed also cubic boundaries
+inline size_t prep_smem(const PrepGeom& g, int Lp, bool mixed) {
+    return size_t(g.warps) * Lp * (sizeof(float) + sizeof(int) + (mixed ? sizeof(float) : 0));
+}
 
 // Candidate lists.  Lines are split by window half-width into tiers (at most 256, 4096, 65536
 // wavelength points, and wider).  Within a tier the lines keep list order, so their centre

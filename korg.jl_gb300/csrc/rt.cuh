@@ -25,6 +25,7 @@ struct RtArgs {
     const double* alpha_ref; // [L]
     const MathTables* math;
     CntmDev cn;              // nk > 0: also run the continuum-only transfer into cntm
+    const double* cseg;      // [nk - 1][CSEG_P] continuum flux series per knot interval (cntm_segment_kernel), or null
     double* flux;
     double* cntm;
     double unit;             // multiplies 2*pi*I (1e-8 in synthesize, src/synthesize.jl:315-318)
@@ -73,48 +74,207 @@ struct RtPass {
     }
 };
 
-__global__ void __launch_bounds__(128) rt_kernel(RtArgs a) {
+// ---- continuum-only transfer, once per knot interval
+// Between two continuum knots every layer's opacity is linear in wavelength, so each optical depth is
+// too, and the continuum flux is a smooth function of wavelength there, unless a layer's optical depth
+// crosses an end of the piecewise E2 (expint2_64), where the flux steps.  Each interval's flux is
+// evaluated at CSEG_P Chebyshev-Lobatto points, ends included; if every layer is on the same piece of
+// E2 at all of them (and so, linear as they are, in between) and nothing varies by more than CSEG_VAR,
+// the interval's flux is their Chebyshev series: with a variation of 2 % the next term is below
+// (0.01)^8 / 8 of the flux.  Other intervals are marked by a NaN, and their wavelengths transferred
+// one by one.  A grid of 0.01 A has 100 points per 1 A interval: 8 columns in the place of 100.
+constexpr int CSEG_P = 8;
+constexpr double CSEG_VAR = 0.02;
+// cos(pi i / 7), i = 0..7
+__device__ __constant__ double c_cos7[8] = {1.0, 0.9009688679024191, 0.6234898018587336, 0.22252093395631445, -0.22252093395631434, -0.6234898018587335, -0.900968867902419, -1.0};
+__device__ __forceinline__ double cos_pi7(int i) {
+    i %= 14;
+    return c_cos7[i <= 7 ? i : 14 - i];
+}
+
+// piece of expint2_64 that holds x
+__device__ __forceinline__ int expint2_piece(double x) {
+    return x == 0 ? 0 : 1 + (x >= 1.1) + (x >= 2.5) + (x >= 3.5) + (x >= 4.5) + (x >= 5.5) + (x >= 6.5) + (x >= 7.5) +
+                            (x >= 9);
+}
+
+struct RtLayers {  // per-layer constants in shared memory
+    double *fac, *hdl, *ikT;
+};
+__device__ __forceinline__ RtLayers rt_layers(const RtArgs& a, double* sh) {
+    const int L = a.L;
+    RtLayers y{sh, sh + L, sh + 2 * L};
+    for (int l = threadIdx.x; l < L; l += blockDim.x) {
+        y.fac[l] = a.tau_ref[l] / a.alpha_ref[l] * 1.0;  // RadiativeTransfer.jl:160
+        y.hdl[l] = l > 0 ? 0.5 * (log(a.tau_ref[l]) - log(a.tau_ref[l - 1])) : 0.0;  // :114, :250-251
+        y.ikT[l] = a.T ? 1.0 / (KBOLTZ_CGS * a.T[l]) : 0.0;
+    }
+    return y;
+}
+
+constexpr int CSEG_THREADS = 32;  // 4 intervals per block: a few thousand columns spread over the SMs
+__global__ void __launch_bounds__(CSEG_THREADS) cntm_segment_kernel(RtArgs a, double* cseg) {
+    extern __shared__ double s_rt[];
+    __shared__ MathTables s_math;
+    load_math_tables(s_math, a.math);
+    const RtLayers y = rt_layers(a, s_rt);
+    __syncthreads();
+    const int64_t k = int64_t(blockIdx.x) * (CSEG_THREADS / CSEG_P) + threadIdx.x / CSEG_P, nseg = a.cn.nk - 1;
+    const int m = threadIdx.x % CSEG_P;
+    const int64_t kk = min(k, nseg - 1);  // threads past the end repeat the last interval
+    const double w0 = a.cn.knots[kk], w1 = a.cn.knots[kk + 1];
+    const double t = m == 0 ? 0.0 : (m == CSEG_P - 1 ? 1.0 : 0.5 - 0.5 * cos_pi7(m));
+    const double wl = w0 + t * (w1 - w0);
+    const double pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl), hcw = HPLANCK_CGS * C_CGS / wl;
+    bool ok = true;
+    double S_prev = 0.0;
+    RtPass p{0.0, 0.0, -1.0, -1.0, 0.0, true};
+    for (int l = 0; l < a.L; l++) {
+        const double* v = a.cn.vals + int64_t(l) * a.cn.nk + kk;
+        const double v0 = v[0], v1 = v[1];
+        const double alpha = v0 * (1.0 - t) + v1 * t;
+        ok = ok && fabs(v1 - v0) <= CSEG_VAR * fmin(v0, v1) && (w1 - w0) * (hcw * y.ikT[l] + 5.0) <= CSEG_VAR * wl;
+        if (p.live) {
+            const double S = planck_t(pre, hcw, y.ikT[l], s_math);
+            if (l == 0)
+                p.ib_prev = alpha * y.fac[0];
+            else
+                p.step(alpha, y.fac[l], y.hdl[l], S - S_prev, 0.5 * S_prev, s_math);
+            S_prev = S;
+        }
+        // past TAU_STOP every path is on the last piece
+        const int piece = p.live ? expint2_piece(p.tau_prev) : expint2_piece(TAU_STOP);
+        const int first = __shfl_sync(0xffffffffu, piece, 0, CSEG_P);  // (every lane takes part)
+        ok = ok && first == piece;
+    }
+    double coef = 0.0;
+#pragma unroll
+    for (int q = 0; q < CSEG_P; q++) {
+        const double vq = __shfl_sync(0xffffffffu, p.I, q, CSEG_P);
+        coef = fma((q == 0 || q == CSEG_P - 1 ? 0.5 : 1.0) * vq, cos_pi7(m * q), coef);
+    }
+    coef *= (m == 0 || m == CSEG_P - 1 ? 1.0 : 2.0) / (CSEG_P - 1);
+    const unsigned grp = 0xffu << (threadIdx.x & 24);
+    ok = (__ballot_sync(0xffffffffu, ok) & grp) == grp;
+    if (k < nseg) cseg[k * CSEG_P + m] = ok ? coef : nan("");
+}
+
+// Planck function of every layer over a block's wavelengths as a Chebyshev series: PLANCK_P
+// evaluations per (layer, block) and PLANCK_P - 1 FMAs per (layer, wavelength) in the place of the
+// ~20 FP64 operations of planck_t.  Used where the block spans at most PLANCK_VAR of hc / (lambda kT)
+// in the exponent (half range): the next term is below PLANCK_VAR^6 / (2^5 6!) = 4e-17.
+constexpr int PLANCK_P = 6;
+constexpr double PLANCK_VAR = 0.01;
+// cos(pi i / 12), i = 0..6
+__device__ __constant__ double c_cos12[7] = {1.0, 0.9659258262890683, 0.8660254037844387, 0.7071067811865476, 0.5000000000000001, 0.25881904510252074, 0.0};
+__device__ __forceinline__ double cos_pi12(int i) {
+    i %= 24;
+    if (i > 12) i = 24 - i;
+    return i <= 6 ? c_cos12[i] : -c_cos12[12 - i];
+}
+
+// FP64 pipe bound (45 operations per pass, layer and wavelength); the Planck series and the continuum
+// intervals take the rest of it away.  BLK threads: 128, or 32 on short grids, whose columns then spread
+// over the SMs (one FP64 warp instruction takes 16 cycles of an SM's pipe).  Measured, both transfers:
+// 700,001 columns x 56 layers XXX -> XXX ms; 2,001 columns 294 -> XXX us.
+template <int BLK>
+__global__ void __launch_bounds__(BLK) rt_kernel(RtArgs a) {
     extern __shared__ double s_rt[];
     __shared__ MathTables s_math;
     load_math_tables(s_math, a.math);
     const int L = a.L;
-    double* s_fac = s_rt;           // tau_ref/alpha_ref * ds/dz (= 1)
-    double* s_hdl = s_rt + L;       // (log tau_ref[l] - log tau_ref[l-1]) / 2
-    double* s_ikT = s_rt + 2 * L;   // 1/(k T)
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-        s_fac[l] = a.tau_ref[l] / a.alpha_ref[l] * 1.0;  // RadiativeTransfer.jl:160
-        s_hdl[l] = l > 0 ? 0.5 * (log(a.tau_ref[l]) - log(a.tau_ref[l - 1])) : 0.0;  // :114, :250-251
-        s_ikT[l] = a.T ? 1.0 / (KBOLTZ_CGS * a.T[l]) : 0.0;
-    }
+    const RtLayers y = rt_layers(a, s_rt);
+    double* s_pl = s_rt + 3 * L;  // [L][PLANCK_P] Planck series
     __syncthreads();
-    const int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (j >= a.nwl) return;
+    const int64_t j0 = int64_t(blockIdx.x) * BLK, j = j0 + threadIdx.x;
     const bool two = a.cn.nk > 0;
+    bool series = false;
+    double T1 = 0.0;  // wavelength in [-1, 1] over the block
+    if (!a.S) {  // uniform
+        const double wa = a.wls[j0], hw = 0.5 * (a.wls[min(j0 + BLK, a.nwl) - 1] - wa);
+        double xmax = 0.0;
+        for (int l = 0; l < L; l++) xmax = fmax(xmax, y.ikT[l]);
+        series = hw * (HPLANCK_CGS * C_CGS / wa * xmax + 5.0) <= PLANCK_VAR * wa;
+        if (series) {
+            for (int e = threadIdx.x; e < L * PLANCK_P; e += BLK) {
+                const int l = e / PLANCK_P, m = e - l * PLANCK_P;
+                const double w = wa + (hw + hw * cos_pi12(2 * m + 1));
+                s_pl[e] = planck_t(2 * HPLANCK_CGS * (C_CGS * C_CGS) / (w * w * w * w * w), HPLANCK_CGS * C_CGS / w,
+                                   y.ikT[l], s_math);
+            }
+            __syncthreads();
+            for (int l = threadIdx.x; l < L; l += BLK) {
+                double v[PLANCK_P], c[PLANCK_P];
+#pragma unroll
+                for (int m = 0; m < PLANCK_P; m++) v[m] = s_pl[l * PLANCK_P + m];
+#pragma unroll
+                for (int n = 0; n < PLANCK_P; n++) {
+                    c[n] = 0.0;
+#pragma unroll
+                    for (int m = 0; m < PLANCK_P; m++) c[n] = fma(v[m], cos_pi12(n * (2 * m + 1)), c[n]);
+                    c[n] *= (n == 0 ? 1.0 : 2.0) / PLANCK_P;
+                }
+                // to powers of the normalised wavelength: T2 = 2u^2 - 1, ..., T5 = 16u^5 - 20u^3 + 5u
+                double* d = s_pl + l * PLANCK_P;
+                d[0] = c[0] - c[2] + c[4];
+                d[1] = c[1] - 3 * c[3] + 5 * c[5];
+                d[2] = 2 * c[2] - 8 * c[4];
+                d[3] = 4 * c[3] - 20 * c[5];
+                d[4] = 8 * c[4];
+                d[5] = 16 * c[5];
+            }
+            __syncthreads();
+            T1 = hw > 0 && j < a.nwl ? ((a.wls[j] - wa) - hw) / hw : 0.0;
+        }
+    }
+    if (j >= a.nwl) return;
     double pre = 0, hcw = 0;
     KnotPos kp{0, 0.0};
-    if (!a.S || two) {
+    bool each = two;  // this wavelength's continuum transfer runs in the layer loop
+    if ((!a.S && !series) || two) {
         const double wl = a.wls[j];
         pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl);
         hcw = HPLANCK_CGS * C_CGS / wl;
-        if (two) kp = knot_pos(a.cn.knots, a.cn.nk, wl);
+        if (two) {
+            kp = knot_pos(a.cn.knots, a.cn.nk, wl);
+            const double* cs = a.cseg ? a.cseg + kp.i * CSEG_P : nullptr;
+            if (cs && kp.t >= 0.0 && kp.t <= 1.0 && cs[0] == cs[0]) {
+                const double u = 1.0 - 2.0 * kp.t;  // node m of the interval lies at t = (1 - cos(pi m / 7)) / 2
+                double t0 = 1.0, t1 = u, v = cs[0];
+#pragma unroll
+                for (int n = 1; n < CSEG_P; n++) {
+                    v = fma(cs[n], t1, v);
+                    const double t2 = fma(2 * u, t1, -t0);
+                    t0 = t1;
+                    t1 = t2;
+                }
+                a.cntm[j] = 2 * PI * (v * 1.0) * a.unit;
+                each = false;
+            }
+        }
     }
+    auto source = [&](int l) {
+        if (!series) return planck_t(pre, hcw, y.ikT[l], s_math);
+        const double* d = s_pl + l * PLANCK_P;
+        return fma(fma(fma(fma(fma(d[5], T1, d[4]), T1, d[3]), T1, d[2]), T1, d[1]), T1, d[0]);
+    };
     const double* al = a.alpha + j * L;
     const double* Sc = a.S ? a.S + j * L : nullptr;
 
     // layer 0: tau = 0, E2(0) = 1, exp(0) = 1, so G = -1 and H = -1
-    double S_prev = Sc ? Sc[0] : planck_t(pre, hcw, s_ikT[0], s_math);
-    RtPass full{al[0] * s_fac[0], 0.0, -1.0, -1.0, 0.0, true};
-    RtPass cont{two ? knot_eval(a.cn.vals, a.cn.nk, kp) * s_fac[0] : 0.0, 0.0, -1.0, -1.0, 0.0, two};
+    double S_prev = Sc ? Sc[0] : source(0);
+    RtPass full{al[0] * y.fac[0], 0.0, -1.0, -1.0, 0.0, true};
+    RtPass cont{each ? knot_eval(a.cn.vals, a.cn.nk, kp) * y.fac[0] : 0.0, 0.0, -1.0, -1.0, 0.0, each};
     for (int l = 1; l < L && (full.live || cont.live); l++) {
-        const double S = Sc ? Sc[l] : planck_t(pre, hcw, s_ikT[l], s_math);
-        const double hdl = s_hdl[l], dS = S - S_prev, half_Sp = 0.5 * S_prev;
-        if (full.live) full.step(al[l], s_fac[l], hdl, dS, half_Sp, s_math);
+        const double S = Sc ? Sc[l] : source(l);
+        const double hdl = y.hdl[l], dS = S - S_prev, half_Sp = 0.5 * S_prev;
+        if (full.live) full.step(al[l], y.fac[l], hdl, dS, half_Sp, s_math);
         if (cont.live)
-            cont.step(knot_eval(a.cn.vals + int64_t(l) * a.cn.nk, a.cn.nk, kp), s_fac[l], hdl, dS, half_Sp, s_math);
+            cont.step(knot_eval(a.cn.vals + int64_t(l) * a.cn.nk, a.cn.nk, kp), y.fac[l], hdl, dS, half_Sp, s_math);
         S_prev = S;
     }
     a.flux[j] = 2 * PI * (full.I * 1.0) * a.unit;  // :136
-    if (two) a.cntm[j] = 2 * PI * (cont.I * 1.0) * a.unit;
+    if (each) a.cntm[j] = 2 * PI * (cont.I * 1.0) * a.unit;
 }
 
 // alpha[j][l] = continuum interpolant of layer l at wl_j (src/synthesize.jl:226-252)
