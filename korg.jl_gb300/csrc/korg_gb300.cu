@@ -56,7 +56,7 @@ struct korg_ctx {
     cudaStream_t stream = nullptr;  // used by the host-pointer calls and for graph capture
     std::string err;
     // scratch arena: grown on demand, never shrunk, freed by korg_destroy
-    DevBuf lines_scratch, ref_part, counters, tune_alpha;
+    DevBuf lines_scratch, ref_part, cseg, counters, tune_alpha;
     DevBuf hrec, hQ, hQ32, hulb, huub;
     DevBuf stage_dev, aref, alpha, flux, cntm, math;
     DevBuf vjp_g, vjp_dpar, vjp_small, vjp_hder, vjp_hdq;  // reverse mode
@@ -579,9 +579,21 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
 int run_rt(korg_ctx* ctx, const double* alpha, const double* S, const double* T, const double* wls, int64_t nwl,
            int L, const double* tau_ref, const double* alpha_ref, CntmDev cn, double* flux, double* cntm,
            double unit, cudaStream_t s) {
-    RtArgs ra{alpha, S, T, wls, nwl, L, tau_ref, alpha_ref, static_cast<MathTables*>(ctx->math.p), cn, flux, cntm, unit};
-    const unsigned blocks = unsigned((nwl + 127) / 128);
-    rt_kernel<<<blocks, 128, sizeof(double) * 3 * L, s>>>(ra);
+    RtArgs ra{alpha, S, T, wls, nwl, L, tau_ref, alpha_ref, static_cast<MathTables*>(ctx->math.p), cn, nullptr, flux,
+              cntm, unit};
+    // continuum transfer per knot interval (8 columns each) where that at least halves the columns
+    if (cn.nk >= 2 && nwl >= 2 * CSEG_P * (cn.nk - 1)) {
+        KCHECK(ensure(ctx, ctx->cseg, sizeof(double) * CSEG_P * size_t(cn.nk - 1)));
+        double* cseg = static_cast<double*>(ctx->cseg.p);
+        const unsigned blocks = unsigned(std::min<int64_t>(cn.nk - 1, int64_t(ctx->sms) * 6));
+        cntm_segment_kernel<<<blocks, 32 * CSEG_P, (sizeof(double) * 3 + CSEG_P) * size_t(L), s>>>(ra, cseg);
+        KCUDA(cudaGetLastError());
+        ra.cseg = cseg;
+    }
+    if (nwl <= RT_WARP_COLS)
+        rt_warp_kernel<<<unsigned((nwl + RT_WARPS - 1) / RT_WARPS), 32 * RT_WARPS, sizeof(double) * 3 * L, s>>>(ra);
+    else
+        rt_kernel<<<unsigned((nwl + RT_BLK - 1) / RT_BLK), RT_BLK, sizeof(double) * (3 + PLANCK_P) * L, s>>>(ra);
     KCUDA(cudaGetLastError());
     return KORG_OK;
 }
@@ -1282,7 +1294,7 @@ KORG_API void korg_destroy(korg_ctx* ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     drop_graph(ctx);
-    DevBuf* bufs[] = {&ctx->lines_scratch, &ctx->ref_part, &ctx->counters, &ctx->tune_alpha, &ctx->hrec, &ctx->hQ, &ctx->hQ32,
+    DevBuf* bufs[] = {&ctx->lines_scratch, &ctx->ref_part, &ctx->cseg, &ctx->counters, &ctx->tune_alpha, &ctx->hrec, &ctx->hQ, &ctx->hQ32,
                       &ctx->hulb, &ctx->huub, &ctx->stage_dev, &ctx->aref, &ctx->alpha, &ctx->flux, &ctx->cntm,
                       &ctx->math, &ctx->b_alpha, &ctx->b_lines, &ctx->b_meta, &ctx->vjp_g, &ctx->vjp_dpar,
                       &ctx->vjp_small, &ctx->vjp_hder, &ctx->vjp_hdq, &ctx->mx_layers};

@@ -112,51 +112,146 @@ __device__ __forceinline__ RtLayers rt_layers(const RtArgs& a, double* sh) {
     return y;
 }
 
-constexpr int CSEG_THREADS = 32;  // 4 intervals per block: a few thousand columns spread over the SMs
-__global__ void __launch_bounds__(CSEG_THREADS) cntm_segment_kernel(RtArgs a, double* cseg) {
+// expint2_ex with its seven middle pieces as rows of a table (centre, six coefficients; the same operations
+// in the same order): lanes of a warp at different optical depths then share one path.
+constexpr int E2_ROW = 7;
+__device__ __constant__ double c_e2_mid[7 * E2_ROW] = {
+    2, 0.037534261820486914, -0.04890051070806112, 0.033833820809153176, -0.016916910404576574, 0.007048712668573576,
+    -0.0026785108140579598,
+    3, 0.010641925085272673, -0.013048381094197039, 0.008297844727977323, -0.003687930990212144, 0.0013061422257001345,
+    -0.0003995258572729822,
+    4, 0.0031982292493385146, -0.0037793524098489054, 0.0022894548610917728, -0.0009539395254549051,
+    0.00031003034577284415, -8.466213288412284e-5,
+    5, 0.000996469042708825, -0.0011482955912753257, 0.0006737946999085467, -0.00026951787996341863,
+    8.310134632205409e-5, -2.1202073223788938e-5,
+    6, 0.0003182574636904001, -0.0003600824521626587, 0.00020656268138886323, -8.032993165122457e-5,
+    2.390771775334065e-5, -5.8334831318151185e-6,
+    7, 0.00010350984428214624, -0.00011548173161033826, 6.513442611103688e-5, -2.4813114708966427e-5,
+    7.200234178941151e-6, -1.7027366981408086e-6,
+    8, 3.413764515111217e-5, -3.76656228439249e-5, 2.096641424390699e-5, -7.862405341465122e-6, 2.2386015208338193e-6,
+    -5.173353514609864e-7};
+__device__ __forceinline__ double expint2_lanes(double x, double ex, const double* mid, const MathTables& t) {
+    if (x >= 1.1 && x < 9) {
+        const double* r = mid + E2_ROW * (expint2_piece(x) - 2);
+        x -= r[0];
+        return r[1] + (r[2] + (r[3] + (r[4] + (r[5] + r[6] * x) * x) * x) * x) * x;
+    }
+    return expint2_ex(x, ex, t);
+}
+
+// One column by one warp, lanes over layers (RtPass's recursion with a prefix sum of the optical depth):
+// for grids too short to fill the GPU with one thread per column, whose serial chain of 100 dependent
+// FP64 operations a layer takes 3 us a layer.  visit(l, tau) is called for every layer (valid lanes).
+template <class Alpha, class Source, class Visit>
+__device__ __forceinline__ double rt_column_warp(int L, const RtLayers& y, const MathTables& mt, const double* e2_mid,
+                                                 Alpha alpha, Source source, Visit visit) {
+    const int lane = threadIdx.x & 31;
+    double I = 0.0, c_ib = 0.0, c_S = 0.0, c_tau = 0.0, c_G = -1.0, c_H = -1.0;  // the layer before the chunk
+    for (int l0 = 0; l0 < L; l0 += 32) {
+        const int l = l0 + lane;
+        const bool in = l < L;
+        const double ib = in ? alpha(l) * y.fac[l] : 0.0, S = in ? source(l) : 0.0;
+        double ibp = __shfl_up_sync(0xffffffffu, ib, 1), Sp = __shfl_up_sync(0xffffffffu, S, 1);
+        if (lane == 0) {
+            ibp = c_ib;
+            Sp = c_S;
+        }
+        const double dtau = in && l > 0 ? (ib + ibp) * y.hdl[l] : 0.0;  // RadiativeTransfer.jl:250-251
+        double tau = dtau;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double v = __shfl_up_sync(0xffffffffu, tau, o);
+            if (lane >= o) tau += v;
+        }
+        tau += c_tau;
+        double taup = __shfl_up_sync(0xffffffffu, tau, 1);
+        if (lane == 0) taup = c_tau;
+        if (in) visit(l, tau);
+        const double ex = fexp64(-tau, mt), e2 = expint2_lanes(tau, ex, e2_mid, mt);
+        const double G = fma(tau, e2, -ex), H = fma(tau, G, -ex);
+        double Gp = __shfl_up_sync(0xffffffffu, G, 1), Hp = __shfl_up_sync(0xffffffffu, H, 1);
+        if (lane == 0) {
+            Gp = c_G;
+            Hp = c_H;
+        }
+        if (in && l > 0 && taup <= TAU_STOP) {
+            const double m = (S - Sp) * recip64(dtau), dG = G - Gp, dH = H - Hp;  // :382-385
+            I = fma(0.5 * Sp, dG, I);
+            I = fma(m, fma(-0.5 * taup, dG, dH * (1.0 / 3.0)), I);
+        }
+        c_ib = __shfl_sync(0xffffffffu, ib, 31);
+        c_S = __shfl_sync(0xffffffffu, S, 31);
+        c_tau = __shfl_sync(0xffffffffu, tau, 31);
+        c_G = __shfl_sync(0xffffffffu, G, 31);
+        c_H = __shfl_sync(0xffffffffu, H, 31);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) I += __shfl_xor_sync(0xffffffffu, I, o);
+    return I;
+}
+
+// one block per interval at a time, one warp per node
+__global__ void __launch_bounds__(32 * CSEG_P) cntm_segment_kernel(RtArgs a, double* cseg) {
     extern __shared__ double s_rt[];
     __shared__ MathTables s_math;
+    __shared__ double s_I[CSEG_P], s_e2[7 * E2_ROW];
     load_math_tables(s_math, a.math);
+    if (threadIdx.x < 7 * E2_ROW) s_e2[threadIdx.x] = c_e2_mid[threadIdx.x];
     const RtLayers y = rt_layers(a, s_rt);
+    unsigned char* s_piece = reinterpret_cast<unsigned char*>(s_rt + 3 * a.L);  // [CSEG_P][L]
     __syncthreads();
-    const int64_t k = int64_t(blockIdx.x) * (CSEG_THREADS / CSEG_P) + threadIdx.x / CSEG_P, nseg = a.cn.nk - 1;
-    const int m = threadIdx.x % CSEG_P;
-    const int64_t kk = min(k, nseg - 1);  // threads past the end repeat the last interval
-    const double w0 = a.cn.knots[kk], w1 = a.cn.knots[kk + 1];
-    const double t = m == 0 ? 0.0 : (m == CSEG_P - 1 ? 1.0 : 0.5 - 0.5 * cos_pi7(m));
-    const double wl = w0 + t * (w1 - w0);
-    const double pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl), hcw = HPLANCK_CGS * C_CGS / wl;
-    bool ok = true;
-    double S_prev = 0.0;
-    RtPass p{0.0, 0.0, -1.0, -1.0, 0.0, true};
-    for (int l = 0; l < a.L; l++) {
-        const double* v = a.cn.vals + int64_t(l) * a.cn.nk + kk;
-        const double v0 = v[0], v1 = v[1];
-        const double alpha = v0 * (1.0 - t) + v1 * t;
-        ok = ok && fabs(v1 - v0) <= CSEG_VAR * fmin(v0, v1) && (w1 - w0) * (hcw * y.ikT[l] + 5.0) <= CSEG_VAR * wl;
-        if (p.live) {
-            const double S = planck_t(pre, hcw, y.ikT[l], s_math);
-            if (l == 0)
-                p.ib_prev = alpha * y.fac[0];
-            else
-                p.step(alpha, y.fac[l], y.hdl[l], S - S_prev, 0.5 * S_prev, s_math);
-            S_prev = S;
+    const int m = threadIdx.x >> 5;  // this warp's node
+    for (int64_t k = blockIdx.x; k < a.cn.nk - 1; k += gridDim.x) {
+        const double w0 = a.cn.knots[k], w1 = a.cn.knots[k + 1];
+        const double t = m == 0 ? 0.0 : (m == CSEG_P - 1 ? 1.0 : 0.5 - 0.5 * cos_pi7(m));
+        const double wl = w0 + t * (w1 - w0);
+        const double pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl), hcw = HPLANCK_CGS * C_CGS / wl;
+        int ok = 1;
+        const double I = rt_column_warp(
+            a.L, y, s_math, s_e2,
+            [&](int l) {
+                const double* v = a.cn.vals + int64_t(l) * a.cn.nk + k;
+                const double v0 = v[0], v1 = v[1];
+                if (!(fabs(v1 - v0) <= CSEG_VAR * fmin(v0, v1))) ok = 0;
+                return v0 * (1.0 - t) + v1 * t;
+            },
+            [&](int l) {
+                if (!((w1 - w0) * (hcw * y.ikT[l] + 5.0) <= CSEG_VAR * wl)) ok = 0;
+                return planck_t(pre, hcw, y.ikT[l], s_math);
+            },
+            // past TAU_STOP every path is on the last piece
+            [&](int l, double tau) { s_piece[m * a.L + l] = (unsigned char)(expint2_piece(fmin(tau, TAU_STOP))); });
+        if ((threadIdx.x & 31) == 0) s_I[m] = I;
+        __syncthreads();
+        for (int e = threadIdx.x; e < (CSEG_P - 1) * a.L; e += blockDim.x)
+            if (s_piece[e] != s_piece[e + a.L]) ok = 0;  // node by node against the next
+        ok = __syncthreads_and(ok);
+        if (threadIdx.x < CSEG_P) {
+            const int n = threadIdx.x;
+            double coef = 0.0;
+            for (int q = 0; q < CSEG_P; q++)
+                coef = fma((q == 0 || q == CSEG_P - 1 ? 0.5 : 1.0) * s_I[q], cos_pi7(n * q), coef);
+            coef *= (n == 0 || n == CSEG_P - 1 ? 1.0 : 2.0) / (CSEG_P - 1);
+            cseg[k * CSEG_P + n] = ok ? coef : nan("");
         }
-        // past TAU_STOP every path is on the last piece
-        const int piece = p.live ? expint2_piece(p.tau_prev) : expint2_piece(TAU_STOP);
-        const int first = __shfl_sync(0xffffffffu, piece, 0, CSEG_P);  // (every lane takes part)
-        ok = ok && first == piece;
+        __syncthreads();  // s_I and s_piece are rewritten for the next interval
     }
-    double coef = 0.0;
+}
+
+// continuum flux (without 2 pi and unit) at an interval's position t from its series, or NaN
+__device__ __forceinline__ double cntm_series(const double* cseg, const KnotPos& kp) {
+    if (!cseg || !(kp.t >= 0.0 && kp.t <= 1.0)) return nan("");
+    const double* cs = cseg + kp.i * CSEG_P;
+    const double u = 1.0 - 2.0 * kp.t;  // node m of the interval lies at t = (1 - cos(pi m / 7)) / 2
+    double t0 = 1.0, t1 = u, v = cs[0];
 #pragma unroll
-    for (int q = 0; q < CSEG_P; q++) {
-        const double vq = __shfl_sync(0xffffffffu, p.I, q, CSEG_P);
-        coef = fma((q == 0 || q == CSEG_P - 1 ? 0.5 : 1.0) * vq, cos_pi7(m * q), coef);
+    for (int n = 1; n < CSEG_P; n++) {
+        v = fma(cs[n], t1, v);
+        const double t2 = fma(2 * u, t1, -t0);
+        t0 = t1;
+        t1 = t2;
     }
-    coef *= (m == 0 || m == CSEG_P - 1 ? 1.0 : 2.0) / (CSEG_P - 1);
-    const unsigned grp = 0xffu << (threadIdx.x & 24);
-    ok = (__ballot_sync(0xffffffffu, ok) & grp) == grp;
-    if (k < nseg) cseg[k * CSEG_P + m] = ok ? coef : nan("");
+    return v;
 }
 
 // Planck function of every layer over a block's wavelengths as a Chebyshev series: PLANCK_P
@@ -173,12 +268,11 @@ __device__ __forceinline__ double cos_pi12(int i) {
     return i <= 6 ? c_cos12[i] : -c_cos12[12 - i];
 }
 
-// FP64 pipe bound (45 operations per pass, layer and wavelength); the Planck series and the continuum
-// intervals take the rest of it away.  BLK threads: 128, or 32 on short grids, whose columns then spread
-// over the SMs (one FP64 warp instruction takes 16 cycles of an SM's pipe).  Measured, both transfers:
-// 700,001 columns x 56 layers XXX -> XXX ms; 2,001 columns 294 -> XXX us.
-template <int BLK>
-__global__ void __launch_bounds__(BLK) rt_kernel(RtArgs a) {
+// One thread per column.  FP64 pipe bound (45 operations per pass, layer and wavelength); the Planck
+// series and the continuum intervals take the rest of it away.  Both transfers of 700,001 columns x 56
+// layers: 8.11 -> 3.86 ms, and 0.5 for the intervals.
+constexpr int RT_BLK = 128;
+__global__ void __launch_bounds__(RT_BLK) rt_kernel(RtArgs a) {
     extern __shared__ double s_rt[];
     __shared__ MathTables s_math;
     load_math_tables(s_math, a.math);
@@ -186,24 +280,24 @@ __global__ void __launch_bounds__(BLK) rt_kernel(RtArgs a) {
     const RtLayers y = rt_layers(a, s_rt);
     double* s_pl = s_rt + 3 * L;  // [L][PLANCK_P] Planck series
     __syncthreads();
-    const int64_t j0 = int64_t(blockIdx.x) * BLK, j = j0 + threadIdx.x;
+    const int64_t j0 = int64_t(blockIdx.x) * RT_BLK, j = j0 + threadIdx.x;
     const bool two = a.cn.nk > 0;
     bool series = false;
     double T1 = 0.0;  // wavelength in [-1, 1] over the block
     if (!a.S) {  // uniform
-        const double wa = a.wls[j0], hw = 0.5 * (a.wls[min(j0 + BLK, a.nwl) - 1] - wa);
+        const double wa = a.wls[j0], hw = 0.5 * (a.wls[min(j0 + RT_BLK, a.nwl) - 1] - wa);
         double xmax = 0.0;
         for (int l = 0; l < L; l++) xmax = fmax(xmax, y.ikT[l]);
         series = hw * (HPLANCK_CGS * C_CGS / wa * xmax + 5.0) <= PLANCK_VAR * wa;
         if (series) {
-            for (int e = threadIdx.x; e < L * PLANCK_P; e += BLK) {
+            for (int e = threadIdx.x; e < L * PLANCK_P; e += RT_BLK) {
                 const int l = e / PLANCK_P, m = e - l * PLANCK_P;
                 const double w = wa + (hw + hw * cos_pi12(2 * m + 1));
                 s_pl[e] = planck_t(2 * HPLANCK_CGS * (C_CGS * C_CGS) / (w * w * w * w * w), HPLANCK_CGS * C_CGS / w,
                                    y.ikT[l], s_math);
             }
             __syncthreads();
-            for (int l = threadIdx.x; l < L; l += BLK) {
+            for (int l = threadIdx.x; l < L; l += RT_BLK) {
                 double v[PLANCK_P], c[PLANCK_P];
 #pragma unroll
                 for (int m = 0; m < PLANCK_P; m++) v[m] = s_pl[l * PLANCK_P + m];
@@ -237,17 +331,8 @@ __global__ void __launch_bounds__(BLK) rt_kernel(RtArgs a) {
         hcw = HPLANCK_CGS * C_CGS / wl;
         if (two) {
             kp = knot_pos(a.cn.knots, a.cn.nk, wl);
-            const double* cs = a.cseg ? a.cseg + kp.i * CSEG_P : nullptr;
-            if (cs && kp.t >= 0.0 && kp.t <= 1.0 && cs[0] == cs[0]) {
-                const double u = 1.0 - 2.0 * kp.t;  // node m of the interval lies at t = (1 - cos(pi m / 7)) / 2
-                double t0 = 1.0, t1 = u, v = cs[0];
-#pragma unroll
-                for (int n = 1; n < CSEG_P; n++) {
-                    v = fma(cs[n], t1, v);
-                    const double t2 = fma(2 * u, t1, -t0);
-                    t0 = t1;
-                    t1 = t2;
-                }
+            const double v = cntm_series(a.cseg, kp);
+            if (v == v) {
                 a.cntm[j] = 2 * PI * (v * 1.0) * a.unit;
                 each = false;
             }
@@ -277,24 +362,61 @@ __global__ void __launch_bounds__(BLK) rt_kernel(RtArgs a) {
     if (each) a.cntm[j] = 2 * PI * (cont.I * 1.0) * a.unit;
 }
 
+// One warp per column: grids of at most RT_WARP_COLS columns, where one thread per column is bound by its
+// serial chain (180 us for 56 layers at any size; 2,001 columns 46 us here).
+constexpr int64_t RT_WARP_COLS = 16384;
+constexpr int RT_WARPS = 4;
+__global__ void __launch_bounds__(32 * RT_WARPS) rt_warp_kernel(RtArgs a) {
+    extern __shared__ double s_rt[];
+    __shared__ MathTables s_math;
+    __shared__ double s_e2[7 * E2_ROW];
+    load_math_tables(s_math, a.math);
+    if (threadIdx.x < 7 * E2_ROW) s_e2[threadIdx.x] = c_e2_mid[threadIdx.x];
+    const RtLayers y = rt_layers(a, s_rt);
+    __syncthreads();
+    const int64_t j = int64_t(blockIdx.x) * RT_WARPS + (threadIdx.x >> 5);
+    if (j >= a.nwl) return;  // uniform across the warp
+    const int lane = threadIdx.x & 31, L = a.L;
+    const bool two = a.cn.nk > 0;
+    double pre = 0, hcw = 0;
+    if (!a.S || two) {
+        const double wl = a.wls[j];
+        pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl);
+        hcw = HPLANCK_CGS * C_CGS / wl;
+    }
+    const double *al = a.alpha + j * L, *Sc = a.S ? a.S + j * L : nullptr;
+    auto source = [&](int l) { return Sc ? Sc[l] : planck_t(pre, hcw, y.ikT[l], s_math); };
+    auto nothing = [](int, double) {};
+    const double F = rt_column_warp(L, y, s_math, s_e2, [&](int l) { return al[l]; }, source, nothing);
+    if (lane == 0) a.flux[j] = 2 * PI * (F * 1.0) * a.unit;  // :136
+    if (!two) return;
+    const KnotPos kp = knot_pos(a.cn.knots, a.cn.nk, a.wls[j]);
+    double C = cntm_series(a.cseg, kp);
+    if (!(C == C))
+        C = rt_column_warp(
+            L, y, s_math, s_e2, [&](int l) { return knot_eval(a.cn.vals + int64_t(l) * a.cn.nk, a.cn.nk, kp); }, source, nothing);
+    if (lane == 0) a.cntm[j] = 2 * PI * (C * 1.0) * a.unit;
+}
+
 // alpha[j][l] = continuum interpolant of layer l at wl_j (src/synthesize.jl:226-252)
 __global__ void __launch_bounds__(256) alpha_init_kernel(double* alpha, const double* wls, int64_t nwl, int32_t L,
                                                          CntmDev cn) {
     __shared__ int64_t s_i[64];
-    __shared__ double s_t[64];
+    __shared__ double s_t[64], s_u[64];
     const int64_t j0 = int64_t(blockIdx.x) * 64;
     const int64_t jn = min(int64_t(64), nwl - j0);
     if (threadIdx.x < jn) {
         const KnotPos p = knot_pos(cn.knots, cn.nk, wls[j0 + threadIdx.x]);
         s_i[threadIdx.x] = p.i;
         s_t[threadIdx.x] = p.t;
+        s_u[threadIdx.x] = 1.0 - p.t;
     }
     __syncthreads();
     const int64_t n = jn * L;
     for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
         const int jj = int(e / L), l = int(e % L);
-        const KnotPos p{s_i[jj], s_t[jj]};
-        alpha[j0 * L + e] = knot_eval(cn.vals + int64_t(l) * cn.nk, cn.nk, p);
+        const double* v = cn.vals + int64_t(l) * cn.nk + s_i[jj];
+        alpha[j0 * L + e] = cn.nk == 1 ? v[0] : fma(v[1], s_t[jj], v[0] * s_u[jj]);  // knot_eval, two operations
     }
 }
 
