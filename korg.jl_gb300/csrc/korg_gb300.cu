@@ -2271,6 +2271,12 @@ int rot_args(korg_ctx* ctx, const double* wls, int64_t nwl, const korg_wl_range*
     a->c3 = PI * (1 - eps / 3);
     return KORG_OK;
 }
+// blocks of ROT_TP points that do not straddle ranges
+unsigned rot_blocks(const RotArgs& a) {
+    int64_t n = 0;
+    for (int k = 0; k < a.nranges; k++) n += (a.r[k].n + ROT_TP - 1) / ROT_TP;
+    return unsigned(n);
+}
 __global__ void add_kernel(double* dst, const double* src, int64_t n) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) dst[i] += src[i];
@@ -2344,7 +2350,12 @@ KORG_API int korg_apply_rotation_dev(korg_ctx* ctx, const double* wls, int64_t n
         KCUDA(cudaMemcpyAsync(out, flux, sizeof(double) * size_t(nwl) * nspec, cudaMemcpyDeviceToDevice, s));
         return KORG_OK;
     }
-    rotation_fwd_kernel<<<unsigned((nwl + ROT_TP - 1) / ROT_TP), ROT_TP, 0, s>>>(a, flux, nspec, out);
+    const auto go = [&](auto kern, int ns) {
+        kern<<<dim3(rot_blocks(a), unsigned((nspec + ns - 1) / ns)), ROT_TP, 0, s>>>(a, flux, nspec, out);
+    };
+    if (nspec > 4) go(rotation_fwd_kernel<16>, 16);
+    else if (nspec > 1) go(rotation_fwd_kernel<4>, 4);
+    else go(rotation_fwd_kernel<1>, 1);
     KCUDA(cudaGetLastError());
     return KORG_OK;
 }
@@ -2362,8 +2373,12 @@ KORG_API int korg_apply_rotation_vjp_dev(korg_ctx* ctx, const double* wls, int64
         const int64_t n = nwl * nspec;
         add_kernel<<<unsigned((n + 255) / 256), 256, 0, s>>>(dflux, dout, n);
     } else {
-        rotation_vjp_kernel<<<dim3(unsigned((nwl + 127) / 128), unsigned((nspec + ROT_SPEC - 1) / ROT_SPEC)), 128, 0,
-                              s>>>(a, dout, nspec, dflux);
+        const auto go = [&](auto kern, int ns) {
+            kern<<<dim3(rot_blocks(a), unsigned((nspec + ns - 1) / ns)), ROT_TP, 0, s>>>(a, dout, nspec, dflux);
+        };
+        if (nspec > 4) go(rotation_vjp_kernel<16>, 16);
+        else if (nspec > 1) go(rotation_vjp_kernel<4>, 4);
+        else go(rotation_vjp_kernel<1>, 1);
     }
     KCUDA(cudaGetLastError());
     return KORG_OK;
