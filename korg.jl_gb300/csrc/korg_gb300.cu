@@ -2030,7 +2030,16 @@ KORG_API int korg_radiative_transfer_general(korg_ctx* ctx, const double* alpha,
                  (double*)(b + o_rf), (double*)(b + o_rl), (double*)(b + o_rp), (double*)(b + o_w), tau_scheme,
                  I_scheme, static_cast<MathTables*>(ctx->math.p), (double*)(b + o_f),
                  I_surface ? (double*)(b + o_i) : nullptr};
-    rt_general_kernel<<<unsigned((nwl + 127) / 128), 128, 0, ctx->stream>>>(ra);
+    // inward ray r seeds outward ray r: the one-pass kernel takes them when they are the same ray
+    bool paired = tau_scheme == 0 && I_scheme <= 1;
+    for (int r = 0; r < n_in; r++) paired = paired && in_idx[r] == r;
+    if (paired) {
+        const size_t smem = rt_rays_smem(L, n_mu);
+        KCUDA(cudaFuncSetAttribute(rt_rays_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        rt_rays_kernel<<<unsigned((nwl + 31) / 32), 32 * RAY_WARPS, smem, ctx->stream>>>(ra);
+    } else {
+        rt_general_kernel<<<unsigned((nwl + 127) / 128), 128, 0, ctx->stream>>>(ra);
+    }
     KCUDA(cudaGetLastError());
     KCUDA(cudaMemcpyAsync(flux, b + o_f, 8 * size_t(nwl), cudaMemcpyDeviceToHost, ctx->stream));
     if (I_surface)

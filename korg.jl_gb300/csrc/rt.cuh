@@ -558,4 +558,75 @@ __global__ void __launch_bounds__(128) rt_general_kernel(RtGenArgs a) {
     a.flux[j] = 2 * PI * F;
 }
 
+// Rays with anchored optical depth and the linear formal solution (I_scheme 0) or its flux-only form (1):
+// along a segment of optical depth d with source slope m = (S_deep - S_shallow) / d both give
+//   outward  I += T [(S_shallow + m) - e^-d (S_deep + m)],  T = product of e^-d from the surface,
+//   inward   I  = I e^-d + (S_deep - m) - e^-d (S_shallow - m)
+// (they differ where d = 0: the flux-only form divides by 1), so one pass from the surface down serves an
+// outward ray and the inward ray that seeds it (RadiativeTransfer.jl:196-198: the outward ray gets T times
+// what the inward ray brings to the deepest layer), without arrays per thread.  A ray ends where T < 1e-27:
+// what lies below contributes less than that much of the largest source function.
+// A block stages 32 columns in shared memory (coalesced loads, read once, transposed); its warps share the
+// rays, lanes hold columns.  FP64 pipe bound, 27 operations per (ray, layer, column): 20,001 columns, 20
+// rays, 56 layers, the whole call 3.37 -> 2.04 ms (kernel 2.5 ms before: four arrays of 128 doubles per
+// thread in local memory).
+constexpr int RAY_WARPS = 8;
+constexpr double RAY_STOP = 1e-27;
+inline size_t rt_rays_smem(int L, int n_mu) { return sizeof(double) * (size_t(2 * L) * 33 + L + size_t(n_mu) * 32); }
+__global__ void __launch_bounds__(32 * RAY_WARPS) rt_rays_kernel(RtGenArgs a) {
+    extern __shared__ double s_ray[];
+    __shared__ MathTables s_math;
+    load_math_tables(s_math, a.math);
+    const int L = a.L, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *s_al = s_ray, *s_S = s_al + L * 33, *s_hd = s_S + L * 33, *s_I = s_hd + L;  // [L][33] x 2, [L], [n_mu][32]
+    const int64_t j0 = int64_t(blockIdx.x) * 32;
+    const int nj = int(min(int64_t(32), a.nwl - j0));
+    for (int e = threadIdx.x; e < nj * L; e += blockDim.x) {
+        const int jj = e / L, k = e - jj * L;
+        s_al[k * 33 + jj] = a.alpha[j0 * L + e];
+        s_S[k * 33 + jj] = a.S[j0 * L + e];
+    }
+    // half the steps of log tau_ref, from a ray that holds every layer it needs: outward rays share them
+    for (int k = threadIdx.x; k < L; k += blockDim.x) {
+        double h = 0.0;
+        for (int u = 0; u < a.n_mu; u++)
+            if (k > 0 && k < a.ray_n[a.n_in + u]) {
+                const double* lt = a.ray_lt + int64_t(a.n_in + u) * L;
+                h = 0.5 * (lt[k] - lt[k - 1]);
+                break;
+            }
+        s_hd[k] = h;
+    }
+    __syncthreads();
+    const int c = min(lane, nj - 1);
+    for (int u = warp; u < a.n_mu; u += RAY_WARPS) {
+        const int n = a.ray_n[a.n_in + u];
+        const double* fac = a.ray_fac + int64_t(a.n_in + u) * L;
+        const bool inward = u < a.n_in;
+        double T = 1.0, Iout = 0.0, Iin = 0.0;
+        double ibp = n > 0 ? s_al[c] * fac[0] : 0.0, Sp = s_S[c];
+        for (int k = 1; k < n; k++) {
+            const double ib = s_al[k * 33 + c] * fac[k], S = s_S[k * 33 + c];
+            const double d = (ib + ibp) * s_hd[k];
+            const double m = (S - Sp) * recip64(a.I_scheme == 1 && d == 0 ? 1.0 : d);
+            const double e = fexp64(-d, s_math);
+            Iout = fma(T, fma(-e, S + m, Sp + m), Iout);
+            if (inward) Iin = fma(e, Iin - (Sp - m), S - m);
+            T *= e;
+            ibp = ib;
+            Sp = S;
+            if (!__any_sync(0xffffffffu, T >= RAY_STOP)) break;
+        }
+        if (inward) Iout = fma(T, Iin, Iout);
+        s_I[u * 32 + lane] = Iout;
+        if (a.Isurf && lane < nj) a.Isurf[int64_t(u) * a.nwl + j0 + lane] = Iout;
+    }
+    __syncthreads();
+    if (warp == 0 && lane < nj) {
+        double F = 0.0;
+        for (int u = 0; u < a.n_mu; u++) F += s_I[u * 32 + lane] * a.wmu[u];
+        a.flux[j0 + lane] = 2 * PI * F;
+    }
+}
+
 }  // namespace korg
