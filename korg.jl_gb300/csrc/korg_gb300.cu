@@ -1697,6 +1697,7 @@ KORG_API int korg_set_equilibrium_tables(korg_ctx* ctx, const korg_equilibrium_t
         cudaFree(ctx->chem_buf);
     }
     ctx->chem_buf = buf;
+    d.exp2j = static_cast<MathTables*>(ctx->math.p)->exp2j;
     ctx->chem_tab = d;
     ctx->chem_lnT0 = t->lnT[0];
     ctx->chem_lnT1 = t->lnT[t->n_knots - 1];

@@ -29,11 +29,9 @@
 // factorisation meets a zero pivot, the same elimination runs in FP64 on the FP64 matrix, as
 // LAPACK's getrf + getrs would.
 //
-// Elimination: partial pivoting (largest |entry| of the pivot column, lowest row on ties) with
-// rows left in place and a double-buffered logical-to-physical row permutation; one barrier per
-// column (warps over columns, lanes over rows; multipliers written back one column late); warp
-// 0, which updates the next pivot column, also picks the next pivot.  Triangular solves run in
-// one warp with the vector in registers.
+// Elimination: partial pivoting (largest |entry| of the pivot column) with rows left in place; in FP32
+// by panels of 4 columns (ce_lu32), in FP64 by columns (ce_lu64).  Triangular solves run in one warp
+// with the vector in registers.
 //
 // Every loop is bounded: at most KORG_CHEM_MAX_ITER Newton iterations per layer in total (the
 // reference's own loops are finite but its worst case is ~5e5 iterations); a layer that runs out
@@ -70,6 +68,7 @@ struct ChemTables {
     const int64_t *off;                  // [n_mol + 1]
     const double *t, *u, *z;             // concatenated molecule splines
     const double *D00, *lmr;             // polyatomics
+    const double* exp2j;                 // 2^(j / 256), j < 256 (MathTables)
     const int32_t *nat;                  // atoms per molecule, with multiplicity
     const int32_t *inc_ptr, *inc_mol, *inc_cnt;  // element Z-1 -> (molecule, count) at [inc_ptr[Z-1], inc_ptr[Z])
     int32_t n_items;                     // element sums split in items of <= CE_CHUNK incidences
@@ -123,6 +122,28 @@ __device__ inline double spline_deriv(const double* t, const double* u, const do
     const double a = t[i + 1] - x, b = x - t[i];
     return -z[i] * (a * a) / (2 * h) + z[i + 1] * (b * b) / (2 * h) + (u[i + 1] / h - z[i + 1] * h / 6) -
            (u[i] / h - z[i] * h / 6);
+}
+
+// 10^x by the table-driven exponential of physics.cuh (Tang's method): k = round(256 x log2 10), r = x - k
+// log10(2) / 256 in two parts, 2^(k / 256) e^(r ln 10); about a fifth of exp10's FP64 operations, of
+// which a Newton step evaluates 584 (12.6k of its cycles before).
+__device__ inline double exp10_t(double x, const double* exp2j) {
+    if (!(fabs(x) < 300.0)) return exp10(x);
+    const double INV = 850.4135922911647;         // 256 log2(10)
+    const double HI = 0.0011758984203424916, LO = 2.19934953385746e-13;  // log10(2) / 256, the first to 33 bits
+    const double MAGIC = 6755399441055744.0;      // 1.5 * 2^52
+    double kd = fma(x, INV, MAGIC);
+    const int k = __double2loint(kd);
+    kd -= MAGIC;
+    double r = fma(-kd, HI, x);
+    r = fma(-kd, LO, r) * LN10;
+    double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1.0);
+    p *= r;
+    const double t = exp2j[k & 255];
+    const double v = fma(t, p, t);
+    return __longlong_as_double(__double_as_longlong(v) + ((long long)(k >> 8) << 52));
 }
 
 __device__ inline double translational_U(double m, double T) {  // src/statmech.jl:47-51
@@ -204,8 +225,9 @@ struct CeShared {
     long long redl[4][CE_WARPS];
     double ne, nHm, nn_mol, qn, dNe_mol, ion1, ion2, lognK_Hm, transU, lnT, dlognK_Hm;
     double vsum[3];
+    double exp2j[256];
+    alignas(16) float lu_u[CE_WARPS][16 * 8];  // a warp's columns' pivot-row entries (ce_lu32: at most 13 columns x 4)
     double piv64[2];
-    float piv32[2];
     int perm[2][CE_LD];
     // the molecule tables, copied from global memory once per layer
     unsigned char m_atoms[CE_MAXMOL * CE_MAXATOMS], m_charge[CE_MAXMOL], m_nat[CE_MAXMOL];
@@ -232,18 +254,18 @@ __device__ inline double ce_block_max(CeShared& s, double v) {
 // LU factorisation with partial pivoting of the n x n column-major matrix M (stride CE_LD, rows
 // left in place): multipliers below the diagonal, U on and above it in logical row order; the
 // final logical-to-physical permutation in s.perm[(CE_N - 1) & 1]; uinv = reciprocals of U's
-// diagonal.  Returns false on a zero (or non-finite) pivot.  T = float or double.
+// diagonal.  Returns false on a zero (or non-finite) pivot.
 //
 // One barrier per column: every warp derives the multipliers of its rows from the pivot column
 // (read-only during the step) and updates its columns of the trailing matrix; warp 0, whose first
 // column is the next pivot column, also picks the next pivot, and writes this step's multipliers
 // into the pivot column during the next step, when nothing reads it any more.
-template <typename T>
-__device__ bool ce_lu(CeShared& s, T* M, T* uinv) {
+__device__ bool ce_lu64(CeShared& s, double* M, double* uinv) {
+    using T = double;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // pivot slots, double-buffered by step parity (read at a step's start, the next one written
     // by warp 0 during the step)
-    T* piv = reinterpret_cast<T*>(sizeof(T) == 4 ? (void*)s.piv32 : (void*)s.piv64);
+    T* piv = s.piv64;
     if (tid < CE_N) s.perm[0][tid] = tid;
     if (warp == 0) {  // first pivot: column 0
         T v = T(-1), sv = 0;
@@ -350,34 +372,228 @@ __device__ bool ce_lu(CeShared& s, T* M, T* uinv) {
     return ok;
 }
 
+// The same factorisation in FP32, in panels of CE_PB columns: warp 0 factors a panel in registers (3 rows x 4
+// columns a lane; the pivot by one warp reduction over keys of magnitude and row: largest |entry| to 2^-16
+// of it, lowest row on ties) while the other warps apply the previous panel to the columns beyond; then
+// one barrier.  A trailing column is loaded and stored once per panel.  The loop over a panel's columns
+// stays rolled (the panel's registers shift by one column a step), so that its code stays small: one warp
+// alone is bound by latency and instruction fetch.
+// The column form above, a barrier and two passes over shared memory per column, took 154k cycles a
+// factorisation (146k on a dense random matrix), more than half a Newton step; this one 60k on that matrix
+// (panels of 8: 71k), a whole step's solve 238k -> 142k.
+constexpr int CE_PB = 4;
+__device__ __forceinline__ float ce_pick(const float (&v)[3], int slot) {
+    return slot == 0 ? v[0] : (slot == 1 ? v[1] : v[2]);
+}
+__device__ bool ce_lu32(CeShared& s, float* M, float* uinv) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* P = s.perm[(CE_N - 1) & 1];
+    // which of this lane's rows (lane, +32, +64) are not pivot rows yet; rows beyond CE_N take no part
+    bool open[3] = {true, true, lane + 64 < CE_N};
+    float a[CE_PB][3];  // warp 0: the panel's columns
+    if (warp == 0) {
+#pragma unroll
+        for (int c = 0; c < CE_PB; ++c)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) a[c][r] = lane + 32 * r < CE_N ? M[c * CE_LD + lane + 32 * r] : 0.f;
+    }
+    for (int k0 = 0; k0 < CE_N; k0 += CE_PB) {
+        const int nb = min(CE_PB, CE_N - k0);
+        if (warp == 0) {
+            bool ok = true, now[3] = {open[0], open[1], open[2]};
+#pragma unroll 1
+            for (int q = 0; q < nb; ++q) {
+                unsigned key = 0;
+                float inv[3];  // reciprocals of every candidate, ready when the pivot is known
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    const unsigned kr = (__float_as_uint(a[0][r]) & 0x7fffff80u) | unsigned(127 - lane - 32 * r);
+                    key = max(key, now[r] ? kr : 0u);
+                    inv[r] = __fdividef(1.f, a[0][r]);
+                }
+                key = __reduce_max_sync(0xffffffffu, key);
+                const int pr = 127 - int(key & 127u), slot = pr >> 5, owner = pr & 31;
+                const float pinv = __shfl_sync(0xffffffffu, ce_pick(inv, slot), owner);
+                ok = ok && fabsf(pinv) > 0.f && isfinite(pinv);  // the pivot is neither 0 nor infinite
+                if (lane == 0) {
+                    P[k0 + q] = pr;
+                    uinv[k0 + q] = pinv;
+                }
+                float lq[3];  // multipliers, 0 for pivot rows
+#pragma unroll
+                for (int r = 0; r < 3; ++r) {
+                    if (lane + 32 * r == pr) now[r] = false;
+                    const float m = a[0][r] * pinv;
+                    lq[r] = now[r] ? m : 0.f;
+                    if (lane + 32 * r < CE_N) M[(k0 + q) * CE_LD + lane + 32 * r] = now[r] ? m : a[0][r];
+                }
+#pragma unroll
+                for (int c = 1; c < CE_PB; ++c) {
+                    const float u = __shfl_sync(0xffffffffu, ce_pick(a[c], slot), owner);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) a[c - 1][r] = fmaf(-lq[r], u, a[c][r]);
+                }
+#pragma unroll
+                for (int r = 0; r < 3; ++r) a[CE_PB - 1][r] = 0.f;
+            }
+            if (lane == 0) s.pivi[(k0 / CE_PB) & 1] = ok;  // (slot free: read before the last barrier)
+        }
+        __syncthreads();
+        if (!s.pivi[(k0 / CE_PB) & 1]) return false;  // uniform
+        if (k0 + nb >= CE_N) break;
+        // the panel's pivot rows (a byte each), and act[r] bit q: this lane's row r is below the pivot of
+        // step k0 + q
+        unsigned long long rows = 0;
+        unsigned act[3] = {0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < CE_PB; ++q) {
+            const int pr = P[k0 + q];
+            rows |= (unsigned long long)(pr) << (8 * q);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                open[r] = open[r] && pr != lane + 32 * r;
+                act[r] |= unsigned(open[r]) << q;
+            }
+        }
+        // Columns c0 .. c0 + n - 1 (at most 13) get the panel: lanes hold columns for the pivot rows'
+        // entries (a forward substitution with the panel's unit triangle), which go to the warp's buffer;
+        // then lanes hold rows again.  (Passing the pivot rows by shuffles, one per step and column, was
+        // bound by them.)
+        float* ub = s.lu_u[warp];
+        auto pivot_rows = [&](int c0, int n) {
+            __syncwarp();
+            if (lane < n) {
+                float* col = M + (c0 + lane) * CE_LD;
+                float u[CE_PB];
+#pragma unroll
+                for (int q = 0; q < CE_PB; ++q) u[q] = col[int(rows >> (8 * q)) & 127];
+#pragma unroll
+                for (int q = 0; q < CE_PB; ++q)
+#pragma unroll
+                    for (int t = q + 1; t < CE_PB; ++t)
+                        u[t] = fmaf(-M[(k0 + q) * CE_LD + (int(rows >> (8 * t)) & 127)], u[q], u[t]);
+#pragma unroll
+                for (int q = 0; q < CE_PB; ++q) ub[lane * CE_PB + q] = u[q];
+            }
+            __syncwarp();
+        };
+        // one column, this lane's rows: v -= sum over q of multiplier q times the column's pivot entry q
+        float l[CE_PB][3];
+#pragma unroll
+        for (int q = 0; q < CE_PB; ++q)
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+                l[q][r] = (act[r] >> q) & 1u ? M[(k0 + q) * CE_LD + lane + 32 * r] : 0.f;
+        auto update = [&](int c0, int e, float (&v)[3]) {
+            float u[CE_PB];
+#pragma unroll
+            for (int q = 0; q < CE_PB; q += 4)
+                *reinterpret_cast<float4*>(u + q) = *reinterpret_cast<const float4*>(ub + e * CE_PB + q);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                v[r] = lane + 32 * r < CE_N ? M[(c0 + e) * CE_LD + lane + 32 * r] : 0.f;
+#pragma unroll
+                for (int q = 0; q < CE_PB; ++q) v[r] = fmaf(-l[q][r], u[q], v[r]);
+            }
+        };
+        if (warp == 0) {  // the next panel
+            const int c0 = k0 + CE_PB, n = min(CE_PB, CE_N - c0);
+            pivot_rows(c0, n);
+#pragma unroll
+            for (int c = 0; c < CE_PB; ++c) {
+                if (c < n) update(c0, c, a[c]);
+                else a[c][0] = a[c][1] = a[c][2] = 0.f;
+            }
+        } else {  // the columns beyond, an even share per warp
+            const int rest = CE_N - (k0 + 2 * CE_PB), share = (rest + CE_WARPS - 2) / (CE_WARPS - 1);
+            const int c0 = k0 + 2 * CE_PB + (warp - 1) * share, n = min(share, CE_N - c0);
+            if (n > 0) {
+                pivot_rows(c0, n);
+#pragma unroll 2
+                for (int e = 0; e < n; ++e) {
+                    float v[3];
+                    update(c0, e, v);
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+                        if (lane + 32 * r < CE_N) M[(c0 + e) * CE_LD + lane + 32 * r] = v[r];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
 // Solve L U x = P b in one warp (warp 0): b in physical row order, x in column order; M, the
 // permutation P (logical -> physical row) and uinv from the factorisation.  Other warps return
-// at once.
+// at once.  Steps in groups of 32 unknowns, so that a step's operand needs no selection and the
+// columns of the steps ahead are loaded early.
+__device__ __forceinline__ float ce_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double ce_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 template <typename T>
 __device__ void ce_trisolve(const int* P, const T* M, const T* uinv, const T* b, T* x) {
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid >= 32) return;
     const int i0 = lane, i1 = lane + 32, i2 = lane + 64;
     const bool v2 = i2 < CE_N;
-    const int r0 = P[i0], r1 = P[i1], r2 = v2 ? P[i2] : 0;
+    const int r0 = P[i0], r1 = P[i1], r2 = v2 ? P[i2] : P[i0];  // (lanes without a third row: any row, unused)
     T y0 = b[r0], y1 = b[r1], y2 = v2 ? b[r2] : T(0);
-    for (int j = 0; j < CE_N - 1; ++j) {  // forward: unit lower L
-        const T yj = __shfl_sync(0xffffffffu, j < 32 ? y0 : (j < 64 ? y1 : y2), j & 31);
+    // multipliers of rows that a step does not touch are 0, so that no step branches
+#pragma unroll 4
+    for (int j = 0; j < 32; ++j) {  // forward: unit lower L
         const T* col = M + j * CE_LD;
-        if (i0 > j) y0 = fma(-col[r0], yj, y0);
-        if (i1 > j) y1 = fma(-col[r1], yj, y1);
-        if (v2 && i2 > j) y2 = fma(-col[r2], yj, y2);
+        T m0 = col[r0], m1 = col[r1], m2 = col[r2];
+        m0 = lane > j ? m0 : T(0);
+        const T yj = __shfl_sync(0xffffffffu, y0, j);
+        y0 = ce_fma(-m0, yj, y0);
+        y1 = ce_fma(-m1, yj, y1);
+        y2 = ce_fma(-m2, yj, y2);
     }
-    for (int j = CE_N - 1; j >= 0; --j) {  // backward: U
-        const T yj = __shfl_sync(0xffffffffu, j < 32 ? y0 : (j < 64 ? y1 : y2), j & 31);
-        const T xj = yj * uinv[j];
-        if (lane == (j & 31)) {
-            if (j < 32) y0 = xj; else if (j < 64) y1 = xj; else y2 = xj;
-        }
-        const T* col = M + j * CE_LD;
-        if (i0 < j) y0 = fma(-col[r0], xj, y0);
-        if (i1 < j) y1 = fma(-col[r1], xj, y1);
-        if (v2 && i2 < j) y2 = fma(-col[r2], xj, y2);
+#pragma unroll 4
+    for (int j = 0; j < 32; ++j) {
+        const T* col = M + (j + 32) * CE_LD;
+        T m1 = col[r1], m2 = col[r2];
+        m1 = lane > j ? m1 : T(0);
+        const T yj = __shfl_sync(0xffffffffu, y1, j);
+        y1 = ce_fma(-m1, yj, y1);
+        y2 = ce_fma(-m2, yj, y2);
+    }
+#pragma unroll 4
+    for (int j = 0; j < CE_N - 65; ++j) {
+        T m2 = M[(j + 64) * CE_LD + r2];
+        m2 = lane > j ? m2 : T(0);
+        const T yj = __shfl_sync(0xffffffffu, y2, j);
+        y2 = ce_fma(-m2, yj, y2);
+    }
+    const T d0 = uinv[i0], d1 = uinv[i1], d2 = v2 ? uinv[i2] : T(0);
+#pragma unroll 4
+    for (int j = CE_N - 65; j >= 0; --j) {  // backward: U
+        const T* col = M + (j + 64) * CE_LD;
+        T m0 = col[r0], m1 = col[r1], m2 = col[r2];
+        m2 = lane < j ? m2 : T(0);
+        y2 = lane == j ? y2 * d2 : y2;
+        const T xj = __shfl_sync(0xffffffffu, y2, j);
+        y0 = ce_fma(-m0, xj, y0);
+        y1 = ce_fma(-m1, xj, y1);
+        y2 = ce_fma(-m2, xj, y2);
+    }
+#pragma unroll 4
+    for (int j = 31; j >= 0; --j) {
+        const T* col = M + (j + 32) * CE_LD;
+        T m0 = col[r0], m1 = col[r1];
+        m1 = lane < j ? m1 : T(0);
+        y1 = lane == j ? y1 * d1 : y1;
+        const T xj = __shfl_sync(0xffffffffu, y1, j);
+        y0 = ce_fma(-m0, xj, y0);
+        y1 = ce_fma(-m1, xj, y1);
+    }
+#pragma unroll 4
+    for (int j = 31; j >= 0; --j) {
+        T m0 = M[j * CE_LD + r0];
+        m0 = lane < j ? m0 : T(0);
+        y0 = lane == j ? y0 * d0 : y0;
+        const T xj = __shfl_sync(0xffffffffu, y0, j);
+        y0 = ce_fma(-m0, xj, y0);
     }
     x[i0] = y0;
     x[i1] = y1;
@@ -401,14 +617,14 @@ __device__ bool ce_solve(CeShared& s, bool& refined) {
         s.rexp[tid] = m ? int(m >> 52) - 1023 : 0;
     }
     if (__syncthreads_or(bad)) return false;
-    if (tid < CE_N) {
+    for (int c = warp; c < CE_N; c += CE_WARPS) {  // a warp per column (a thread per column: 32-way bank conflicts)
         long long m = 0;
-        const double* col = s.A + tid * CE_LD;
-        for (int r = 0; r < CE_N; ++r) {
-            const long long a = ce::abits(col[r]);
+        for (int r = lane; r < CE_N; r += 32) {
+            const long long a = ce::abits(s.A[c * CE_LD + r]);
             if (a) m = max(m, a - ((long long)s.rexp[r] << 52));
         }
-        s.cexp[tid] = m > 0 ? int(m >> 52) - 1023 : 0;
+        m = ce::warp_max_ll(m);
+        if (lane == 0) s.cexp[c] = m > 0 ? int(m >> 52) - 1023 : 0;
     }
     __syncthreads();
     for (int idx = tid; idx < CE_N * CE_N; idx += CE_THREADS) {
@@ -427,7 +643,7 @@ __device__ bool ce_solve(CeShared& s, bool& refined) {
             for (int c = 0; c < CE_N; ++c) a += fabsf(s.B[c * CE_LD + tid]);
         return double(a);
     }());
-    refined = ce_lu<float>(s, s.B, s.uinv32);
+    refined = ce_lu32(s, s.B, s.uinv32);
     if (refined) {
         // iterative refinement (as LAPACK's dsgesv): stop when the equilibrated residual is at
         // the level of an FP64 backward-stable solve, |R r| <= |C^-1 s| |J^| eps sqrt(n)
@@ -470,8 +686,15 @@ __device__ bool ce_solve(CeShared& s, bool& refined) {
             // residual F - J s in FP64, its equilibrated norm and that of the step
             long long rl = 0, xl = 0;
             if (tid < CE_N) {
-                double r = s.A[CE_N * CE_LD + tid];
-                for (int c = 0; c < CE_N; ++c) r = fma(-s.A[c * CE_LD + tid], s.sol[c], r);
+                // three chains (a dependent FP64 FMA takes ~70 cycles)
+                double r = s.A[CE_N * CE_LD + tid], ra = 0.0, rb = 0.0;
+#pragma unroll 1
+                for (int c = 0; c < CE_N; c += 3) {
+                    r = fma(-s.A[c * CE_LD + tid], s.sol[c], r);
+                    ra = fma(-s.A[(c + 1) * CE_LD + tid], s.sol[c + 1], ra);
+                    rb = fma(-s.A[(c + 2) * CE_LD + tid], s.sol[c + 2], rb);
+                }
+                r += ra + rb;
                 s.res[tid] = r;
                 const long long a = ce::abits(r);
                 if (a) rl = max(0LL, a - ((long long)s.rexp[tid] << 52));
@@ -507,7 +730,7 @@ __device__ bool ce_solve(CeShared& s, bool& refined) {
         // FP64 elimination in place (J is rebuilt by the next iteration); F from column CE_N
         if (tid < CE_N) s.res[tid] = s.A[CE_N * CE_LD + tid];
         __syncthreads();
-        if (!ce_lu<double>(s, s.A, s.uinv64)) return false;
+        if (!ce_lu64(s, s.A, s.uinv64)) return false;
         ce_trisolve<double>(s.perm[(CE_N - 1) & 1], s.A, s.uinv64, s.res, s.sol);
         __syncthreads();
     }
@@ -537,17 +760,17 @@ __device__ int ce_assemble(const ChemTables& tb, CeShared& s, double nt, double 
             const int Z1 = at[0] - 1, Z2 = at[1] - 1;
             lg += ((s.x[Z1] + s.lwII[Z1]) - xe) + s.x[Z2];
         }
-        s.nmol[m] = exp10(lg);
+        s.nmol[m] = ce::exp10_t(lg, s.exp2j);
     }
     for (int Z = tid; Z < CE_NZ; Z += CE_THREADS) {
         const double xz = s.x[Z];
-        s.nI[Z] = exp10(xz);
-        s.nII[Z] = exp10((xz + s.lwII[Z]) - xe);
-        s.nIII[Z] = exp10((xz + s.lwIII[Z]) - 2 * xe);
+        s.nI[Z] = ce::exp10_t(xz, s.exp2j);
+        s.nII[Z] = ce::exp10_t((xz + s.lwII[Z]) - xe, s.exp2j);
+        s.nIII[Z] = ce::exp10_t((xz + s.lwIII[Z]) - 2 * xe, s.exp2j);
     }
     if (tid == 0) {
-        s.ne = exp10(xe);
-        s.nHm = exp10(((s.lognK_Hm + s.x[0]) + xe) + logxi);
+        s.ne = ce::exp10_t(xe, s.exp2j);
+        s.nHm = ce::exp10_t(((s.lognK_Hm + s.x[0]) + xe) + logxi, s.exp2j);
     }
     __syncthreads();
     // element sums in work items of <= CE_CHUNK incidences (warps 0-6), the block-wide sums
@@ -675,6 +898,7 @@ __device__ void ce_prologue(const ChemTables& tb, const ChemLayersDev& ly, int l
     const double lnT = log(T);
     const double transU = ce::translational_U(ce::ME_CGS, T);
     const double iTl = 1.0 / (T * ce::LN10);  // d log10(f) / dT = (d ln f / d ln T) / (T ln10)
+    for (int i = tid; i < 256; i += CE_THREADS) s.exp2j[i] = tb.exp2j[i];
     for (int i = tid; i < M * CE_MAXATOMS; i += CE_THREADS) s.m_atoms[i] = (unsigned char)tb.atoms[i];
     for (int m = tid; m < M; m += CE_THREADS) {
         s.m_charge[m] = (unsigned char)tb.charge[m];
@@ -820,7 +1044,7 @@ __device__ bool ce_newton(const ChemTables& tb, CeShared& s, double nt, double l
     return false;
 }
 
-__global__ void __launch_bounds__(CE_THREADS) chem_eq_kernel(ChemTables tb, ChemLayersDev ly, double* __restrict__ dens,
+__global__ void __launch_bounds__(CE_THREADS, 1) chem_eq_kernel(ChemTables tb, ChemLayersDev ly, double* __restrict__ dens,
                                                              int32_t* __restrict__ status, double* __restrict__ info) {
     extern __shared__ __align__(16) unsigned char ce_smem[];
     CeShared& s = *reinterpret_cast<CeShared*>(ce_smem);
