@@ -14,9 +14,9 @@
 // Metal bound-free absorption (absorption_metals_bf.jl) needs the bf_cross-sections.h5 blob,
 // which is not part of the reference checkout: it is not included.
 //
-// One thread per (layer, wavelength); the work is tiny next to the line opacity (a few hundred
-// thousand points per atmosphere), so the kernel favours plainness: binary searches on the
-// (read-only, cached) tables.
+// One block per (layer, 128 wavelengths), one thread per wavelength.  What depends on the layer alone
+// (the occupation of the 40 H I levels, the positions in the temperature tables) is computed once per
+// block; binary searches run on the (read-only, cached) tables.
 #pragma once
 #include "physics.cuh"
 
@@ -89,47 +89,78 @@ __device__ __forceinline__ double mhd_w(double n_eff, double nH, double nHe, dou
     return hummer_mihalas_w(n_eff, nH, nHe, ne);
 }
 
-// absorption_H.jl:54-163
-__device__ double H_I_bf(const CntmTables& t, double nu, double T, double nH_I, double nHe_I, double ne,
-                         double invU_H) {
-    double total = 0.0;
-    for (int n = 1; n <= 6; n++) {
-        const double* Es = t.h_E + (n - 1) * t.h_n;
-        const double* sig = t.h_sigma + (n - 1) * t.h_n;
-        const double w_lower = mhd_w(double(n), nH_I, nHe_I, ne);
-        const double occ = w_lower * exp(-CHI_H * (1 - 1.0 / (n * n)) / (KB_EV * T));
-        const double nu_break = CHI_H / (n * n * H_EV);
-        double cs, frac;
-        if (nu > nu_break) {
-            frac = 1.0;
-            cs = lerp(Es, sig, t.h_n, H_EV * nu);
+// Per-layer part of H I bound-free, computed by a block: the levels' populations, and the sums over the
+// hydrogenic levels n, n+1, ..., 40 of their cross-sections' factors (every level whose edge lies below
+// the photon energy contributes: a suffix of them).  Each thread's own 40 exponentials and as many
+// dissociation factors per wavelength before.
+constexpr int HI_LEVELS = 40;
+struct HILayer {
+    double w[7];               // MHD occupation probability of levels 1..6
+    double occ[7];             // their populations
+    double brk[7];             // cross-section at the edge, times the edge's nu^3
+    double suffix[HI_LEVELS + 2];  // sum over n.. of 2 n^2 w exp(..) 2.815e29 / n^5 1e18, n >= 7
+};
+__device__ void H_I_layer(const CntmTables& t, double T, double nH_I, double nHe_I, double ne, HILayer& h) {
+    __shared__ double s_w[HI_LEVELS + 1];
+    const int n = threadIdx.x + 1;
+    if (n <= HI_LEVELS) {
+        const double w = mhd_w(double(n), nH_I, nHe_I, ne);
+        const double e = w * exp(-CHI_H * (1 - 1.0 / (n * n)) / (KB_EV * T));
+        s_w[n] = w;
+        if (n <= 6) {
+            const double nu_break = CHI_H / (n * n * H_EV);
+            h.w[n] = w;
+            h.occ[n] = e;
+            h.brk[n] = lerp(t.h_E + (n - 1) * t.h_n, t.h_sigma + (n - 1) * t.h_n, t.h_n, nu_break * H_EV) *
+                       (nu_break * nu_break * nu_break);
         } else {
-            if (n == 1) {
-                frac = 0.0;
-            } else {
-                const double n_eff = 1 / sqrt(1.0 / (n * n) - H_EV * nu / CHI_H);
-                frac = 1 - mhd_w(n_eff, nH_I, nHe_I, ne) / w_lower;
-            }
-            const double sigma_break = lerp(Es, sig, t.h_n, nu_break * H_EV);
-            cs = pow(nu, -3.0) * (sigma_break / pow(nu_break, -3.0));
-        }
-        total += occ * cs * frac;
-    }
-    for (int n = 7; n <= 40; n++) {
-        const double w_lower = mhd_w(double(n), nH_I, nHe_I, ne);
-        if (w_lower < 1e-5) break;
-        const double occ = 2.0 * n * n * w_lower * exp(-CHI_H * (1 - 1.0 / (n * n)) / (KB_EV * T));
-        const double inv_n = 1.0 / n, inv_n2 = inv_n * inv_n;
-        if (!(H_EV * nu < RYH_EV * inv_n2)) {
-            const double inv_nu = 1.0 / nu;
-            total += occ * (2.815e29 * (inv_n2 * inv_n2 * inv_n) * (inv_nu * inv_nu * inv_nu) * 1e18);
+            const double inv_n = 1.0 / n, inv_n2 = inv_n * inv_n;
+            h.suffix[n] = 2.0 * n * n * e * (2.815e29 * (inv_n2 * inv_n2 * inv_n) * 1e18);
         }
     }
-    return nH_I * invU_H * total * (1.0 - exp(-H_EV * nu / (KB_EV * T))) * 1e-18;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int last = 6;  // the first level dissolved below 1e-5 ends the sum
+        while (last < HI_LEVELS && !(s_w[last + 1] < 1e-5)) last++;
+        double sum = 0.0;
+        for (int k = HI_LEVELS + 1; k >= 7; k--) {
+            if (k <= last) sum += h.suffix[k];
+            h.suffix[k] = sum;
+        }
+    }
+    __syncthreads();
+}
+
+// absorption_H.jl:54-163
+__device__ double H_I_bf(const CntmTables& t, const HILayer& h, double nu, double stim, double nH_I, double nHe_I,
+                         double ne, double invU_H) {
+    double total = 0.0;
+    const double inv_nu = 1.0 / nu, inv_nu3 = inv_nu * inv_nu * inv_nu;
+    for (int n = 1; n <= 6; n++) {
+        const double nu_break = CHI_H / (n * n * H_EV);
+        if (nu > nu_break) {
+            total += h.occ[n] * lerp(t.h_E + (n - 1) * t.h_n, t.h_sigma + (n - 1) * t.h_n, t.h_n, H_EV * nu);
+        } else if (n > 1) {
+            const double n_eff = 1 / sqrt(1.0 / (n * n) - H_EV * nu / CHI_H);
+            const double frac = 1 - mhd_w(n_eff, nH_I, nHe_I, ne) / h.w[n];
+            total += h.occ[n] * (inv_nu3 * h.brk[n]) * frac;
+        }
+    }
+    // levels with H_EV nu >= RYH_EV / n^2: the first of them from the quotient, then by the test itself
+    int n0 = HI_LEVELS + 1;
+    const double q = RYH_EV / (H_EV * nu);
+    if (q <= double(HI_LEVELS * HI_LEVELS)) {
+        n0 = max(7, int(sqrt(q)) - 1);
+        while (n0 <= HI_LEVELS && H_EV * nu < RYH_EV * ((1.0 / n0) * (1.0 / n0))) n0++;
+    } else if (!(H_EV * nu < RYH_EV * ((1.0 / HI_LEVELS) * (1.0 / HI_LEVELS)))) {
+        n0 = HI_LEVELS;
+    }
+    total += h.suffix[n0] * inv_nu3;
+    return nH_I * invU_H * total * stim * 1e-18;
 }
 
 // absorption_H.jl:170-228
-__device__ double Hminus_bf(const CntmTables& t, double nu, double T, double n_Hminus) {
+__device__ double Hminus_bf(const CntmTables& t, double nu, double T, double n_Hminus, double stim) {
     if (!(nu >= 0.0 && nu <= 2.417989242625068e19 && T > 0)) return 0.0;
     const double nu_ion = HMINUS_ION_EV / H_EV, nu_min = t.hm_nu[0];
     double cs;
@@ -142,7 +173,7 @@ __device__ double Hminus_bf(const CntmTables& t, double nu, double T, double n_H
         const double s = (t.hm_sigma[i + 1] - t.hm_sigma[i]) / (t.hm_nu[i + 1] - t.hm_nu[i]);
         cs = s * (nu - t.hm_nu[i]) + t.hm_sigma[i];
     }
-    return n_Hminus * cs * (1 - exp(-H_CGS * nu / (KB_CGS * T)));
+    return n_Hminus * cs * stim;
 }
 
 // absorption_H.jl:261-325: 1823 A <= lambda <= 151890 A, 1400 K <= T <= 10080 K
@@ -153,13 +184,13 @@ __device__ double Hminus_ff(const CntmTables& t, double nu, double T, double nH_
 }
 
 // absorption_H.jl:327-380, Stancil1994.jl: 700 A <= lambda <= 200000 A, 3150 K <= T <= 25200 K
-__device__ double H2plus(const CntmTables& t, double nu, double T, double nH_I, double nH_II) {
+__device__ double H2plus(const CntmTables& t, double nu, double T, double nH_I, double nH_II, double stim) {
     if (!(in(nu, C / 2e-3, C / 7e-6) && in(T, 3150, 25200))) return 0.0;
     const double lam = C * 1e8 / nu;
     const double K = lerp(t.h2_T, t.h2_K, t.h2_nT, T);
     const double sbf = 1e-18 * bilerp(t.h2_bf_lambda, t.h2_nbf, t.h2_T, t.h2_nT, t.h2_bf_sigma, lam, T);
     const double sff = 1e-39 * bilerp(t.h2_ff_lambda, t.h2_nff, t.h2_T, t.h2_nT, t.h2_ff_sigma, lam, T);
-    return (sbf / K + sff) * nH_I * nH_II * (1 - exp(-H_EV * nu / (KB_EV * T)));
+    return (sbf / K + sff) * nH_I * nH_II * stim;
 }
 
 // absorption_He.jl:31-95: 5063 A <= lambda <= 151878 A, 1400 K <= T <= 10080 K
@@ -170,14 +201,13 @@ __device__ double Heminus_ff(const CntmTables& t, double nu, double T, double nH
     return K * nHe_I_div_U * (ne * KB_CGS * T);
 }
 
-// hydrogenic_bf_ff.jl:116-176
-__device__ double hydrogenic_ff(const CntmTables& t, double nu, double T, int Z, double ni, double ne) {
+// hydrogenic_bf_ff.jl:116-176 without the ion's density
+__device__ double hydrogenic_ff(const CntmTables& t, double nu, double T, int Z, double ne, double stim) {
     const double inv_T = 1.0 / T, Z2 = double(Z * Z);
     const double hnu_kT = (H_EV / KB_EV) * nu * inv_T;
     const double g = bilerp(t.g_log_u, t.g_nu, t.g_log_g2, t.g_ng, t.g_ff, log10(hnu_kT),
                             log10((RY_EV / KB_EV) * Z2 * inv_T));
-    const double F = 3.6919e8 * g * Z2 * sqrt(inv_T) / (nu * nu * nu);
-    return ni * ne * F * (1 - exp(-hnu_kT));
+    return ne * (3.6919e8 * g * Z2 * sqrt(inv_T) / (nu * nu * nu)) * stim;
 }
 
 // Peach1970.jl: bilinear in (T, sigma), zero outside the table
@@ -189,15 +219,13 @@ __device__ double peach(const CntmTables& t, int k, double T, double sigma) {
 }
 
 // absorption_ff_positive_ion.jl:44-84: 100 K <= T <= 1e6 K, 1e-6 cm < lambda < 1e-2 cm
-__device__ double positive_ion_ff(const CntmTables& t, const CntmLayers& y, int l, double nu, double T, double ne) {
+__device__ double positive_ion_ff(const CntmTables& t, const CntmLayers& y, int l, double nu, double T, double ne,
+                                  double stim) {
     if (!(T >= 100.0 && T <= 1e6) || !(C / 1e-2 < nu && nu < C / 1e-6)) return 0.0;
-    double a = 0.0;
+    double n1 = y.n_Z1[l];  // singly charged ions, weighted by their departure from the hydrogenic form
     const double sig = nu * (H_EV / RY_EV);  // photon energy in Rydberg Z^2 (Z = 1)
-    for (int k = 0; k < CNT_PEACH; k++)
-        a += hydrogenic_ff(t, nu, T, 1, y.n_peach[k][l], ne) * (1 + peach(t, k, T, sig));
-    a += hydrogenic_ff(t, nu, T, 1, y.n_Z1[l], ne);
-    a += hydrogenic_ff(t, nu, T, 2, y.n_Z2[l], ne);
-    return a;
+    for (int k = 0; k < CNT_PEACH; k++) n1 += y.n_peach[k][l] * (1 + peach(t, k, T, sig));
+    return n1 * hydrogenic_ff(t, nu, T, 1, ne, stim) + y.n_Z2[l] * hydrogenic_ff(t, nu, T, 2, ne, stim);
 }
 
 // scattering.jl
@@ -217,24 +245,30 @@ __device__ __forceinline__ double electron_scattering(double ne) {
 }  // namespace cnt
 
 // vals[l * nwl + j] = total continuum absorption of layer l at wavelength wls[j] (cm), the
-// layout of the continuum interpolants (korg_cntm)
-__global__ void __launch_bounds__(256) continuum_kernel(CntmTables t, CntmLayers y, const double* wls, int64_t nwl,
-                                                        double* vals) {
-    const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= nwl * y.L) return;
-    const int l = int(e / nwl);
-    const int64_t j = e - int64_t(l) * nwl;
-    const double nu = cnt::C / wls[j];
+// layout of the continuum interpolants (korg_cntm).  Latency and FP64: 56 layers x 122 wavelengths and
+// the call of one wavelength per layer that goes with it 817 -> 161 us.
+constexpr int CNT_THREADS = 128;
+__global__ void __launch_bounds__(CNT_THREADS) continuum_kernel(CntmTables t, CntmLayers y, const double* wls,
+                                                                int64_t nwl, double* vals) {
+    __shared__ cnt::HILayer s_h;
+    const int64_t nb = (nwl + CNT_THREADS - 1) / CNT_THREADS;
+    const int l = int(blockIdx.x / nb);
+    const int64_t j = (blockIdx.x - l * nb) * CNT_THREADS + threadIdx.x;
     const double T = y.T[l], ne = y.ne[l], nH = y.nH_I[l], nHe = y.nHe_I[l];
-    double a = cnt::H_I_bf(t, nu, T, nH, nHe, ne, y.invU_H_I[l]);
-    a += cnt::Hminus_bf(t, nu, T, y.nH_minus[l]);
+    cnt::H_I_layer(t, T, nH, nHe, ne, s_h);
+    if (j >= nwl) return;
+    const double nu = cnt::C / wls[j];
+    // stimulated emission, in the two units' constants that the reference uses
+    const double stim_eV = 1.0 - exp(-cnt::H_EV * nu / (cnt::KB_EV * T)), stim = 1 - exp(-cnt::H_CGS * nu / (cnt::KB_CGS * T));
+    double a = cnt::H_I_bf(t, s_h, nu, stim_eV, nH, nHe, ne, y.invU_H_I[l]);
+    a += cnt::Hminus_bf(t, nu, T, y.nH_minus[l], stim);
     a += cnt::Hminus_ff(t, nu, T, nH * y.invU_H_I[l], ne);
-    a += cnt::H2plus(t, nu, T, nH, y.nH_II[l]);
+    a += cnt::H2plus(t, nu, T, nH, y.nH_II[l], stim_eV);
     a += cnt::Heminus_ff(t, nu, T, nHe * y.invU_He_I[l], ne);
-    a += cnt::positive_ion_ff(t, y, l, nu, T, ne);
+    a += cnt::positive_ion_ff(t, y, l, nu, T, ne, stim_eV);
     a += cnt::electron_scattering(ne);
     a += cnt::rayleigh(nu, nH, nHe, y.nH2[l]);
-    vals[e] = a;
+    vals[int64_t(l) * nwl + j] = a;
 }
 
 }  // namespace korg

@@ -1503,8 +1503,8 @@ KORG_API int korg_continuum_absorption_dev(korg_ctx* ctx, const double* wls, int
     if (!wls || nwl < 1 || !vals || !cntm_layers_ok(layers)) return set_err(ctx, KORG_EINVAL, "bad arguments");
     if (!ctx->have_cntm) return set_err(ctx, KORG_ENOTABLES, "korg_set_continuum_tables() has not been called");
     KCUDA(cudaSetDevice(ctx->device));
-    const int64_t n = nwl * layers->L;
-    continuum_kernel<<<unsigned((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const int64_t blocks = (nwl + CNT_THREADS - 1) / CNT_THREADS * layers->L;
+    continuum_kernel<<<unsigned(blocks), CNT_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
         ctx->cntm_tab, cntm_layers(layers), wls, nwl, vals);
     KCUDA(cudaGetLastError());
     return KORG_OK;
