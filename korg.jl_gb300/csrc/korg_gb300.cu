@@ -261,9 +261,10 @@ size_t line_scratch(unsigned char* base, int64_t n, int L, int Lp, int G, bool m
 }
 
 // Tile-kernel arguments that follow from the scratch and the inputs (launch geometry aside).
-TileArgs make_tile_args(const LineScratch& sc, double* alpha, const double* wls, int64_t nwl, const LinesDev& ln,
-                        int L, int Lp, int G) {
+TileArgs make_tile_args(const korg_ctx* ctx, const LineScratch& sc, double* alpha, const double* wls, int64_t nwl,
+                        const LinesDev& ln, int L, int Lp, int G) {
     TileArgs ta{};
+    ta.math = static_cast<const MathTables*>(ctx->math.p);
     ta.alpha = alpha;
     ta.wls = wls;
     ta.nwl = nwl;
@@ -321,11 +322,16 @@ struct TileGeom {
     size_t smem;
 };
 
+// Lines per batch where the shape leaves it open.  FP64, one layer group per CTA: 32 and not 16, since the
+// far lines of a batch are spread over 8 slots of threads (line_absorption! of 2,000 lines x 10,001
+// wavelengths 4.52 -> 4.25 ms, its FP64 gradient over 10 A 6.21 -> 5.94 ms); all groups: 16, for space.
+int default_stage(bool mixed, int split) { return mixed ? 2 * STAGE_LINES : (split ? STAGE_LINES : STAGE_LINES / 2); }
+
 // One wavelength per thread; the mixed form always takes one layer group per CTA, the FP64 form
 // one or all layer groups.
 bool tile_geom(bool mixed, int Lp, int G, TileCfg c, TileGeom* g) {
     const size_t psz = mixed ? sizeof(float4) : sizeof(P64);
-    const int B = c.stage > 0 ? c.stage : (mixed ? 2 * STAGE_LINES : STAGE_LINES / 2);
+    const int B = c.stage > 0 ? c.stage : default_stage(mixed, c.split);
     if (mixed && !c.split) return false;
     const int Gc = c.split ? 1 : G;  // layer groups per CTA
     const int SL = c.split ? Lp / G : Lp;
@@ -341,11 +347,10 @@ bool tile_geom(bool mixed, int Lp, int G, TileCfg c, TileGeom* g) {
     g->split = c.split ? 1 : 0;
     g->G = G;
     g->smem = 2 * region + size_t(g->threads) * (mixed ? sizeof(LineStage32) : sizeof(LineStage));
-    if (!mixed) g->smem += sizeof(double) * SL * (FAR_P + 1);  // Chebyshev coefficients of the far lines
     return g->smem <= 227 * 1024;
 }
 
-// Default tile shape: 128 wavelengths x one layer group (mixed: 64-line batches, FP64: 16).
+// Default tile shape: 128 wavelengths x one layer group.
 TileCfg default_tile(bool) { return TileCfg{TILE_TW, 0, 1}; }
 
 // far_lines: whether some tile can hold FAR_MIN_CAND32 candidates (mixed: line_far_kernel runs first).
@@ -408,8 +413,8 @@ TileCfg tile_cfg(const korg_ctx* ctx, int L, bool mixed) {
     return it != ctx->tuned.end() ? it->second : default_tile(mixed);
 }
 
-// Autotuner: times every candidate shape (FP64: TW in {32, 64, 128} x stage in {8, 16} x split
-// or not; mixed: TW in {64, 128, 256} x stage in {32, 64}, split) on the real candidate lists of
+// Autotuner: times every candidate shape (FP64: TW in {32, 64, 128} x stage in {8, 16}, or
+// {16, 32} when split; mixed: TW in {64, 128, 256} x stage in {32, 64}, split) on the real candidate lists of
 // one spectrum, writing into a scratch alpha, and keeps the fastest for (L, precision).  Runs
 // once per (L, precision) per context, outside any stream capture.
 int autotune_tiles(korg_ctx* ctx, const TileArgs& ta0, int kmax, bool mixed, cudaStream_t s) {
@@ -420,12 +425,11 @@ int autotune_tiles(korg_ctx* ctx, const TileArgs& ta0, int kmax, bool mixed, cud
     KCUDA(cudaMemsetAsync(ctx->tune_alpha.p, 0, sizeof(double) * size_t(L) * ta0.nwl, s));
     TileArgs ta = ta0;
     ta.alpha = static_cast<double*>(ctx->tune_alpha.p);
-    const int B0 = mixed ? 2 * STAGE_LINES : STAGE_LINES / 2;
     TileCfg best = default_tile(mixed);
     float best_ms = 1e30f;
     for (int split : {0, 1})
     for (int tw : {64, 32, 128, 256, 512})
-        for (int B : {B0, B0 / 2}) {
+        for (int B : {default_stage(mixed, split), default_stage(mixed, split) / 2}) {
             if (mixed ? (tw < 64 || !split) : tw > 128) continue;
             TileGeom g;
             if (!tile_geom(mixed, Lp, G, TileCfg{tw, B, split}, &g)) continue;
@@ -464,7 +468,7 @@ int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t
     line_scratch(static_cast<unsigned char*>(ctx->lines_scratch.p), ln.n, L, Lp, G, mixed, &sc);
     KCHECK(prep_lines(ctx, sc, wls, nwl, ln, lay, cn, cutoff, mixed, kmax, G, s));
     record(ctx, 2, s);
-    TileArgs ta = make_tile_args(sc, alpha, wls, nwl, ln, L, Lp, G);
+    TileArgs ta = make_tile_args(ctx, sc, alpha, wls, nwl, ln, L, Lp, G);
     ta.far32 = far32;
     if (ctx->autotune && !ctx->capturing && worth_tuning(nwl, ln.n)) KCHECK(autotune_tiles(ctx, ta, kmax, mixed, s));
     TileGeom g;
@@ -780,7 +784,7 @@ void fill_batch_host(korg_ctx* ctx, const BatchPlan& p, int nspec, const korg_ba
         if (it[i].lines.n == 0) {
             sc.tier_meta = zero;  // all tier runs empty
         }
-        TileArgs ta = make_tile_args(sc, batch_alpha(ctx, p, i, nwl), wls, nwl, lines_dev(&it[i].lines), p.L, p.Lp, p.G);
+        TileArgs ta = make_tile_args(ctx, sc, batch_alpha(ctx, p, i, nwl), wls, nwl, lines_dev(&it[i].lines), p.L, p.Lp, p.G);
         ta.stage = p.geom.stage;
         ta.region = p.geom.region;
         ta.split = p.geom.split;
@@ -2518,7 +2522,7 @@ KORG_API int korg_get_tile_config(korg_ctx* ctx, int32_t L, int precision, int32
     const bool mixed = precision == KORG_MIXED;
     const TileCfg c = tile_cfg(ctx, L, mixed);
     *tw = c.tw;
-    *stage = c.stage > 0 ? c.stage : (mixed ? 2 * STAGE_LINES : STAGE_LINES / 2);
+    *stage = c.stage > 0 ? c.stage : default_stage(mixed, c.split);
     if (split) *split = c.split;
     if (tuned) *tuned = ctx->tuned.count(std::make_pair(int(L), int(mixed))) ? 1 : 0;
     return KORG_OK;
@@ -2573,7 +2577,7 @@ KORG_API int korg_synthesize_batch_dev(korg_ctx* ctx, int32_t nspec, const korg_
             KCHECK(prep_lines(ctx, sc, wls, nwl, ln, layers_dev(&b.in.layers),
                               CntmDev{b.in.cntm.nk, b.in.cntm.knots, b.in.cntm.vals}, b.in.cutoff_threshold, mixed,
                               p.kmax, p.G, us));
-            KCHECK(autotune_tiles(ctx, make_tile_args(sc, nullptr, wls, nwl, ln, p.L, p.Lp, p.G), p.kmax, mixed, us));
+            KCHECK(autotune_tiles(ctx, make_tile_args(ctx, sc, nullptr, wls, nwl, ln, p.L, p.Lp, p.G), p.kmax, mixed, us));
             KCHECK(plan_batch(ctx, nspec, items, nwl, mixed, &p));
             key = batch_key(ctx, nspec, items, wls, nwl, precision);
         }
@@ -2906,5 +2910,6 @@ extern "C" KORG_API int korg_line_absorption_noalloc(double* alpha, const double
     ta.tier_start = tl.start;
     ta.unsorted = tl.unsorted;
     ta.far32 = 1;
+    ta.math = math;
     return noalloc_tiles(ta, G, kmax, mixed, s);
 }

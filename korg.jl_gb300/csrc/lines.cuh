@@ -647,6 +647,7 @@ struct TileArgs {
     int32_t far32;            // mixed: line_far_kernel takes the far lines of tiles with FAR_MIN_CAND32 candidates
     const float4* params_w;   // mixed, or null: wing cubics (see PrepOut)
     const float* xcub;        // mixed, or null: cubic boundaries (see PrepOut)
+    const MathTables* math;   // FP64: tables of the table-driven exp
 };
 
 // first index in [lo, hi) with a[i] >= v (a non-decreasing)
@@ -727,7 +728,7 @@ __device__ __forceinline__ float far_lorentz32(float4 p, float x2) {
 }
 __device__ __forceinline__ double far_lorentz64(const P64& p, double x2) {
     const double r2 = x2 * p.w;
-    const double au = 1 / SQRT_2 / ((r2 + 1) * p.a);
+    const double au = (1 / SQRT_2) * recip64((r2 + 1) * p.a);
     const double au2 = au * au;
     return 0.7978845608028654 * au * (1 + (3 * r2 - 1 + ((r2 - 2) * 15 * r2 + 2) * au2) * au2) * p.scale;
 }
@@ -793,6 +794,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     LineStage* s_ln = reinterpret_cast<LineStage*>(smem + 2 * size_t(a.region));  // [blockDim]
     __shared__ int32_t s_warp[32];
     __shared__ int32_t s_count;
+    const double* exp2j = a.math->exp2j;  // (read through L1: shared memory belongs to the tile shape)
 
     // gsplit >= 0: this CTA computes layer group gsplit only (its own candidate list, constants
     // and barriers), so groups of cheap and expensive layers do not wait for each other
@@ -907,7 +909,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
             const P64* s_par = reinterpret_cast<const P64*>(smem + size_t(q & 1) * a.region);
             // closed-form wing branches of one staged line at distance x
             auto add_wing = [&](double (&sum)[K], const P64* pr, double x) {
-                const double x2 = x * x, t = 1 / x2;
+                const double x2 = x * x, t = recip64(x2);
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     if (pr[k].a <= 0.2) {
@@ -929,7 +931,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
                         add_wing(acc, pr, x);
                     } else {
 #pragma unroll
-                        for (int k = 0; k < K; k++) acc[k] += voigt64(pr[k].a, x * pr[k].inv_s) * pr[k].scale;
+                        for (int k = 0; k < K; k++) acc[k] += voigt64t(pr[k].a, x * pr[k].inv_s, exp2j) * pr[k].scale;
                     }
                 }
             }
@@ -952,8 +954,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     if constexpr (FAR) {
         if (use_far) {
             // node sums of the line slots -> Chebyshev coefficients -> this thread's wavelength
-            double* s_node = s_alpha;                                                    // [SL][TW]
-            double* s_cf = reinterpret_cast<double*>(s_ln + nthr);                       // [SL][FAR_P + 1]
+            double* s_node = s_alpha;  // [SL][TW], then per layer FAR_P node values and FAR_P coefficients
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < K; k++) s_node[(goff + k) * TW + jl] = accn[k];
@@ -966,21 +967,23 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
             }
             __syncthreads();
             for (int e = tid; e < SL * FAR_P; e += nthr)
-                s_cf[(e / FAR_P) * (FAR_P + 1) + e % FAR_P] = far_coef(s_node + (e / FAR_P) * TW, 1, e % FAR_P);
+                s_node[(e / FAR_P) * TW + FAR_P + e % FAR_P] = far_coef(s_node + (e / FAR_P) * TW, 1, e % FAR_P);
             __syncthreads();
+            const double* cf = s_node + goff * TW + FAR_P;
             const double u = hw > 0 ? fmin(fmax(((wl_j - wl_ref) - hw) / hw, -1.0), 1.0) : 0.0;
             double t0 = 1.0, t1 = u, far[K];
 #pragma unroll
-            for (int k = 0; k < K; k++) far[k] = s_cf[(goff + k) * (FAR_P + 1)];
+            for (int k = 0; k < K; k++) far[k] = cf[k * TW];
             for (int n = 1; n < FAR_P; n++) {
 #pragma unroll
-                for (int k = 0; k < K; k++) far[k] = fma(s_cf[(goff + k) * (FAR_P + 1) + n], t1, far[k]);
+                for (int k = 0; k < K; k++) far[k] = fma(cf[k * TW + n], t1, far[k]);
                 const double t2 = fma(2 * u, t1, -t0);
                 t0 = t1;
                 t1 = t2;
             }
 #pragma unroll
             for (int k = 0; k < K; k++) acc[k] += far[k];
+            __syncthreads();  // s_alpha overlays the coefficients
         }
     }
     // alpha += accumulated lines, staged through shared memory for coalesced updates

@@ -36,7 +36,7 @@ def _opacity(gpu_lib, oracle_lib, inp, wls, precision, tile=None):
     return got, ref
 
 
-@pytest.mark.parametrize("L,tile", [(56, None), (56, (64, 0, 1)), (56, (96, 0, 0)), (80, None), (130, None)])
+@pytest.mark.parametrize("L,tile", [(56, None), (56, (64, 0, 1)), (56, (96, 0, 0)), (56, (128, 169, 1)), (80, None), (130, None)])
 @pytest.mark.parametrize("extra", [0, 1, 63, 64, 65, 127])
 def test_fp64_far_lines_match_oracle(gpu_lib, oracle_lib, L, tile, extra):
     """The sum of a few hundred positive terms and the 16-node series both round at 1e-15 each: 1e-12."""
@@ -45,6 +45,16 @@ def test_fp64_far_lines_match_oracle(gpu_lib, oracle_lib, L, tile, extra):
     inp = _inputs(L, 5000, 5010, 400)
     wls = inp.wls.all_wls[:512 + extra] if extra else inp.wls.all_wls[:512]
     got, ref = _opacity(gpu_lib, oracle_lib, inp, wls, "fp64", tile)
+    np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("lo,hi", [(7.0, 9.0), (9.5, 11.5), (8.0, 12.5)])
+def test_fp64_profile_branches_match_oracle(gpu_lib, oracle_lib, lo, hi):
+    """Damping from a = 1e-4 to some 30, so that every branch of the Hjerting function and both far
+    series occur; each term is a few roundings of positive factors: 1e-12."""
+    inp = _inputs(56, 5000, 5010, 120)
+    inp.linelist.gamma_rad[:] = 10.0 ** np.random.default_rng(3).uniform(lo, hi, 120)
+    got, ref = _opacity(gpu_lib, oracle_lib, inp, inp.wls.all_wls[:700], "fp64")
     np.testing.assert_allclose(got, ref, rtol=1e-12, atol=0)
 
 
