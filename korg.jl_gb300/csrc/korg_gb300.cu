@@ -1136,6 +1136,30 @@ __global__ void fill_kernel(double* x, int n, const double* v, double scale) {
     if (i < n) x[i] = *v * scale;
 }
 
+// Tile arguments of `n` prologues of one line list whose scratch pieces lie `stride` bytes apart, each with
+// an opacity of its own, `slice` elements apart.
+__global__ void tile_series_kernel(TileArgs base, int n, size_t stride, size_t slice, TileArgs* out) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= n) return;
+    auto shift = [&](auto*& p) {
+        using P = std::remove_reference_t<decltype(p)>;
+        if (p) p = reinterpret_cast<P>(reinterpret_cast<uintptr_t>(p) + size_t(v) * stride);
+    };
+    base.alpha += size_t(v) * slice;
+    shift(base.params);
+    shift(base.params_w);
+    shift(base.xfar);
+    shift(base.xcub);
+    shift(base.amask);
+    shift(base.lb);
+    shift(base.ub);
+    shift(base.tier_idx);
+    shift(base.tier_ci);
+    shift(base.tier_start);
+    shift(base.unsorted);
+    out[v] = base;
+}
+
 __global__ void scale_kernel(double* x, int64_t n, double s) {
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
         x[i] *= s;
@@ -2398,6 +2422,9 @@ KORG_API int korg_apply_rotation_vjp_dev(korg_ctx* ctx, const double* wls, int64
     return KORG_OK;
 }
 
+// Scratch that the prologues of one launch of a cross-section table share.
+constexpr size_t MX_SCRATCH = size_t(256) << 20;
+
 KORG_API int korg_molecular_cross_section_dev(korg_ctx* ctx, const korg_lines* lines, const double* wls,
                                               int64_t nwl, const double* T, const double* inv_U, int32_t nT,
                                               const double* vmic_vals, int32_t nv, double cutoff_alpha,
@@ -2412,10 +2439,33 @@ KORG_API int korg_molecular_cross_section_dev(korg_ctx* ctx, const korg_lines* l
     // molecule's n / U = (1 / cutoff_alpha) / U(T), continuum 1 and cutoff threshold 1, so a line
     // is truncated where its absorption coefficient per molecule falls to cutoff_alpha; the vdW
     // perturber density is NaN (molecular lines have no vdW broadening)
-    const size_t bytes = sizeof(double) * 6 * size_t(nT);
-    KCHECK(ensure(ctx, ctx->mx_layers, bytes));
+    const bool mixed = precision == KORG_MIXED;
+    const LinesDev ln = lines_dev(lines);
+    int kmax = 0;
+    const int G = layer_groups(nT, &kmax), Lp = G * kmax;
+    // The microturbulences of one table are one launch of tiles: its 79 x 4 CTAs (10,001 wavelengths, 51
+    // temperatures) would leave SMs with 2 and with 3 of them 11 times over.  As many at a time as their
+    // prologues' scratch fits MX_SCRATCH (at least one).  1,000 lines: 77.2 -> 38.3 ms.
+    const size_t per = G > 0 ? line_scratch(nullptr, ln.n, nT, Lp, G, mixed, nullptr) : 0;
+    int series = per > 0 ? int(std::min<size_t>(size_t(nv), std::max<size_t>(MX_SCRATCH / per, 1))) : 1;
+    if (ln.n == 0 || ln.n > INT32_MAX || nwl > INT32_MAX - 1) series = 1;
+    const size_t o_targs = sizeof(double) * 6 * size_t(nT) + sizeof(unsigned long long);
+    const auto fits = [&] {
+        return ctx->lines_scratch.cap >= per * series && ctx->mx_layers.cap >= o_targs + sizeof(TileArgs) * series;
+    };
+    if (series > 1 && !fits()) {  // where it cannot grow (captured, or out of memory): one by one, as before
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+            ensure(ctx, ctx->lines_scratch, per * series) != KORG_OK) {
+            cudaGetLastError();
+            series = 1;
+        }
+    }
+    KCHECK(ensure(ctx, ctx->mx_layers, series > 1 ? o_targs + sizeof(TileArgs) * series : sizeof(double) * 6 * size_t(nT)));
     double* d = static_cast<double*>(ctx->mx_layers.p);
     double* xi = d + 4 * nT;
+    auto* d_next = reinterpret_cast<unsigned long long*>(d + 6 * nT);
+    auto* d_targs = reinterpret_cast<TileArgs*>(d_next + 1);
     molxs_layers_kernel<<<(nT + 127) / 128, 128, 0, s>>>(inv_U, nT, cutoff_alpha, d);
     KCUDA(cudaGetLastError());
     KCHECK(reset_counters(ctx, s));
@@ -2423,11 +2473,35 @@ KORG_API int korg_molecular_cross_section_dev(korg_ctx* ctx, const korg_lines* l
     const CntmDev cn{1, nullptr, d + 3 * nT};
     const size_t slice = size_t(nwl) * nT;
     KCUDA(cudaMemsetAsync(table, 0, sizeof(double) * slice * nv, s));
-    for (int v = 0; v < nv; v++) {
-        fill_kernel<<<(nT + 127) / 128, 128, 0, s>>>(xi, nT, vmic_vals + v, 1e5);  // km/s -> cm/s
+    const bool tune = ctx->autotune && !ctx->capturing && worth_tuning(nwl, ln.n);
+    for (int v0 = 0; v0 < nv; v0 += series) {
+        const int m = std::min(series, nv - v0);
+        TileArgs first{};
+        for (int v = v0; v < v0 + m; v++) {
+            fill_kernel<<<(nT + 127) / 128, 128, 0, s>>>(xi, nT, vmic_vals + v, 1e5);  // km/s -> cm/s
+            KCUDA(cudaGetLastError());
+            if (series == 1) {
+                KCHECK(run_line_absorption(ctx, table + v * slice, wls, nwl, ln, lay, cn, 1.0, mixed, s));
+                continue;
+            }
+            LineScratch sc;
+            line_scratch(static_cast<unsigned char*>(ctx->lines_scratch.p) + per * (v - v0), ln.n, nT, Lp, G, mixed, &sc);
+            KCHECK(prep_lines(ctx, sc, wls, nwl, ln, lay, cn, 1.0, mixed, kmax, G, s));
+            if (v == v0) first = make_tile_args(ctx, sc, table + v * slice, wls, nwl, ln, nT, Lp, G);
+        }
+        if (series == 1) continue;
+        if (tune) KCHECK(autotune_tiles(ctx, first, kmax, mixed, s));
+        TileGeom g;
+        if (!tile_geom(mixed, Lp, G, tile_cfg(ctx, nT, mixed), &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
+        first.stage = g.stage;
+        first.region = g.region;
+        first.split = g.split;
+        tile_series_kernel<<<(m + 127) / 128, 128, 0, s>>>(first, m, per, slice, d_targs);
         KCUDA(cudaGetLastError());
-        KCHECK(run_line_absorption(ctx, table + v * slice, wls, nwl, lines_dev(lines), lay, cn, 1.0,
-                                   precision == KORG_MIXED, s));
+        KCUDA(cudaMemsetAsync(d_next, 0, sizeof *d_next, s));
+        const int groups = g.split ? G : 1;
+        const TileQueue q{d_targs, m, groups, int64_t(m) * ((nwl + g.tw - 1) / g.tw) * groups, d_next};
+        KCHECK(run_tiles(ctx, TileArgs{}, kmax, g, &q, mixed, ln.n, s));
     }
     scale_kernel<<<ctx->sms * 4, 256, 0, s>>>(table, int64_t(slice) * nv, cutoff_alpha);
     KCUDA(cudaGetLastError());

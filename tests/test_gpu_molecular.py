@@ -35,6 +35,22 @@ def test_cross_section_table_matches_oracle(gpu_lib, oracle_lib):
     assert np.all(tab >= 0) and tab.max() > 0
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,nT,nv,hi", [(1, 1, 2, 15000.01), (300, 14, 3, 15001.27), (300, 51, 11, 15001.28),
+                                        (20000, 51, 7, 15001.0)])
+def test_cross_section_series_equal_single_tables(gpu_lib, precision, n, nT, nv, hi):
+    """The microturbulences of a table share launches (20,000 lines: scratch for a few at a time); each
+    gives the bits that a table of its own gives."""
+    from korg_gb300.molecular import MolecularCrossSection
+    from korg_gb300.wavelengths import Wavelengths
+    ll, wls = _co_lines(n), Wavelengths((15000.0, hi, 0.01))
+    vm, lt = np.linspace(0.0, 4.0, nv), np.linspace(3.0, 4.0, nT)
+    tab = MolecularCrossSection(ll, wls, vmic_vals=vm, log_temp_vals=lt, precision=precision).table_numpy()
+    for v in range(nv):
+        one = MolecularCrossSection(ll, wls, vmic_vals=vm[v:v + 1], log_temp_vals=lt, precision=precision)
+        assert np.array_equal(tab[v], one.table_numpy()[0])
+
+
 def test_cross_section_interpolation(gpu_lib):
     torch = pytest.importorskip("torch")
     from scipy.interpolate import RegularGridInterpolator
