@@ -7,7 +7,8 @@
 //   rt_adjoint_kernel    one warp per wavelength column: tau by a warp-shuffle prefix scan,
 //                        E2 / exp per layer in parallel, the segment partial derivatives of the
 //                        exponential-integral formal solution, and the reverse (suffix) scan of
-//                        the tau recursion.  Outputs dL/dalpha[l, j] (the opacity cotangent G),
+//                        the tau recursion; the continuum's pass per knot interval where its flux is
+//                        a series there.  Outputs dL/dalpha[l, j] (the opacity cotangent G),
 //                        and per-layer sums through the Planck source function and alpha_ref.
 //   line_adj_kernel      (line, window chunk) items, one thread per layer, a sequential walk
 //                        over the chunk's wavelengths: sums of G * dphi/d(amplitude, sigma,
@@ -140,10 +141,13 @@ struct RtAdjArgs {
     double* dT;               // out [L] (+=): through the source function
     double* daref;            // out [L] (+=): through alpha_ref
     double* dvals;            // out [L][nk] (+=) or null: continuum knots
+    const double* cseg;       // [nk - 1][CSEG_P] of cntm_segment_kernel, or null
+    double* wnode;            // [nk - 1][CSEG_P] cotangents of the intervals' nodes, zero before the first launch
 };
 
 constexpr int RTA_WARPS = 4;
 constexpr int RTA_LMAX = 128;
+constexpr double RTA_THIN = 0.05;  // optical depth below which G + 1 and H + 1 are kept
 constexpr int RTA_ARRAYS = 14;  // per-warp column arrays of the kernel's dynamic shared memory
 
 // Per-warp scratch of one column (each array L + 1 doubles of dynamic shared memory).
@@ -151,70 +155,42 @@ struct RtaCol {
     double *S, *tau, *e2, *d2, *ex, *ib, *ta, *tb, *sa, *sb, *Sbar, *col, *g, *gc;
 };
 
-// Taylor coefficients of the piecewise E2 (RadiativeTransfer.jl:441-490) around x0 = 2..8
-__device__ __constant__ double c_e2poly[7][6] = {
-    {0.037534261820486914, -0.04890051070806112, 0.033833820809153176, -0.016916910404576574,
-     0.007048712668573576, -0.0026785108140579598},
-    {0.010641925085272673, -0.013048381094197039, 0.008297844727977323, -0.003687930990212144,
-     0.0013061422257001345, -0.0003995258572729822},
-    {0.0031982292493385146, -0.0037793524098489054, 0.0022894548610917728, -0.0009539395254549051,
-     0.00031003034577284415, -8.466213288412284e-5},
-    {0.000996469042708825, -0.0011482955912753257, 0.0006737946999085467, -0.00026951787996341863,
-     8.310134632205409e-5, -2.1202073223788938e-5},
-    {0.0003182574636904001, -0.0003600824521626587, 0.00020656268138886323, -8.032993165122457e-5,
-     2.390771775334065e-5, -5.8334831318151185e-6},
-    {0.00010350984428214624, -0.00011548173161033826, 6.513442611103688e-5, -2.4813114708966427e-5,
-     7.200234178941151e-6, -1.7027366981408086e-6},
-    {3.413764515111217e-5, -3.76656228439249e-5, 2.096641424390699e-5, -7.862405341465122e-6,
-     2.2386015208338193e-6, -5.173353514609864e-7}};
-
-// d/dx of that piecewise approximation of E2, branch by branch (the derivative ForwardDiff
-// takes), given e2 = E2(x) and ex = exp(-x) of the same branch.
-__device__ __forceinline__ double expint2_deriv(double x, double e2, double ex, const MathTables& t) {
+// E2(x) as expint2_lanes evaluates it, with d/dx of that piecewise approximation, piece by piece (the
+// derivative ForwardDiff takes); ex = exp(-x).
+__device__ __forceinline__ double expint2_and_deriv(double x, double ex, const double* mid, const MathTables& t,
+                                                    double& d2) {
     if (x < 1.1) {  // E2 = 1 + x (ln x + EM - 1) + x Q(x)
-        const double EM = 0.57721566490153286060651209008240243104215933593992;
-        const double c2 = 0.08333333333333333, c3 = -0.013888888888888888, c4 = 0.0020833333333333333;
-        const double Q = (-0.5 + (c2 + (c3 + c4 * x) * x) * x) * x;
-        const double dQ = -0.5 + (2 * c2 + (3 * c3 + 4 * c4 * x) * x) * x;
-        return flog64(x, t) + EM + Q + x * dQ;
-    }
-    if (x < 9) {
-        const int k = x < 2.5 ? 0 : (x < 3.5 ? 1 : (x < 4.5 ? 2 : (x < 5.5 ? 3 : (x < 6.5 ? 4 : (x < 7.5 ? 5 : 6)))));
-        const double y = x - (2 + k);
-        const double* a = c_e2poly[k];
-        return a[1] + y * (2 * a[2] + y * (3 * a[3] + y * (4 * a[4] + y * 5 * a[5])));
-    }
-    // E2 = e^-x u R(u), u = 1/x
-    const double u = recip64(x);
-    const double R = 1 + (-2 + (6 + (-24 + 120 * u) * u) * u) * u;
-    const double dR = -2 + (12 + (-72 + 480 * u) * u) * u;
-    return -e2 - ex * u * u * (R + u * dR);
-}
-
-// E2(x) as expint2_ex evaluates it, with d/dx of the same branch (expint2_deriv) from one
-// logarithm: for x < 1.1 both need ln x.
-__device__ __forceinline__ double expint2_and_deriv(double x, double ex, const MathTables& t, double& d2) {
-    if (x < 1.1 && x != 0) {  // E2 = 1 + x (ln x + EM - 1) + x Q(x)
         const double EM = 0.57721566490153286060651209008240243104215933593992;
         const double c2 = 0.08333333333333333, c3 = -0.013888888888888888, c4 = 0.0020833333333333333;
         const double lg = flog64(x, t);
         const double Q = (-0.5 + (c2 + (c3 + c4 * x) * x) * x) * x;
         const double dQ = -0.5 + (2 * c2 + (3 * c3 + 4 * c4 * x) * x) * x;
         d2 = lg + EM + Q + x * dQ;
-        return 1 + ((lg + EM - 1) + Q) * x;
+        return x != 0 ? 1 + ((lg + EM - 1) + Q) * x : 1.0;
     }
-    const double e2 = expint2_ex(x, ex, t);
-    d2 = expint2_deriv(x, e2, ex, t);
+    if (x < 9) {  // Taylor rows (RadiativeTransfer.jl:441-490)
+        const double* r = mid + E2_ROW * (expint2_piece(x) - 2);
+        const double y = x - r[0];
+        d2 = r[2] + y * (2 * r[3] + y * (3 * r[4] + y * (4 * r[5] + y * 5 * r[6])));
+        return r[1] + (r[2] + (r[3] + (r[4] + (r[5] + r[6] * y) * y) * y) * y) * y;
+    }
+    // E2 = e^-x u R(u), u = 1/x
+    const double u = recip64(x);
+    const double R = 1 + (-2 + (6 + (-24 + 120 * u) * u) * u) * u;
+    const double dR = -2 + (12 + (-72 + 480 * u) * u) * u;
+    const double e2 = ex * R * u;
+    d2 = -e2 - ex * u * u * (R + u * dR);
     return e2;
 }
 
 // One transfer pass over the column `al` (global or shared) with cotangent w of 2 pi I unit:
 // writes dL/dalpha of the pass into gout[l], adds dL/dS into c.Sbar and dL/dalpha_ref into
-// s_daref (shared, atomically).  s_iaref = 1 / alpha_ref.  No FP64 division: one Newton
+// s_daref (shared, atomically).  al may be c.col and gout c.gc, which hold H and G in between.
+// s_iaref = 1 / alpha_ref.  No FP64 division: one Newton
 // reciprocal of each segment's dtau (recip64) serves its three quotients.
 __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, double w, const double* s_fac,
                                             const double* s_dlt, const double* s_iaref, int L, const MathTables& mt,
-                                            double* gout, double* s_daref, int lane) {
+                                            const double* e2_mid, double* gout, double* s_daref, int lane) {
     // optical depth (RadiativeTransfer.jl:244-253): ib, trapezoid increments, warp scans
     for (int l = lane; l < L; l += 32) c.ib[l] = al[l] * s_fac[l];
     __syncwarp();
@@ -240,13 +216,29 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
     }
     for (int l = lane; l <= L; l += 32) {
         if (l < L) {
-            const double t = c.tau[l];
-            const double ex = l == 0 ? 1.0 : fexp64(-t, mt);
-            double d2 = 0.0;  // tau_0 = 0 is not a variable
-            const double e2 = l == 0 ? 1.0 : expint2_and_deriv(t, ex, mt, d2);
-            c.ex[l] = ex;
-            c.e2[l] = e2;
-            c.d2[l] = d2;
+            if (l <= lc) {  // (deeper layers enter no segment)
+                const double t = c.tau[l];
+                const double ex = l == 0 ? 1.0 : fexp64(-t, mt);
+                double d2 = 0.0;  // tau_0 = 0 is not a variable
+                const double e2 = l == 0 ? 1.0 : expint2_and_deriv(t, ex, e2_mid, mt, d2);
+                c.ex[l] = ex;
+                c.e2[l] = e2;
+                c.d2[l] = d2;
+                // G = t E2 - e^-t and H = t G - e^-t; near the surface G + 1 and H + 1, with
+                // 1 - e^-t = t - q by its series: differences over a segment there are of the order of
+                // its depth and (H) its square, which 1e-16 of G = H = -1 would drown (depth 1e-6: error of
+                // the H term 7e-3 -> 3e-6)
+                if (t < RTA_THIN) {
+                    const double q = t * t *
+                        (1.0 / 2 - t * (1.0 / 6 - t * (1.0 / 24 - t * (1.0 / 120 - t * (1.0 / 720 - t * (1.0 / 5040 -
+                                   t * (1.0 / 40320 - t * (1.0 / 362880))))))));
+                    c.gc[l] = t * e2 + (t - q);
+                    c.col[l] = t * c.gc[l] - q;
+                } else {
+                    c.gc[l] = t * e2 - ex;
+                    c.col[l] = t * c.gc[l] - ex;
+                }
+            }
             c.tb[l] = 0.0;
             c.sb[l] = 0.0;
         }
@@ -269,9 +261,9 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
         const double iD = recip64(D);
         const double m = (Sb - Sa) * iD;
         const double bb = Sa - m * ta_;
-        const double Pb = 0.5 * ((tb_ * c.e2[l] - c.ex[l]) - (ta_ * c.e2[l - 1] - c.ex[l - 1]));
-        const double Pm = (1.0 / 3.0) * ((tb_ * tb_ * c.e2[l] - c.ex[l] * (tb_ + 1)) -
-                                         (ta_ * ta_ * c.e2[l - 1] - c.ex[l - 1] * (ta_ + 1)));
+        const double seam = double(int(ta_ < RTA_THIN) - int(tb_ < RTA_THIN));
+        const double Pb = 0.5 * (c.gc[l] - (c.gc[l - 1] - seam));
+        const double Pm = (1.0 / 3.0) * (c.col[l] - (c.col[l - 1] - seam));
         const double Q = Pm - ta_ * Pb;  // total derivative through m (b depends on m)
         const double Ctb = dC(tb_, c.e2[l], c.d2[l], c.ex[l], m, bb);
         const double Cta = l == 1 ? 0.0 : dC(ta_, c.e2[l - 1], c.d2[l - 1], c.ex[l - 1], m, bb);
@@ -309,12 +301,33 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
     __syncwarp();
 }
 
+// Lagrange polynomial of node q of a knot interval (cntm_segment_kernel's nodes) at u = 1 - 2 t
+__device__ __forceinline__ double cseg_basis(int q, double u) {
+    double t0 = 1.0, t1 = u, v = 0.5;
+    for (int n = 1; n < CSEG_P; n++) {
+        v = fma((n == CSEG_P - 1 ? 0.5 : 1.0) * cos_pi7(n * q), t1, v);
+        const double t2 = fma(2 * u, t1, -t0);
+        t0 = t1;
+        t1 = t2;
+    }
+    return v * ((q == 0 || q == CSEG_P - 1 ? 1.0 : 2.0) / (CSEG_P - 1));
+}
+
+// The continuum pass's outputs are linear in its cotangents and as smooth in wavelength within a knot
+// interval as the continuum flux itself, so where cntm_segment_kernel found an interval's flux to be a
+// series over its nodes (a.cseg not NaN), the columns there only add their cotangents, times the nodes'
+// Lagrange polynomials, to the nodes' (a.wnode), and a second launch (NODES) does the pass at the nodes.
+// FP64 pipe and latency bound, some 150 operations per (layer, column, pass).  100,001 columns x 72 layers, both
+// passes: 2.70 -> 1.38 ms, and 0.1 for the intervals and their nodes.
+template <bool NODES>
 __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a) {
     __shared__ MathTables s_math;
+    __shared__ double s_e2[7 * E2_ROW];
     __shared__ double s_fac[RTA_LMAX], s_dlt[RTA_LMAX], s_iaref[RTA_LMAX], s_iT[RTA_LMAX], s_ikT[RTA_LMAX];
     __shared__ double s_dT[RTA_LMAX], s_dar[RTA_LMAX];
     extern __shared__ double s_cols[];  // [warps][RTA_ARRAYS][L + 1]
     load_math_tables(s_math, a.math);
+    if (threadIdx.x < 7 * E2_ROW) s_e2[threadIdx.x] = c_e2_mid[threadIdx.x];
     const int L = a.L;
     for (int l = threadIdx.x; l < L; l += blockDim.x) {
         s_fac[l] = a.tau_ref[l] / a.alpha_ref[l];
@@ -332,12 +345,32 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
     double** f[RTA_ARRAYS] = {&c.S, &c.tau, &c.e2, &c.d2, &c.ex, &c.ib, &c.ta, &c.tb, &c.sa, &c.sb, &c.Sbar, &c.col,
                               &c.g, &c.gc};
     for (int k = 0; k < RTA_ARRAYS; k++) *f[k] = base + k * (L + 1);
-    const bool two = a.cn.nk > 0;
-    const int64_t stride = int64_t(gridDim.x) * RTA_WARPS;
-    for (int64_t j = int64_t(blockIdx.x) * RTA_WARPS + warp; j < a.nwl; j += stride) {
-        const double wl = a.wls[j];
-        const double wf = a.dflux ? a.dflux[j] * 2 * PI * a.unit : 0.0;
-        const double wc = (two && a.dcntm) ? a.dcntm[j] * 2 * PI * a.unit : 0.0;
+    const bool two = a.cn.nk > 0 && a.dcntm;
+    const int64_t stride = int64_t(gridDim.x) * RTA_WARPS, ncol = NODES ? (a.cn.nk - 1) * CSEG_P : a.nwl;
+    for (int64_t j = int64_t(blockIdx.x) * RTA_WARPS + warp; j < ncol; j += stride) {
+        double wl, wf = 0.0, wc;
+        KnotPos kp{0, 0.0};
+        bool pass_c = true;
+        if constexpr (NODES) {
+            wc = a.wnode[j];
+            if (wc == 0.0) continue;
+            const int m = int(j % CSEG_P);
+            kp.i = j / CSEG_P;
+            kp.t = m == 0 ? 0.0 : (m == CSEG_P - 1 ? 1.0 : 0.5 - 0.5 * cos_pi7(m));
+            const double w0 = a.cn.knots[kp.i];
+            wl = w0 + kp.t * (a.cn.knots[kp.i + 1] - w0);
+        } else {
+            wl = a.wls[j];
+            wf = a.dflux ? a.dflux[j] * 2 * PI * a.unit : 0.0;
+            wc = two ? a.dcntm[j] * 2 * PI * a.unit : 0.0;
+            pass_c = two;
+            if (a.cn.nk > 0) kp = knot_pos(a.cn.knots, a.cn.nk, wl);
+            if (two && a.cseg && isfinite(wc) && kp.t >= 0.0 && kp.t <= 1.0 && !isnan(a.cseg[kp.i * CSEG_P])) {
+                pass_c = false;
+                if (lane < CSEG_P && wc != 0.0)
+                    atomicAdd(a.wnode + kp.i * CSEG_P + lane, wc * cseg_basis(lane, 1.0 - 2.0 * kp.t));
+            }
+        }
         const double pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl);
         const double hcw = HPLANCK_CGS * C_CGS / wl;
         const double ipre = recip64(pre);
@@ -346,17 +379,19 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
             c.Sbar[l] = 0.0;
         }
         __syncwarp();
-        rt_adj_pass(c, a.alpha + j * L, wf, s_fac, s_dlt, s_iaref, L, s_math, c.g, s_dar, lane);
-        if (two) {
+        if constexpr (!NODES)
+            rt_adj_pass(c, a.alpha + j * L, wf, s_fac, s_dlt, s_iaref, L, s_math, s_e2, c.g, s_dar, lane);
+        if (pass_c) {
             // continuum-only column (src/synthesize.jl:287-291), as the forward interpolates it
-            const KnotPos kp = knot_pos(a.cn.knots, a.cn.nk, wl);
             for (int l = lane; l < L; l += 32) c.col[l] = knot_eval(a.cn.vals + int64_t(l) * a.cn.nk, a.cn.nk, kp);
             __syncwarp();
-            rt_adj_pass(c, c.col, wc, s_fac, s_dlt, s_iaref, L, s_math, c.gc, s_dar, lane);
+            rt_adj_pass(c, c.col, wc, s_fac, s_dlt, s_iaref, L, s_math, s_e2, c.gc, s_dar, lane);
+        }
+        if (a.cn.nk > 0) {
             // the knots feed both passes' opacity (alpha = continuum + hydrogen + lines)
             if (a.dvals) {
                 for (int l = lane; l < L; l += 32) {
-                    const double gsum = c.g[l] + c.gc[l];
+                    const double gsum = (NODES ? 0.0 : c.g[l]) + (pass_c ? c.gc[l] : 0.0);
                     if (gsum == 0.0) continue;
                     double* row = a.dvals + int64_t(l) * a.cn.nk;
                     if (a.cn.nk == 1) {
@@ -374,6 +409,7 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
             const double x = hcw * s_ikT[l];
             const double d = c.Sbar[l] * B * (x * s_iT[l]) * (1.0 + B * ipre);
             if (d != 0.0) atomicAdd(s_dT + l, d);
+            if constexpr (NODES) continue;
             if (a.g32)
                 static_cast<float*>(a.G)[j * L + l] = float(c.g[l]);
             else
