@@ -354,7 +354,7 @@ bool tile_geom(bool mixed, int Lp, int G, TileCfg c, TileGeom* g) {
 TileCfg default_tile(bool) { return TileCfg{TILE_TW, 0, 1}; }
 
 // far_lines: whether some tile can hold FAR_MIN_CAND32 candidates (mixed: line_far_kernel runs first).
-template <bool MIXED, int KMAX, int MAXT, int MINB>
+template <bool MIXED, int KMAX, int MAXT, int MINB, int SUB = 1>
 int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* q, bool far_lines, cudaStream_t s) {
     ta.stage = g.stage;
     ta.region = g.region;
@@ -375,10 +375,10 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
         const int64_t grid = std::min<int64_t>(q->nitems, int64_t(ctx->sms) * std::max(per_sm, 1));
         if (grid > 0) kern<<<unsigned(grid), g.threads, g.smem, s>>>(*q);
     } else {
-        auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB>;
+        auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB, SUB>;
         KCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
         const int64_t tiles = (ta.nwl + g.tw - 1) / g.tw;
-        kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) : 1u), g.threads, g.smem, s>>>(ta);
+        kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) * SUB : 1u), g.threads, g.smem, s>>>(ta);
     }
     KCUDA(cudaGetLastError());
     return KORG_OK;
@@ -392,6 +392,15 @@ int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g
         if (kmax == 16) return launch_tile<true, 16, 256, 2>(ctx, ta, g, q, far_lines, s);
         return launch_tile<true, 32, 256, 2>(ctx, ta, g, q, far_lines, s);
     } else {
+        // Fewer CTAs than the GPU holds (4 of 128 threads per SM): half a layer group each, for twice the
+        // warps, as the FP64 pipe wants more than the 4 or 8 per SM that whole groups give.
+        // line_absorption! of 2,000 lines, 79 x 4 CTAs: 4.28 -> 3.54 ms; FP64 gradient over 20 A, 16 x 4:
+        // 5.75 -> 4.62 ms.
+        const int64_t ctas = (ta.nwl + g.tw - 1) / g.tw * g.G;
+        if (!q && g.split && g.threads <= 128 && ctas < int64_t(ctx->sms) * 4) {
+            if (kmax == 14) return launch_tile<false, 7, 128, 6, 2>(ctx, ta, g, q, far_lines, s);
+            if (kmax == 16) return launch_tile<false, 8, 128, 6, 2>(ctx, ta, g, q, far_lines, s);
+        }
         if (kmax == 14 && g.threads <= 256) return launch_tile<false, 14, 256, 2>(ctx, ta, g, q, far_lines, s);
         if (kmax == 14) return launch_tile<false, 14, 512, 1>(ctx, ta, g, q, far_lines, s);
         if (kmax == 16) return launch_tile<false, 16, 512, 1>(ctx, ta, g, q, far_lines, s);

@@ -727,10 +727,11 @@ __device__ __forceinline__ float far_lorentz32(float4 p, float x2) {
     return 0.7978845608028654f * au * (1.f + (3.f * r2 - 1.f + ((r2 - 2.f) * 15.f * r2 + 2.f) * au2) * au2) * p.w;
 }
 __device__ __forceinline__ double far_lorentz64(const P64& p, double x2) {
-    const double r2 = x2 * p.w;
-    const double au = (1 / SQRT_2) * recip64((r2 + 1) * p.a);
-    const double au2 = au * au;
-    return 0.7978845608028654 * au * (1 + (3 * r2 - 1 + ((r2 - 2) * 15 * r2 + 2) * au2) * au2) * p.scale;
+    const double r2 = __dmul_rn(x2, p.w);
+    const double au = __dmul_rn(1 / SQRT_2, recip64(__dmul_rn(__dadd_rn(r2, 1.0), p.a)));
+    const double au2 = __dmul_rn(au, au);
+    const double c = fma(fma(__dmul_rn(__dadd_rn(r2, -2.0), 15.0), r2, 2.0), au2, fma(3.0, r2, -1.0));
+    return __dmul_rn(__dmul_rn(__dmul_rn(0.7978845608028654, au), fma(c, au2, 1.0)), p.scale);
 }
 
 // Far lines of a tile.  A line whose window covers the whole tile and whose centre lies at least
@@ -786,8 +787,9 @@ __device__ __forceinline__ double far_coef(const double* v, int stride, int n) {
 // FP64 tile: TW = blockDim.x / G wavelengths x all layers (or, with gsplit >= 0, x the layers of
 // group gsplit), computed by one CTA.  Thread (j, g) owns wavelength j and the K consecutive
 // (padded) layers g*K .. g*K+K-1, accumulated in FP64 registers.  `smem` is the dynamic shared
-// memory of the launch (two line-constant buffers, then the LineStage array).
-template <int K>
+// memory of the launch (two line-constant buffers, then the LineStage array).  SUB = 2: gsplit counts
+// half groups of K layers (the classes remain those of the whole group).
+template <int K, int SUB = 1>
 __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile, int gsplit, unsigned char* smem) {
     const int L = a.L, Lp = a.Lp, G = a.G, B = a.stage;
     double* s_alpha = reinterpret_cast<double*>(smem);                          // [TW][SL+1], at the end
@@ -800,7 +802,9 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     // and barriers), so groups of cheap and expensive layers do not wait for each other
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int TW = gsplit >= 0 ? nthr : nthr / G;
-    const int jl = tid % TW, g = gsplit >= 0 ? gsplit : tid / TW;
+    const int jl = tid % TW, g = gsplit >= 0 ? gsplit / SUB : tid / TW;
+    const int lfirst = gsplit * K;             // gsplit >= 0: this CTA's first layer
+    if (SUB > 1 && lfirst >= L) return;        // a half group of padding
     const int SL = gsplit >= 0 ? K : Lp;       // layers of one staged line
     const int goff = gsplit >= 0 ? 0 : g * K;  // this thread's first layer within a staged line
     const int64_t j0 = tile * TW;
@@ -834,7 +838,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     const int chunks16 = SL * int(sizeof(P64) / 16);  // 16-byte pieces of one line's staged constants
     const int cb0 = tid / chunks16, cr0 = tid - cb0 * chunks16;       // this thread's first staged piece
     const int cdb = nthr / chunks16, cdr = nthr - cdb * chunks16;     // and the step between its pieces
-    const int64_t src0 = gsplit >= 0 ? int64_t(g) * K * int64_t(sizeof(P64) / 16) : 0;
+    const int64_t src0 = gsplit >= 0 ? int64_t(lfirst) * int64_t(sizeof(P64) / 16) : 0;
     for (int tier = 0; tier < NTIER; tier++)
     for (int64_t base = s_tier[tier][0]; base < s_tier[tier][1]; base += nthr) {
         const int64_t pidx = base + tid;
@@ -861,7 +865,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
             const double wl0 = a.wl[i];
             const double dist = wl0 < wl_ref ? wl_ref - wl0 : (wl0 > wl_last ? wl0 - wl_last : 0.0);
             uint32_t cls = 0;
-            const int g_lo = gsplit >= 0 ? gsplit : 0, g_hi = gsplit >= 0 ? gsplit + 1 : G;
+            const int g_lo = gsplit >= 0 ? g : 0, g_hi = gsplit >= 0 ? g + 1 : G;
             const uint32_t wing = use_far && lbi <= j0 && ubi >= jlast && dist >= FAR_KAPPA64 * (wl_last - wl_ref) ? 3u
                                                                                                                   : 2u;
             for (int gg = g_lo; gg < g_hi; gg++)
@@ -909,14 +913,13 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
             const P64* s_par = reinterpret_cast<const P64*>(smem + size_t(q & 1) * a.region);
             // closed-form wing branches of one staged line at distance x
             auto add_wing = [&](double (&sum)[K], const P64* pr, double x) {
-                const double x2 = x * x, t = recip64(x2);
+                const double x2 = __dmul_rn(x, x), t = recip64(x2);
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     if (pr[k].a <= 0.2) {
-                        const double iv = t * pr[k].c;
-                        sum[k] += (pr[k].w * iv) * (1 + iv * (1.5 + 3.75 * iv));
+                        sum[k] = __dadd_rn(sum[k], voigt_wing64(pr[k].w, __dmul_rn(t, pr[k].c)));
                     } else {
-                        sum[k] += far_lorentz64(pr[k], x2);
+                        sum[k] = __dadd_rn(sum[k], far_lorentz64(pr[k], x2));
                     }
                 }
             };
@@ -931,7 +934,8 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
                         add_wing(acc, pr, x);
                     } else {
 #pragma unroll
-                        for (int k = 0; k < K; k++) acc[k] += voigt64t(pr[k].a, x * pr[k].inv_s, exp2j) * pr[k].scale;
+                        for (int k = 0; k < K; k++)
+                            acc[k] = fma(voigt64t(pr[k].a, __dmul_rn(x, pr[k].inv_s), exp2j), pr[k].scale, acc[k]);
                     }
                 }
             }
@@ -994,7 +998,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     const int64_t nj = jlast - j0 + 1;
     double* dst = a.alpha + j0 * L;
     if (gsplit >= 0) {
-        const int l0 = g * K, nk = min(K, L - l0);
+        const int l0 = lfirst, nk = min(K, L - l0);
         for (int64_t e = tid; e < nj * nk; e += nthr) {
             const int j = int(e / nk), k = int(e - int64_t(j) * nk);
             dst[int64_t(j) * L + l0 + k] += s_alpha[j * stride + k];
@@ -1386,13 +1390,13 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
 }
 
 // One CTA per tile of one spectrum (per tile and layer group in the mixed form).
-template <bool MIXED, int K, int MAXT, int MINB>
+template <bool MIXED, int K, int MAXT, int MINB, int SUB = 1>
 __global__ void __launch_bounds__(MAXT, MINB) line_tile_kernel(TileArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     if constexpr (MIXED)
         line_tile_body_mixed<K>(a, blockIdx.x, int(blockIdx.y), smem);
     else
-        line_tile_body64<K>(a, blockIdx.x, a.split ? int(blockIdx.y) : -1, smem);
+        line_tile_body64<K, SUB>(a, blockIdx.x, a.split ? int(blockIdx.y) : -1, smem);
 }
 
 // Work queue of (spectrum, tile) items for a batch of spectra on one wavelength grid.  Item k
