@@ -392,12 +392,16 @@ int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g
         if (kmax == 16) return launch_tile<true, 16, 256, 2>(ctx, ta, g, q, far_lines, s);
         return launch_tile<true, 32, 256, 2>(ctx, ta, g, q, far_lines, s);
     } else {
-        // Fewer CTAs than the GPU holds (4 of 128 threads per SM): half a layer group each, for twice the
-        // warps, as the FP64 pipe wants more than the 4 or 8 per SM that whole groups give.
+        // Fewer CTAs than the GPU holds (4 of 128 threads per SM): half a layer group each, or 2 layers where
+        // even twice as many would leave SMs idle, as the FP64 pipe wants more warps than whole groups give.
         // line_absorption! of 2,000 lines, 79 x 4 CTAs: 4.28 -> 3.54 ms; FP64 gradient over 20 A, 16 x 4:
-        // 5.75 -> 4.62 ms.
+        // 5.75 -> 4.62 (halves) -> 4.09 ms (2 layers).
         const int64_t ctas = (ta.nwl + g.tw - 1) / g.tw * g.G;
         if (!q && g.split && g.threads <= 128 && ctas < int64_t(ctx->sms) * 4) {
+            if (ctas * 2 <= ctx->sms) {
+                if (kmax == 14) return launch_tile<false, 2, 128, 8, 7>(ctx, ta, g, q, far_lines, s);
+                if (kmax == 16) return launch_tile<false, 2, 128, 8, 8>(ctx, ta, g, q, far_lines, s);
+            }
             if (kmax == 14) return launch_tile<false, 7, 128, 6, 2>(ctx, ta, g, q, far_lines, s);
             if (kmax == 16) return launch_tile<false, 8, 128, 6, 2>(ctx, ta, g, q, far_lines, s);
         }

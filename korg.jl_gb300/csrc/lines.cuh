@@ -787,8 +787,8 @@ __device__ __forceinline__ double far_coef(const double* v, int stride, int n) {
 // FP64 tile: TW = blockDim.x / G wavelengths x all layers (or, with gsplit >= 0, x the layers of
 // group gsplit), computed by one CTA.  Thread (j, g) owns wavelength j and the K consecutive
 // (padded) layers g*K .. g*K+K-1, accumulated in FP64 registers.  `smem` is the dynamic shared
-// memory of the launch (two line-constant buffers, then the LineStage array).  SUB = 2: gsplit counts
-// half groups of K layers (the classes remain those of the whole group).
+// memory of the launch (two line-constant buffers, then the LineStage array).  SUB > 1: gsplit
+// counts SUB-ths of the groups, of K layers each (the classes remain those of the whole group).
 template <int K, int SUB = 1>
 __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile, int gsplit, unsigned char* smem) {
     const int L = a.L, Lp = a.Lp, G = a.G, B = a.stage;
@@ -804,7 +804,7 @@ __device__ __forceinline__ void line_tile_body64(const TileArgs& a, int64_t tile
     const int TW = gsplit >= 0 ? nthr : nthr / G;
     const int jl = tid % TW, g = gsplit >= 0 ? gsplit / SUB : tid / TW;
     const int lfirst = gsplit * K;             // gsplit >= 0: this CTA's first layer
-    if (SUB > 1 && lfirst >= L) return;        // a half group of padding
+    if (SUB > 1 && lfirst >= L) return;        // nothing but padding
     const int SL = gsplit >= 0 ? K : Lp;       // layers of one staged line
     const int goff = gsplit >= 0 ? 0 : g * K;  // this thread's first layer within a staged line
     const int64_t j0 = tile * TW;

@@ -59,18 +59,18 @@ def test_fp64_profile_branches_match_oracle(gpu_lib, oracle_lib, lo, hi):
 
 
 @pytest.mark.parametrize("L", [33, 51, 56, 64, 80])
-def test_fp64_half_groups_match_whole_groups(gpu_lib, oracle_lib, L):
-    """The first 641 points of a grid long enough for whole layer groups per CTA, and by themselves in
-    half groups (of 33 and 51 layers the last ones are padding): the same terms, in the order of their
-    tiers, which the grid's end may change: 1e-13."""
-    inp = _inputs(L, 5000, 5250, 2000)
+@pytest.mark.parametrize("n", [641, 5057])
+def test_fp64_parts_of_groups_match_whole_groups(gpu_lib, oracle_lib, L, n):
+    """The first n points of a grid long enough for whole layer groups per CTA, and by themselves in parts
+    of groups (2 layers or half; of 33 and 51 layers the last ones are padding): the same terms, in the
+    order of their tiers, which the grid's end may change: 1e-13."""
+    inp = _inputs(L, 5000, 5270, 2000)
     wls = inp.wls.all_wls
-    assert (len(wls) + 127) // 128 * ((L + 15) // 16) >= 4 * 152 or L == 33
+    assert (len(wls) + 127) // 128 * ((L + 15) // 16) >= 4 * 152
     whole, _ = _opacity(gpu_lib, oracle_lib, inp, wls, "fp64")
-    half, ref = _opacity(gpu_lib, oracle_lib, inp, wls[:641], "fp64")
-    np.testing.assert_allclose(half, ref, rtol=1e-12, atol=0)
-    if len(wls) > 641:
-        np.testing.assert_allclose(half[:512], whole[:512], rtol=1e-13, atol=0)
+    part, ref = _opacity(gpu_lib, oracle_lib, inp, wls[:n], "fp64")
+    np.testing.assert_allclose(part, ref, rtol=1e-12, atol=0)
+    np.testing.assert_allclose(part[:n // 128 * 128], whole[:n // 128 * 128], rtol=1e-13, atol=0)
 
 
 def test_fp64_far_lines_on_an_uneven_grid(gpu_lib, oracle_lib):
