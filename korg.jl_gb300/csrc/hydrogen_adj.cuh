@@ -325,6 +325,12 @@ __global__ void hline_adj_prep_kernel(StarkDev st, HLayers hl, int use_MHD, cons
     }
 }
 
+// Layer constants of a Brackett profile, on dual numbers in (T, n_e, xi).
+struct BrackettDual {
+    Dn<3> T, F0, sdop, stark_width, wstart, wend, step, GCON1, GCON2, C1, C2, G1, Pp, dbdl;
+    double Knm;
+};
+
 // brackett_prep_kernel (src/hydrogen_line_absorption.jl:147-162, :211-251, :272-369) on dual
 // numbers in (T, n_e, xi); dQ [nbr][L][3][BR_NP]: the profile's derivatives on its grid.  Mixed
 // precision (der32, q32 not null): FP32 records and q32 [nbr][L][4][BR_NP], the profile and its
@@ -339,37 +345,45 @@ __global__ void __launch_bounds__(256) brackett_adj_prep_kernel(HLayers hl, int 
     const int n = 4, m = 5 + blockIdx.x, l = blockIdx.y, L = hl.L, k = threadIdx.x;
     const int slot = ntrans + blockIdx.x;
     if (rec[int64_t(slot) * L + l].kind == HK_OFF) return;  // uniform across the CTA
-    const D T = dn_var<3>(hl.T[l], HD_T), ne = dn_var<3>(hl.ne[l], HD_NE), xi = dn_var<3>(hl.xi[l], HD_XI);
+    // what depends on the layer and the transition only, by one warp: on every thread it was a third of the
+    // kernel's FP64 operations
+    __shared__ BrackettDual s_c;
     const double E = RYDBERGH_EV * (1.0 / (n * n) - 1.0 / (m * m));
     const double wl0 = HPLANCK_EV * C_CGS / E;
-    const D F0 = dn_pow(ne, 2.0 / 3.0) * 1.25e-9;
-    const double Knm = greim_1960_Knm(n, m);
-    const D stark_width = F0 * (1.6678E-18 * Knm * C_CGS);
-    const double Hmass = 1.008 * AMU_CGS;
-    const D sdop = dn_sqrt(T * (KBOLTZ_CGS / Hmass) + xi * xi * 0.5) * (wl0 / C_CGS);
-    const D window = dn_fmax(sdop, stark_width) * 5.0;
-    const double wlmin = wls[0], wlmax = wls[nwl - 1];
-    const D wstart = dn_fmax(wlmin, wl0 - window), wend = dn_fmin(wl0 + window, wlmax);
-    const D step = (wend - wstart) / double(BR_NP - 1);
     const double nu0 = C_CGS / wl0;
-    if (k < BR_NP) s_grid[k] = (k == BR_NP - 1) ? wend : wstart + step * double(k);
+    if (threadIdx.x < 32) {
+        const D T = dn_var<3>(hl.T[l], HD_T), ne = dn_var<3>(hl.ne[l], HD_NE), xi = dn_var<3>(hl.xi[l], HD_XI);
+        const D F0 = dn_pow(ne, 2.0 / 3.0) * 1.25e-9;
+        const double Knm = greim_1960_Knm(n, m);
+        const D stark_width = F0 * (1.6678E-18 * Knm * C_CGS);
+        const double Hmass = 1.008 * AMU_CGS;
+        const D sdop = dn_sqrt(T * (KBOLTZ_CGS / Hmass) + xi * xi * 0.5) * (wl0 / C_CGS);
+        const D window = dn_fmax(sdop, stark_width) * 5.0;
+        const double wlmin = wls[0], wlmax = wls[nwl - 1];
+        const D wstart = dn_fmax(wlmin, wl0 - window), wend = dn_fmin(wl0 + window, wlmax);
+        const D ne_1_6 = dn_pow(ne, 1.0 / 6.0);
+        const double Y1WHT = (m - n <= 3) ? 1e14 : 1e13;
+        const D WTY1 = 1.0 / (1.0 + ne / Y1WHT);
+        const D Y1B = 2.0 / (1.0 + 0.012 / T * dn_sqrt(ne / T));
+        const double mm_nn = double(m * m - n * n);
+        const double C1CON = Knm / wl0 * (mm_nn * mm_nn) / double(n * n * m * m) * 1e-8;
+        const D Y1SCAL = 320.0 * (dn_pow(T / 10000.0, 0.3) / ne_1_6) * WTY1 + Y1B * (1.0 - WTY1);
+        const D C1 = F0 * 78940.0 / T * C1CON * Y1SCAL;
+        const double kl = Knm / wl0;
+        const D C2 = (F0 * F0) / (ne * 5.96E-23) * ((kl * kl) * 1e-16);
+        const BrackettDual v{T, F0, sdop, stark_width, wstart, wend, (wend - wstart) / double(BR_NP - 1),
+                             0.2 + 0.09 * dn_sqrt(T / 10000.0) / (1.0 + ne / 1.E13), 0.2 / (1.0 + ne / 1.E15), C1, C2,
+                             6.77 * dn_sqrt(C1), ne_1_6 * 0.08989 / dn_sqrt(T), 1e8 / (F0 * Knm), Knm};
+        if (threadIdx.x == 0) s_c = v;
+    }
     if (k == 0) s_red = -1;
     __syncthreads();
-    const D ne_1_6 = dn_pow(ne, 1.0 / 6.0);
-    const D GCON1 = 0.2 + 0.09 * dn_sqrt(T / 10000.0) / (1.0 + ne / 1.E13);
-    const D GCON2 = 0.2 / (1.0 + ne / 1.E15);
-    const double Y1WHT = (m - n <= 3) ? 1e14 : 1e13;
-    const D WTY1 = 1.0 / (1.0 + ne / Y1WHT);
-    const D Y1B = 2.0 / (1.0 + 0.012 / T * dn_sqrt(ne / T));
-    const double mm_nn = double(m * m - n * n);
-    const double C1CON = Knm / wl0 * (mm_nn * mm_nn) / double(n * n * m * m) * 1e-8;
-    const D Y1SCAL = 320.0 * (dn_pow(T / 10000.0, 0.3) / ne_1_6) * WTY1 + Y1B * (1.0 - WTY1);
-    const D C1 = F0 * 78940.0 / T * C1CON * Y1SCAL;
-    const double kl = Knm / wl0;
-    const D C2 = (F0 * F0) / (ne * 5.96E-23) * ((kl * kl) * 1e-16);
-    const D G1 = 6.77 * dn_sqrt(C1);
-    const D Pp = ne_1_6 * 0.08989 / dn_sqrt(T);
-    const D dbdl = 1e8 / (F0 * Knm);
+    const D T = s_c.T, F0 = s_c.F0, sdop = s_c.sdop, stark_width = s_c.stark_width, wstart = s_c.wstart,
+            wend = s_c.wend, step = s_c.step, GCON1 = s_c.GCON1, GCON2 = s_c.GCON2, C1 = s_c.C1, C2 = s_c.C2, G1 = s_c.G1,
+            Pp = s_c.Pp, dbdl = s_c.dbdl;
+    const double Knm = s_c.Knm;
+    if (k < BR_NP) s_grid[k] = (k == BR_NP - 1) ? wend : wstart + step * double(k);
+    __syncthreads();
     if (k < BR_NP) {
         const D wl = s_grid[k];
         if (C_CGS / wl.v < nu0) atomicMax(&s_red, k);
@@ -436,7 +450,8 @@ __global__ void __launch_bounds__(256) brackett_adj_prep_kernel(HLayers hl, int 
             for (int p = 0; p < 3; p++) q[(p + 1) * BR_NP + k] = float(s.d[p]);
         }
     }
-    if (k == 0) {
+    static_assert(BR_NP <= 224, "the last warp has no grid point");
+    if (k == 224) {  // while the others convolve
         using D5 = Dn<HP>;
         const D5 T5 = dn_var<HP>(hl.T[l], HD_T), ne5 = dn_var<HP>(hl.ne[l], HD_NE);
         const D5 nH5 = dn_var<HP>(hl.nH[l], HD_NH), nHe5 = dn_var<HP>(hl.nHe[l], HD_NHE);
