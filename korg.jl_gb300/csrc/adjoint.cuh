@@ -7,8 +7,7 @@
 //   rt_adjoint_kernel    one warp per wavelength column: tau by a warp-shuffle prefix scan,
 //                        E2 / exp per layer in parallel, the segment partial derivatives of the
 //                        exponential-integral formal solution, and the reverse (suffix) scan of
-//                        the tau recursion; the continuum's pass per knot interval where its flux is
-//                        a series there.  Outputs dL/dalpha[l, j] (the opacity cotangent G),
+//                        the tau recursion.  Outputs dL/dalpha[l, j] (the opacity cotangent G),
 //                        and per-layer sums through the Planck source function and alpha_ref.
 //   line_adj_kernel      (line, window chunk) items, one thread per layer, a sequential walk
 //                        over the chunk's wavelengths: sums of G * dphi/d(amplitude, sigma,
@@ -141,13 +140,10 @@ struct RtAdjArgs {
     double* dT;               // out [L] (+=): through the source function
     double* daref;            // out [L] (+=): through alpha_ref
     double* dvals;            // out [L][nk] (+=) or null: continuum knots
-    const double* cseg;       // [nk - 1][CSEG_P] of cntm_segment_kernel, or null
-    double* wnode;            // [nk - 1][CSEG_P] cotangents of the intervals' nodes, zero before the first launch
 };
 
 constexpr int RTA_WARPS = 4;
 constexpr int RTA_LMAX = 128;
-constexpr double RTA_THIN = 0.05;  // optical depth below which G + 1 and H + 1 are kept
 constexpr int RTA_ARRAYS = 14;  // per-warp column arrays of the kernel's dynamic shared memory
 
 // Per-warp scratch of one column (each array L + 1 doubles of dynamic shared memory).
@@ -185,8 +181,7 @@ __device__ __forceinline__ double expint2_and_deriv(double x, double ex, const d
 
 // One transfer pass over the column `al` (global or shared) with cotangent w of 2 pi I unit:
 // writes dL/dalpha of the pass into gout[l], adds dL/dS into c.Sbar and dL/dalpha_ref into
-// s_daref (shared, atomically).  al may be c.col and gout c.gc, which hold H and G in between.
-// s_iaref = 1 / alpha_ref.  No FP64 division: one Newton
+// s_daref (shared, atomically).  s_iaref = 1 / alpha_ref.  No FP64 division: one Newton
 // reciprocal of each segment's dtau (recip64) serves its three quotients.
 __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, double w, const double* s_fac,
                                             const double* s_dlt, const double* s_iaref, int L, const MathTables& mt,
@@ -224,20 +219,6 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
                 c.ex[l] = ex;
                 c.e2[l] = e2;
                 c.d2[l] = d2;
-                // G = t E2 - e^-t and H = t G - e^-t; near the surface G + 1 and H + 1, with
-                // 1 - e^-t = t - q by its series: differences over a segment there are of the order of
-                // its depth and (H) its square, which 1e-16 of G = H = -1 would drown (depth 1e-6: error of
-                // the H term 7e-3 -> 3e-6)
-                if (t < RTA_THIN) {
-                    const double q = t * t *
-                        (1.0 / 2 - t * (1.0 / 6 - t * (1.0 / 24 - t * (1.0 / 120 - t * (1.0 / 720 - t * (1.0 / 5040 -
-                                   t * (1.0 / 40320 - t * (1.0 / 362880))))))));
-                    c.gc[l] = t * e2 + (t - q);
-                    c.col[l] = t * c.gc[l] - q;
-                } else {
-                    c.gc[l] = t * e2 - ex;
-                    c.col[l] = t * c.gc[l] - ex;
-                }
             }
             c.tb[l] = 0.0;
             c.sb[l] = 0.0;
@@ -261,9 +242,9 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
         const double iD = recip64(D);
         const double m = (Sb - Sa) * iD;
         const double bb = Sa - m * ta_;
-        const double seam = double(int(ta_ < RTA_THIN) - int(tb_ < RTA_THIN));
-        const double Pb = 0.5 * (c.gc[l] - (c.gc[l - 1] - seam));
-        const double Pm = (1.0 / 3.0) * (c.col[l] - (c.col[l - 1] - seam));
+        const double Pb = 0.5 * ((tb_ * c.e2[l] - c.ex[l]) - (ta_ * c.e2[l - 1] - c.ex[l - 1]));
+        const double Pm = (1.0 / 3.0) * ((tb_ * tb_ * c.e2[l] - c.ex[l] * (tb_ + 1)) -
+                                         (ta_ * ta_ * c.e2[l - 1] - c.ex[l - 1] * (ta_ + 1)));
         const double Q = Pm - ta_ * Pb;  // total derivative through m (b depends on m)
         const double Ctb = dC(tb_, c.e2[l], c.d2[l], c.ex[l], m, bb);
         const double Cta = l == 1 ? 0.0 : dC(ta_, c.e2[l - 1], c.d2[l - 1], c.ex[l - 1], m, bb);
@@ -301,25 +282,12 @@ __device__ __forceinline__ void rt_adj_pass(const RtaCol& c, const double* al, d
     __syncwarp();
 }
 
-// Lagrange polynomial of node q of a knot interval (cntm_segment_kernel's nodes) at u = 1 - 2 t
-__device__ __forceinline__ double cseg_basis(int q, double u) {
-    double t0 = 1.0, t1 = u, v = 0.5;
-    for (int n = 1; n < CSEG_P; n++) {
-        v = fma((n == CSEG_P - 1 ? 0.5 : 1.0) * cos_pi7(n * q), t1, v);
-        const double t2 = fma(2 * u, t1, -t0);
-        t0 = t1;
-        t1 = t2;
-    }
-    return v * ((q == 0 || q == CSEG_P - 1 ? 1.0 : 2.0) / (CSEG_P - 1));
-}
-
-// The continuum pass's outputs are linear in its cotangents and as smooth in wavelength within a knot
-// interval as the continuum flux itself, so where cntm_segment_kernel found an interval's flux to be a
-// series over its nodes (a.cseg not NaN), the columns there only add their cotangents, times the nodes'
-// Lagrange polynomials, to the nodes' (a.wnode), and a second launch (NODES) does the pass at the nodes.
-// FP64 pipe and latency bound, some 150 operations per (layer, column, pass).  100,001 columns x 72 layers, both
-// passes: 2.70 -> 1.38 ms, and 0.1 for the intervals and their nodes.
-template <bool NODES>
+// FP64 pipe and latency bound, some 150 operations per (layer, column, pass).  E2 and its derivative from
+// table rows, so that lanes at different optical depths share a path, and no E2 below the last segment;
+// without continuum cotangents the continuum's pass, all zeros, is left out.  Gradient of
+// 30,000 lines on 400 A at 0.005 A, 72 layers: 43.6 -> 42.6 ms.  (The continuum's pass at nodes of the knot
+// intervals would save 1.3 ms more, but moves the surface layers' T gradient by the rounding of their
+// segment differences.)
 __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a) {
     __shared__ MathTables s_math;
     __shared__ double s_e2[7 * E2_ROW];
@@ -346,31 +314,12 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
                               &c.g, &c.gc};
     for (int k = 0; k < RTA_ARRAYS; k++) *f[k] = base + k * (L + 1);
     const bool two = a.cn.nk > 0 && a.dcntm;
-    const int64_t stride = int64_t(gridDim.x) * RTA_WARPS, ncol = NODES ? (a.cn.nk - 1) * CSEG_P : a.nwl;
-    for (int64_t j = int64_t(blockIdx.x) * RTA_WARPS + warp; j < ncol; j += stride) {
-        double wl, wf = 0.0, wc;
-        KnotPos kp{0, 0.0};
-        bool pass_c = true;
-        if constexpr (NODES) {
-            wc = a.wnode[j];
-            if (wc == 0.0) continue;
-            const int m = int(j % CSEG_P);
-            kp.i = j / CSEG_P;
-            kp.t = m == 0 ? 0.0 : (m == CSEG_P - 1 ? 1.0 : 0.5 - 0.5 * cos_pi7(m));
-            const double w0 = a.cn.knots[kp.i];
-            wl = w0 + kp.t * (a.cn.knots[kp.i + 1] - w0);
-        } else {
-            wl = a.wls[j];
-            wf = a.dflux ? a.dflux[j] * 2 * PI * a.unit : 0.0;
-            wc = two ? a.dcntm[j] * 2 * PI * a.unit : 0.0;
-            pass_c = two;
-            if (a.cn.nk > 0) kp = knot_pos(a.cn.knots, a.cn.nk, wl);
-            if (two && a.cseg && isfinite(wc) && kp.t >= 0.0 && kp.t <= 1.0 && !isnan(a.cseg[kp.i * CSEG_P])) {
-                pass_c = false;
-                if (lane < CSEG_P && wc != 0.0)
-                    atomicAdd(a.wnode + kp.i * CSEG_P + lane, wc * cseg_basis(lane, 1.0 - 2.0 * kp.t));
-            }
-        }
+    const int64_t stride = int64_t(gridDim.x) * RTA_WARPS;
+    for (int64_t j = int64_t(blockIdx.x) * RTA_WARPS + warp; j < a.nwl; j += stride) {
+        const double wl = a.wls[j];
+        const double wf = a.dflux ? a.dflux[j] * 2 * PI * a.unit : 0.0;
+        const double wc = two ? a.dcntm[j] * 2 * PI * a.unit : 0.0;
+        const KnotPos kp = a.cn.nk > 0 ? knot_pos(a.cn.knots, a.cn.nk, wl) : KnotPos{0, 0.0};
         const double pre = 2 * HPLANCK_CGS * (C_CGS * C_CGS) / (wl * wl * wl * wl * wl);
         const double hcw = HPLANCK_CGS * C_CGS / wl;
         const double ipre = recip64(pre);
@@ -379,9 +328,8 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
             c.Sbar[l] = 0.0;
         }
         __syncwarp();
-        if constexpr (!NODES)
-            rt_adj_pass(c, a.alpha + j * L, wf, s_fac, s_dlt, s_iaref, L, s_math, s_e2, c.g, s_dar, lane);
-        if (pass_c) {
+        rt_adj_pass(c, a.alpha + j * L, wf, s_fac, s_dlt, s_iaref, L, s_math, s_e2, c.g, s_dar, lane);
+        if (two) {
             // continuum-only column (src/synthesize.jl:287-291), as the forward interpolates it
             for (int l = lane; l < L; l += 32) c.col[l] = knot_eval(a.cn.vals + int64_t(l) * a.cn.nk, a.cn.nk, kp);
             __syncwarp();
@@ -391,7 +339,7 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
             // the knots feed both passes' opacity (alpha = continuum + hydrogen + lines)
             if (a.dvals) {
                 for (int l = lane; l < L; l += 32) {
-                    const double gsum = (NODES ? 0.0 : c.g[l]) + (pass_c ? c.gc[l] : 0.0);
+                    const double gsum = c.g[l] + (two ? c.gc[l] : 0.0);
                     if (gsum == 0.0) continue;
                     double* row = a.dvals + int64_t(l) * a.cn.nk;
                     if (a.cn.nk == 1) {
@@ -409,7 +357,6 @@ __global__ void __launch_bounds__(32 * RTA_WARPS) rt_adjoint_kernel(RtAdjArgs a)
             const double x = hcw * s_ikT[l];
             const double d = c.Sbar[l] * B * (x * s_iT[l]) * (1.0 + B * ipre);
             if (d != 0.0) atomicAdd(s_dT + l, d);
-            if constexpr (NODES) continue;
             if (a.g32)
                 static_cast<float*>(a.G)[j * L + l] = float(c.g[l]);
             else

@@ -867,12 +867,7 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
     // line-adjoint items ((chunk, tier) pairs) and the wavelengths as FP32 pairs
     const int np_max = int((nwl + ADJ_CHUNK - 1) / ADJ_CHUNK) * NTIER;
     const size_t o_ilo = o_g32 + a256(4 * L), o_ipre = o_ilo + a256(4 * size_t(np_max)),
-                 o_wl2 = o_ipre + a256(8 * size_t(np_max + 1)), o_wn = o_wl2 + a256(8 * size_t(nwl));
-    // knot intervals with nodes, where the columns are more than the GPU holds at a time (8 blocks per SM):
-    // fewer take one warp's latency whatever their number (1,001 columns: two more launches, 5.79 -> 5.86 ms)
-    const bool nodes = dcntm && use_cntm_segments(cn, nwl) && nwl > int64_t(ctx->sms) * 8 * RTA_WARPS;
-    const int64_t nseg = nodes ? cn.nk - 1 : 0;
-    const size_t small = o_wn + a256(8 * CSEG_P * size_t(nseg));
+                 o_wl2 = o_ipre + a256(8 * size_t(np_max + 1)), small = o_wl2 + a256(8 * size_t(nwl));
     KCHECK(ensure(ctx, ctx->vjp_small, small));
     unsigned char* sm = static_cast<unsigned char*>(ctx->vjp_small.p);
     double* daref = reinterpret_cast<double*>(sm + o_dar);
@@ -922,25 +917,12 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
 
     // 2. transfer adjoint: opacity cotangent G, dL/dT through the source function, dL/dalpha_ref
     RtAdjArgs ra{alpha, lay.T, wls, nwl, L, in->tau_ref, aref, static_cast<MathTables*>(ctx->math.p), cn, dflux,
-                 dcntm, 1e-8, ctx->vjp_g.p, int32_t(mixed), dT, daref, gr.cntm_vals, nullptr, nullptr};
+                 dcntm, 1e-8, ctx->vjp_g.p, int32_t(mixed), dT, daref, gr.cntm_vals};
     {
-        if (nseg > 0) {
-            RtArgs fa{alpha, nullptr, lay.T, wls, nwl, L, in->tau_ref, aref, ra.math, cn, nullptr, nullptr, nullptr, 1e-8};
-            KCHECK(run_cntm_segments(ctx, &fa, s));
-            ra.cseg = fa.cseg;
-            ra.wnode = reinterpret_cast<double*>(sm + o_wn);
-            KCUDA(cudaMemsetAsync(ra.wnode, 0, sizeof(double) * CSEG_P * nseg, s));
-        }
         const size_t smem = size_t(RTA_WARPS) * RTA_ARRAYS * (L + 1) * sizeof(double);
-        const auto blocks = [&](int64_t cols) {
-            return unsigned(std::min<int64_t>((cols + RTA_WARPS - 1) / RTA_WARPS, int64_t(ctx->sms) * 8));
-        };
-        KCUDA(cudaFuncSetAttribute(rt_adjoint_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        rt_adjoint_kernel<false><<<blocks(nwl), 32 * RTA_WARPS, smem, s>>>(ra);
-        if (nseg > 0) {
-            KCUDA(cudaFuncSetAttribute(rt_adjoint_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-            rt_adjoint_kernel<true><<<blocks(nseg * CSEG_P), 32 * RTA_WARPS, smem, s>>>(ra);
-        }
+        KCUDA(cudaFuncSetAttribute(rt_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        const int64_t blocks = std::min<int64_t>((nwl + RTA_WARPS - 1) / RTA_WARPS, int64_t(ctx->sms) * 8);
+        rt_adjoint_kernel<<<unsigned(blocks), 32 * RTA_WARPS, smem, s>>>(ra);
         KCUDA(cudaGetLastError());
     }
     record(ctx, 10, s);
