@@ -95,8 +95,8 @@ def test_mixed_far_lines_match_oracle(gpu_lib, oracle_lib, L):
 
 @pytest.mark.parametrize("L", [56, 80, 130])
 def test_mixed_far_lines_of_a_batch(gpu_lib, L):
-    """A batch takes far lines in tiles that a single spectrum evaluates line by line: FP32 roundings of
-    6e-8 of the far opacity, averaged over 20,000 lines, move the flux by less than 1e-7 of it."""
+    """A batch's far lines (a launch over spectra, one of them sparse) against single spectra's: FP32
+    roundings of 6e-8 of the far opacity move the flux by less than 1e-7 of it."""
     from korg_gb300.batch import BatchSynthesis
     from korg_gb300.api import synthesize_prepared
     inps = [_inputs(L, 5000, 5020, n, teff=4500.0) for n in (20000, 300)]
