@@ -11,6 +11,8 @@
 //                 each thread owns one wavelength and a set of layers and accumulates in
 //                 registers, then adds to alpha once.
 #pragma once
+#include <cstddef>
+
 #include <type_traits>
 
 #include "physics.cuh"
@@ -38,6 +40,7 @@ struct HRec {
     float4 abo32;                  // ABO constants packed for profile32x
     int32_t lb, ub, kind, nD;
 };
+static_assert(alignof(HRec) % 16 == 0 && offsetof(HRec, lb) % 16 == 0, "lb .. nD are read in one 16-byte load");
 
 struct HLayers {
     int32_t L;

@@ -16,6 +16,7 @@
 //          are copied to shared memory with cp.async, double buffered.
 #pragma once
 #include <algorithm>
+#include <cstddef>
 
 #include "physics.cuh"
 
@@ -1051,12 +1052,14 @@ template <int K>
 struct FarShared {
     double node[FAR_WARPS][FAR_P][K];       // FP64 node sums of each warp
     double v[K][FAR_P], cf[K][FAR_P + 1];
-    float tp[FAR_WARPS][2][FAR_P];          // t' of the line(s) at hand
+    alignas(16) float tp[FAR_WARPS][2][FAR_P];  // t' of the line(s) at hand, read 16 bytes at a time
     int64_t tier[NTIER][2];
     double stage[32][K + 1];                // alpha of 32 wavelengths
 };
 template <int K>
 __device__ __forceinline__ void line_far_body(const TileArgs& a, int64_t tile, int tw, int g, FarShared<K>& sh) {
+    static_assert(alignof(FarShared<K>) % 16 == 0 && offsetof(FarShared<K>, tp) % 16 == 0 && FAR_P % 4 == 0,
+                  "tp is read in 16-byte loads");
     constexpr int LPW = K <= 16 ? 2 : 1;    // lines a warp works on at a time
     constexpr int HL = 32 / LPW;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = lane / HL, k = lane % HL;

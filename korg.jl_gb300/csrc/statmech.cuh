@@ -485,7 +485,7 @@ __device__ bool ce_lu32(CeShared& s, float* M, float* uinv) {
             for (int r = 0; r < 3; ++r)
                 l[q][r] = (act[r] >> q) & 1u ? M[(k0 + q) * CE_LD + lane + 32 * r] : 0.f;
         auto update = [&](int c0, int e, float (&v)[3]) {
-            float u[CE_PB];
+            alignas(16) float u[CE_PB];
 #pragma unroll
             for (int q = 0; q < CE_PB; q += 4)
                 *reinterpret_cast<float4*>(u + q) = *reinterpret_cast<const float4*>(ub + e * CE_PB + q);
