@@ -594,14 +594,17 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
 
 // ------------------------------------------------------------------ transfer
 // continuum transfer per knot interval (8 columns each) where that at least halves the columns
-bool use_cntm_segments(const CntmDev& cn, int64_t nwl) { return cn.nk >= 2 && nwl >= 2 * CSEG_P * (cn.nk - 1); }
+bool use_cntm_segments(const CntmDev& cn, int64_t nwl, int L) {
+    return cn.nk >= 2 && nwl >= 2 * CSEG_P * (cn.nk - 1) &&
+           cntm_segment_smem(L) + E2_BYTES + sizeof(double) * CSEG_P <= RT_SMEM;
+}
 
 int run_cntm_segments(korg_ctx* ctx, RtArgs* ra, cudaStream_t s) {
-    if (!use_cntm_segments(ra->cn, ra->nwl)) return KORG_OK;
+    if (!use_cntm_segments(ra->cn, ra->nwl, ra->L)) return KORG_OK;
     KCHECK(ensure(ctx, ctx->cseg, sizeof(double) * CSEG_P * size_t(ra->cn.nk - 1)));
     double* cseg = static_cast<double*>(ctx->cseg.p);
     const unsigned blocks = unsigned(std::min<int64_t>(ra->cn.nk - 1, int64_t(ctx->sms) * 6));
-    cntm_segment_kernel<<<blocks, 32 * CSEG_P, (sizeof(double) * 3 + CSEG_P) * size_t(ra->L), s>>>(*ra, cseg);
+    cntm_segment_kernel<<<blocks, 32 * CSEG_P, cntm_segment_smem(ra->L), s>>>(*ra, cseg);
     KCUDA(cudaGetLastError());
     ra->cseg = cseg;
     return KORG_OK;
@@ -611,12 +614,12 @@ int run_rt(korg_ctx* ctx, const double* alpha, const double* S, const double* T,
            int L, const double* tau_ref, const double* alpha_ref, CntmDev cn, double* flux, double* cntm,
            double unit, cudaStream_t s) {
     RtArgs ra{alpha, S, T, wls, nwl, L, tau_ref, alpha_ref, static_cast<MathTables*>(ctx->math.p), cn, nullptr, flux,
-              cntm, unit};
+              cntm, unit, int32_t(!S && rt_planck_smem(L) <= RT_SMEM)};
     KCHECK(run_cntm_segments(ctx, &ra, s));
-    if (nwl <= RT_WARP_COLS)
-        rt_warp_kernel<<<unsigned((nwl + RT_WARPS - 1) / RT_WARPS), 32 * RT_WARPS, sizeof(double) * 3 * L, s>>>(ra);
+    if (nwl <= RT_WARP_COLS && rt_smem(L) + E2_BYTES <= RT_SMEM)
+        rt_warp_kernel<<<unsigned((nwl + RT_WARPS - 1) / RT_WARPS), 32 * RT_WARPS, rt_smem(L), s>>>(ra);
     else
-        rt_kernel<<<unsigned((nwl + RT_BLK - 1) / RT_BLK), RT_BLK, sizeof(double) * (3 + PLANCK_P) * L, s>>>(ra);
+        rt_kernel<<<unsigned((nwl + RT_BLK - 1) / RT_BLK), RT_BLK, ra.planck ? rt_planck_smem(L) : rt_smem(L), s>>>(ra);
     KCUDA(cudaGetLastError());
     return KORG_OK;
 }

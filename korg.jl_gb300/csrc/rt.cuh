@@ -29,6 +29,7 @@ struct RtArgs {
     double* flux;
     double* cntm;
     double unit;             // multiplies 2*pi*I (1e-8 in synthesize, src/synthesize.jl:315-318)
+    int32_t planck;          // rt_kernel: its shared memory holds rows for the Planck series
 };
 
 // src/synthesize.jl:412-418 with the column factors hoisted and 1/(kT) per layer precomputed,
@@ -101,6 +102,11 @@ __device__ __forceinline__ int expint2_piece(double x) {
 struct RtLayers {  // per-layer constants in shared memory
     double *fac, *hdl, *ikT;
 };
+// Shared memory that a transfer launch may ask for beside the kernel's math tables: 48 KB in all, 1,792
+// layers of constants.  What else a kernel keeps there has to fit too: above 597 layers the columns go
+// without Planck rows, above 1,329 without continuum intervals, above 1,775 by threads and not by warps.
+constexpr size_t RT_SMEM = 48 * 1024 - sizeof(MathTables);
+inline size_t rt_smem(int L) { return sizeof(double) * 3 * size_t(L); }
 __device__ __forceinline__ RtLayers rt_layers(const RtArgs& a, double* sh) {
     const int L = a.L;
     RtLayers y{sh, sh + L, sh + 2 * L};
@@ -115,6 +121,7 @@ __device__ __forceinline__ RtLayers rt_layers(const RtArgs& a, double* sh) {
 // expint2_ex with its seven middle pieces as rows of a table (centre, six coefficients; the same operations
 // in the same order): lanes of a warp at different optical depths then share one path.
 constexpr int E2_ROW = 7;
+constexpr size_t E2_BYTES = (sizeof(double) * 7 * E2_ROW + 15) / 16 * 16;  // in shared memory
 __device__ __constant__ double c_e2_mid[7 * E2_ROW] = {
     2, 0.037534261820486914, -0.04890051070806112, 0.033833820809153176, -0.016916910404576574, 0.007048712668573576,
     -0.0026785108140579598,
@@ -190,6 +197,7 @@ __device__ __forceinline__ double rt_column_warp(int L, const RtLayers& y, const
     return I;
 }
 
+inline size_t cntm_segment_smem(int L) { return rt_smem(L) + CSEG_P * size_t(L); }  // constants, pieces of E2
 // one block per interval at a time, one warp per node
 __global__ void __launch_bounds__(32 * CSEG_P) cntm_segment_kernel(RtArgs a, double* cseg) {
     extern __shared__ double s_rt[];
@@ -260,6 +268,7 @@ __device__ __forceinline__ double cntm_series(const double* cseg, const KnotPos&
 // in the exponent (half range): the next term is below PLANCK_VAR^6 / (2^5 6!) = 4e-17.
 constexpr int PLANCK_P = 6;
 constexpr double PLANCK_VAR = 0.01;
+inline size_t rt_planck_smem(int L) { return rt_smem(L) + sizeof(double) * PLANCK_P * size_t(L); }
 // cos(pi i / 12), i = 0..6
 __device__ __constant__ double c_cos12[7] = {1.0, 0.9659258262890683, 0.8660254037844387, 0.7071067811865476, 0.5000000000000001, 0.25881904510252074, 0.0};
 __device__ __forceinline__ double cos_pi12(int i) {
@@ -284,7 +293,7 @@ __global__ void __launch_bounds__(RT_BLK) rt_kernel(RtArgs a) {
     const bool two = a.cn.nk > 0;
     bool series = false;
     double T1 = 0.0;  // wavelength in [-1, 1] over the block
-    if (!a.S) {  // uniform
+    if (!a.S && a.planck) {  // uniform
         const double wa = a.wls[j0], hw = 0.5 * (a.wls[min(j0 + RT_BLK, a.nwl) - 1] - wa);
         double xmax = 0.0;
         for (int l = 0; l < L; l++) xmax = fmax(xmax, y.ikT[l]);
