@@ -182,6 +182,19 @@ int reset_counters(korg_ctx* ctx, cudaStream_t s) {
     return KORG_OK;
 }
 
+// Lets `kern` take all the dynamic shared memory that an SM gives a block, whatever this call needs: the
+// attribute belongs to the process, and set to one call's size, a smaller call of another context's thread
+// in between would have the launch refused.
+constexpr size_t SMEM_BLOCK = 227 * 1024;
+template <class... Args>
+cudaError_t allow_smem(void (*kern)(Args...)) {
+    cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(SMEM_BLOCK - fa.sharedSizeBytes));
+}
+
 void record(korg_ctx* ctx, int i, cudaStream_t s) {
     if (ctx->timing && !ctx->capturing) cudaEventRecord(ctx->ev[i], s);
 }
@@ -369,14 +382,14 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
     }
     if (q) {
         auto kern = line_tile_queue_kernel<MIXED, KMAX, MAXT, MINB>;
-        KCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
+        KCUDA(allow_smem(kern));
         int per_sm = 0;
         KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, g.threads, g.smem));
         const int64_t grid = std::min<int64_t>(q->nitems, int64_t(ctx->sms) * std::max(per_sm, 1));
         if (grid > 0) kern<<<unsigned(grid), g.threads, g.smem, s>>>(*q);
     } else {
         auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB, SUB>;
-        KCUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)));
+        KCUDA(allow_smem(kern));
         const int64_t tiles = (ta.nwl + g.tw - 1) / g.tw;
         kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) * SUB : 1u), g.threads, g.smem, s>>>(ta);
     }
@@ -923,7 +936,7 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
                  dcntm, 1e-8, ctx->vjp_g.p, int32_t(mixed), dT, daref, gr.cntm_vals};
     {
         const size_t smem = size_t(RTA_WARPS) * RTA_ARRAYS * (L + 1) * sizeof(double);
-        KCUDA(cudaFuncSetAttribute(rt_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        KCUDA(allow_smem(rt_adjoint_kernel));
         const int64_t blocks = std::min<int64_t>((nwl + RTA_WARPS - 1) / RTA_WARPS, int64_t(ctx->sms) * 8);
         rt_adjoint_kernel<<<unsigned(blocks), 32 * RTA_WARPS, smem, s>>>(ra);
         KCUDA(cudaGetLastError());
@@ -1034,17 +1047,17 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         const size_t smem = adj_smem(sh, mixed);
         int per_sm = 0;
         if (mixed) {
-            KCUDA(cudaFuncSetAttribute(line_adj_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            KCUDA(allow_smem(line_adj_kernel<true>));
             KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_adj_kernel<true>, threads, smem));
             line_adj_kernel<true><<<ctx->sms * std::max(per_sm, 1), threads, smem, s>>>(la);
         } else {
-            KCUDA(cudaFuncSetAttribute(line_adj_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+            KCUDA(allow_smem(line_adj_kernel<false>));
             KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_adj_kernel<false>, threads, smem));
             line_adj_kernel<false><<<ctx->sms * std::max(per_sm, 1), threads, smem, s>>>(la);
         }
         KCUDA(cudaGetLastError());
         const size_t psmem = sizeof(double) * size_t(4 + S) * L;
-        KCUDA(cudaFuncSetAttribute(line_adj_prologue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(psmem)));
+        KCUDA(allow_smem(line_adj_prologue_kernel));
         line_adj_prologue_kernel<<<unsigned((lns.n * 32 + 255) / 256), 256, psmem, s>>>(
             lns, lay, sc.lc, dpar, Lp, out, static_cast<MathTables*>(ctx->math.p));
         KCUDA(cudaGetLastError());
@@ -2086,7 +2099,7 @@ KORG_API int korg_radiative_transfer_general(korg_ctx* ctx, const double* alpha,
     for (int r = 0; r < n_in; r++) paired = paired && in_idx[r] == r;
     if (paired) {
         const size_t smem = rt_rays_smem(L, n_mu);
-        KCUDA(cudaFuncSetAttribute(rt_rays_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        KCUDA(allow_smem(rt_rays_kernel));
         rt_rays_kernel<<<unsigned((nwl + 31) / 32), 32 * RAY_WARPS, smem, ctx->stream>>>(ra);
     } else {
         rt_general_kernel<<<unsigned((nwl + 127) / 128), 128, 0, ctx->stream>>>(ra);
@@ -2901,7 +2914,7 @@ int noalloc_tiles(const TileArgs& ta, int G, int kmax, bool mixed, cudaStream_t 
     t.G = G;
     const dim3 grid(unsigned((ta.nwl + g.tw - 1) / g.tw), unsigned(G));
     auto go = [&](auto kern) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(g.smem)) != cudaSuccess)
+        if (allow_smem(kern) != cudaSuccess)
             return KORG_ECUDA;
         kern<<<grid, g.threads, g.smem, s>>>(t);
         return cudaGetLastError() == cudaSuccess ? KORG_OK : KORG_ECUDA;
