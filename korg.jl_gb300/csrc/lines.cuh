@@ -1023,9 +1023,10 @@ struct LineStage32 {
 };
 static_assert(sizeof(LineStage32) == 32, "LineStage32 is two 16-byte loads");
 
-// Whether the mixed tile's far lines go to line_far_kernel (see FAR_MIN_CAND32).
+// Whether the mixed tile's far lines go to line_far_kernel (see FAR_MIN_CAND32).  Not for an unsorted list:
+// its runs are whole tiers, whose length says nothing about the tile.
 __device__ __forceinline__ bool far_tile32(const TileArgs& a, const int64_t (&run)[NTIER][2], int64_t npoints) {
-    if (!a.far32 || npoints < FAR_MIN_POINTS) return false;
+    if (!a.far32 || *a.unsorted || npoints < FAR_MIN_POINTS) return false;
     int64_t n = 0;
     for (int t = 0; t < NTIER; t++) n += max(run[t][1] - run[t][0], int64_t(0));
     return n >= FAR_MIN_CAND32;
