@@ -27,6 +27,24 @@ def _lines_only(gpu_lib, inp, ll, cutoff=3e-4):
     return a, n
 
 
+def test_series_of_far_lines_in_fp64(gpu_lib):
+    """9,000 lines, all far from the only tile (three tile widths and more) and weakly damped, so that every one
+    is given by its wing cubic there: the tile's opacity is the polynomial of degree 15 through the nodes.  In
+    FP32 are its terms from the fourth on, 2 (1 + n) 14^-n of the mean, off by n^2 2^-24 of themselves at most
+    (n^2 from the rounded argument): 4e-10 in all, so 1e-9."""
+    from korg_gb300 import synthetic
+    inp = _inputs(14, 5000, 5006, 300, wl=(5000.0, 5001.27))
+    assert len(inp.wls) == 128
+    ll = synthetic.synthetic_linelist(9000, 5005.1, 5006, seed=1, molecular=True)
+    ll.gamma_rad[:] = 1e7
+    a, n = _lines_only(gpu_lib, inp, ll, cutoff=1e-20)
+    assert n == 9000
+    w = inp.wls.all_wls
+    V = np.polynomial.chebyshev.chebvander((w - w[0]) / (0.5 * (w[-1] - w[0])) - 1, 15)
+    fit = V @ np.linalg.lstsq(V, a, rcond=None)[0]
+    assert np.max(np.abs(a / fit - 1)) <= 1e-9
+
+
 def test_sparse_tiles_of_an_unsorted_list(gpu_lib):
     """Forty lines below 5100 A and 14,000 weak ones above 5150 A, which come in reverse: for an unsorted
     list the candidate runs are whole tiers, more than the limit for far lines, but the tiles below 5100 A are as
