@@ -355,7 +355,9 @@ typedef struct {
 } korg_synth_grads;
 /* KORG_VJP_REUSE_FORWARD: the previous call on this context was korg_synthesize[_dev] with the
  * same inputs; its alpha (kept in the context when alpha_out was NULL), alpha_ref, line prologue
- * and hydrogen-line records are reused instead of recomputed. */
+ * and hydrogen-line records are reused instead of recomputed.  (KORG_MIXED: the opacity of tiles
+ * whose far lines the forward summed at nodes, those with 8,192 candidate lines and more, is
+ * evaluated again line by line, so the gradients are those of a recomputing call.) */
 enum { KORG_VJP_HYDROGEN = 1, KORG_VJP_REUSE_FORWARD = 2 };
 KORG_API int korg_synthesize_vjp(korg_ctx *ctx, const korg_synth_inputs *in, const korg_lines *lines,
                                  const korg_lines *lines5, const double *wls, int64_t nwl,
@@ -466,8 +468,8 @@ KORG_API int korg_synthesize_batch_dev(korg_ctx *ctx, int32_t nspec, const korg_
  * pointers, as in korg_synthesize_vjp).  With KORG_VJP_REUSE_FORWARD the previous batch call on
  * the context was korg_synthesize_batch_dev of the same items and ran in one chunk (the default
  * budget holds 256 spectra of 56 x 400,001): every spectrum's opacity, alpha_ref and line
- * prologue are taken from it instead of recomputed, else KORG_EINVAL.  KORG_VJP_HYDROGEN as in
- * korg_synthesize_vjp.  Gradients equal korg_synthesize_vjp_dev's for each spectrum (up to the
+ * prologue are taken from it instead of recomputed (as there, but for the dense tiles of
+ * KORG_MIXED), else KORG_EINVAL.  KORG_VJP_HYDROGEN as in korg_synthesize_vjp.  Gradients equal korg_synthesize_vjp_dev's for each spectrum (up to the
  * order of the FP64 atomic additions of the line adjoint). */
 typedef struct {
     const double *dflux, *dcntm;

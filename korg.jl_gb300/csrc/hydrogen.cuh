@@ -396,6 +396,7 @@ struct HTileArgs {
     const int64_t* d_off;
     const double* logdnu;
     const float* logdnu32;
+    TileMarks marks;       // wavelengths to evaluate
 };
 
 // A block takes TW wavelengths; its thread groups and the grid's second dimension share the layers
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile
     const int jl = tid % TW, g = tid / TW + (blockDim.x / TW) * blockIdx.y;
     const int64_t j0 = int64_t(blockIdx.x) * TW, jg = j0 + jl;
     const int64_t jlast = min(j0 + TW, a.nwl) - 1;
-    const bool live = jg < a.nwl;
+    const bool live = jg < a.nwl && !a.marks.skip(jg);  // (uniform across a warp)
     const double wl = live ? a.wls[jg] : 1.0;
     const double nu = C_CGS / wl;                // :78
     const double dnudl = C_CGS / (wl * wl);      // :79

@@ -38,6 +38,8 @@ struct DevBuf {
 
 constexpr int NEV = 13;  // 0-7: forward stages and probes; 8-12: reverse-mode stages
 
+constexpr int TILE_TW = 128;  // default wavelengths per CTA of the line tile kernel
+
 // Tile shape of the line tile kernel: wavelengths per CTA and lines per shared-memory batch
 // (0: the default for the precision).
 struct TileCfg {
@@ -79,6 +81,7 @@ struct korg_ctx {
     bool b_last_resident = false;
     std::vector<size_t> b_last_line_off;
     size_t b_last_o_aref = 0, b_last_o_refwl = 0;
+    int b_last_tw = TILE_TW;
     // CUDA graph of the last batch: replayed while the same batch is submitted again
     bool use_graph = false, capturing = false;
     cudaGraphExec_t gexec = nullptr;
@@ -103,6 +106,7 @@ struct korg_ctx {
     std::vector<void*> stark_allocs;
     // the hydrogen prep records and tables now in hrec / hQ: -1 none, 0 FP64, 1 mixed (FP64 and FP32)
     int hyd_prep = -1;
+    int last_tw = TILE_TW;  // tile width of the last line opacity
     // statistics
     bool timing = false;
     cudaEvent_t ev[NEV] = {};
@@ -230,8 +234,6 @@ LayersDev layers_dev(const korg_layers* y) {
 }
 
 // ------------------------------------------------------------------ line opacity
-constexpr int TILE_TW = 128;  // default wavelengths per CTA of the line tile kernel
-
 // Pieces of the per-spectrum scratch of the line prologue and candidate lists.
 struct LineScratch {
     LayerConst* lc = nullptr;
@@ -297,7 +299,7 @@ TileArgs make_tile_args(const korg_ctx* ctx, const LineScratch& sc, double* alph
     ta.tier_ci = sc.tier_ci;
     ta.tier_start = sc.tier_meta;                 // [start: NTIER+1][unsorted][block counts]
     ta.unsorted = sc.tier_meta + NTIER + 1;
-    ta.far32 = 1;
+    ta.far32 = FAR_NODES;
     return ta;
 }
 
@@ -428,7 +430,7 @@ int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g
 // nlines: lines of the (largest) list.
 int run_tiles(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g, const TileQueue* q, bool mixed,
               int64_t nlines, cudaStream_t s) {
-    const bool far_lines = nlines >= FAR_MIN_CAND32 && (q || ta.far32);
+    const bool far_lines = nlines >= FAR_MIN_CAND32 && (q || ta.far32 == FAR_NODES);
     return mixed ? dispatch_tile<true>(ctx, ta, kmax, g, q, far_lines, s)
                  : dispatch_tile<false>(ctx, ta, kmax, g, q, far_lines, s);
 }
@@ -481,7 +483,7 @@ bool worth_tuning(int64_t nwl, int64_t nlines) { return nwl >= 100000 && nlines 
 
 int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, const LinesDev& ln,
                         const LayersDev& lay, const CntmDev& cn, double cutoff, bool mixed,
-                        cudaStream_t s, bool far32 = true) {
+                        cudaStream_t s, int far32 = FAR_NODES) {
     if (ln.n == 0) return KORG_OK;  // src/line_absorption.jl:35-37
     const int L = lay.L;
     int kmax = 0;
@@ -499,6 +501,7 @@ int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t
     if (ctx->autotune && !ctx->capturing && worth_tuning(nwl, ln.n)) KCHECK(autotune_tiles(ctx, ta, kmax, mixed, s));
     TileGeom g;
     if (!tile_geom(mixed, Lp, G, tile_cfg(ctx, L, mixed), &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
+    ctx->last_tw = g.tw;
     ctx->stats_pending = true;
     return run_tiles(ctx, ta, kmax, g, nullptr, mixed, ln.n, s);
 }
@@ -560,8 +563,9 @@ int run_hydrogen_prep(korg_ctx* ctx, const double* wls, int64_t nwl, const HLaye
     return KORG_OK;
 }
 
+// prep: records and tables that are there already, else they are made.
 int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, const HLayers& hl, double window,
-                 int use_MHD, bool mixed, cudaStream_t s) {
+                 int use_MHD, bool mixed, cudaStream_t s, const HOut* prep = nullptr, TileMarks marks = {}) {
     const int L = hl.L;
     if (L > 256) return set_err(ctx, KORG_EINVAL, "at most 256 layers are supported (got %d)", L);
     // layer slices (slice g owns layers g, g + slices, ...): thread groups of a block x blocks in y
@@ -569,7 +573,8 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
     const int TW = shrt ? 32 : (L <= 64 ? 128 : 64), groups = shrt || L <= 64 ? 4 : 8, gy = shrt ? 2 : 1;
     const int kmax = (L + groups * gy - 1) / (groups * gy);  // layers per thread
     HOut ho;
-    KCHECK(run_hydrogen_prep(ctx, wls, nwl, hl, window, use_MHD, mixed, s, &ho));
+    if (prep) ho = *prep;
+    else KCHECK(run_hydrogen_prep(ctx, wls, nwl, hl, window, use_MHD, mixed, s, &ho));
     const int ntrans = ctx->stark.ntrans;
     const int ntot = ntrans + std::max(0, ctx->n_max - 4);
     HTileArgs ha{};
@@ -588,6 +593,7 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
     ha.d_off = ctx->stark.d_off;
     ha.logdnu = ctx->stark.logdnu;
     ha.logdnu32 = ctx->stark.logdnu32;
+    ha.marks = marks;
     const dim3 grid(unsigned((nwl + TW - 1) / TW), unsigned(gy));
     const int threads = TW * groups;
     auto go = [&](auto kern) { kern<<<grid, threads, 0, s>>>(ha); };
@@ -883,7 +889,8 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
     // line-adjoint items ((chunk, tier) pairs) and the wavelengths as FP32 pairs
     const int np_max = int((nwl + ADJ_CHUNK - 1) / ADJ_CHUNK) * NTIER;
     const size_t o_ilo = o_g32 + a256(4 * L), o_ipre = o_ilo + a256(4 * size_t(np_max)),
-                 o_wl2 = o_ipre + a256(8 * size_t(np_max + 1)), small = o_wl2 + a256(8 * size_t(nwl));
+                 o_wl2 = o_ipre + a256(8 * size_t(np_max + 1)), o_marks = o_wl2 + a256(8 * size_t(nwl)),
+                 small = o_marks + a256(size_t(nwl) / 32 + 1);
     KCHECK(ensure(ctx, ctx->vjp_small, small));
     unsigned char* sm = static_cast<unsigned char*>(ctx->vjp_small.p);
     double* daref = reinterpret_cast<double*>(sm + o_dar);
@@ -909,7 +916,9 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
 
     // 1. opacity, recomputed (src/synthesize.jl:249-306 as in the forward), unless the caller
     //    states that the previous call on this context was korg_synthesize[_dev] of the same
-    //    inputs, whose alpha, alpha_ref and metal-line prologue are still in the scratch
+    //    inputs, whose alpha, alpha_ref and metal-line prologue are still in the scratch.  Every line
+    //    at every wavelength: the mixed line adjoint rounds the opacity cotangent to FP32, and single
+    //    lines' log gf gradients would move by 4e-8 with the far lines' rounding.
     record(ctx, 8, s);
     double* alpha = op ? op->alpha : static_cast<double*>(ctx->alpha.p);
     double* aref = op ? op->aref : static_cast<double*>(ctx->aref.p);
@@ -922,13 +931,40 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         KCHECK(run_ref_lines(ctx, aref, ref_wl_dev, ln5, lay, cref, in->cutoff_threshold, s));
         if (in->hydrogen_lines)
             KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s));
-        // every line at every wavelength: the mixed line adjoint rounds the opacity cotangent to FP32,
-        // and single lines' log gf gradients would move by 3e-8 with the far lines' rounding
-        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s, false));
+        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s, FAR_DIRECT));
     }
     // the metal-line prologue: the batch's for this spectrum, else the context's line scratch (read
     // after step 1, which may have grown it)
     unsigned char* line_base = op ? op->lines : static_cast<unsigned char*>(ctx->lines_scratch.p);
+    // the forward's hydrogen records and tables, when the caller reuses its opacity (unless a batch
+    // forward, which overwrote them spectrum by spectrum, ran)
+    HOut ho{static_cast<HRec*>(ctx->hrec.p), static_cast<double*>(ctx->hQ.p), static_cast<float*>(ctx->hQ32.p),
+            static_cast<int32_t*>(ctx->hulb.p), static_cast<int32_t*>(ctx->huub.p)};
+    bool have_prep = (flags & KORG_VJP_REUSE_FORWARD) && !op && ctx->hyd_prep >= int(mixed);
+    if (((flags & KORG_VJP_REUSE_FORWARD) || op) && mixed && ln.n >= FAR_MIN_CAND32) {
+        // the forward's dense tiles hold far lines from their nodes: these tiles again, from the start
+        unsigned char* on = sm + o_marks;
+        LineScratch sc;
+        line_scratch(line_base, ln.n, L, Lp, G, mixed, &sc);
+        TileArgs ta = make_tile_args(ctx, sc, alpha, wls, nwl, ln, L, Lp, G);
+        ta.far32 = FAR_REDO;
+        TileCfg cfg = tile_cfg(ctx, L, mixed);
+        cfg.tw = op ? ctx->b_last_tw : ctx->last_tw;
+        TileGeom g;
+        if (!tile_geom(mixed, Lp, G, cfg, &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
+        const TileMarks marks{on, g.tw};
+        const int64_t tiles = (nwl + g.tw - 1) / g.tw;
+        dense_tiles_kernel<<<unsigned((tiles + 127) / 128), 128, 0, s>>>(ta, g.tw, on);
+        KCUDA(cudaGetLastError());
+        alpha_init_kernel<<<unsigned((nwl + 63) / 64), 256, 0, s>>>(alpha, wls, nwl, L, cn, marks);
+        KCUDA(cudaGetLastError());
+        if (in->hydrogen_lines) {
+            if (!have_prep) KCHECK(run_hydrogen_prep(ctx, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s, &ho));
+            have_prep = true;
+            KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s, &ho, marks));
+        }
+        KCHECK(run_tiles(ctx, ta, kmax, g, nullptr, mixed, ln.n, s));
+    }
     record(ctx, 9, s);
 
     // 2. transfer adjoint: opacity cotangent G, dL/dT through the source function, dL/dalpha_ref
@@ -953,11 +989,6 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         if (ntot > HADJ_MAXT)
             return set_err(ctx, KORG_EINVAL, "the hydrogen reverse mode supports %d transitions (got %d)", HADJ_MAXT,
                            ntot);
-        // the forward's records and tables when the caller reuses its opacity (unless a batch
-        // forward, which overwrote them spectrum by spectrum, ran), else the prep again
-        HOut ho{static_cast<HRec*>(ctx->hrec.p), static_cast<double*>(ctx->hQ.p), static_cast<float*>(ctx->hQ32.p),
-                static_cast<int32_t*>(ctx->hulb.p), static_cast<int32_t*>(ctx->huub.p)};
-        const bool have_prep = (flags & KORG_VJP_REUSE_FORWARD) && !op && ctx->hyd_prep >= int(mixed);
         if (!have_prep) KCHECK(run_hydrogen_prep(ctx, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s, &ho));
         const size_t n_dq = size_t(ntrans) * L * 2 * HND_MAX + size_t(nbr) * L * 3 * BR_NP;
         // mixed: the Stehle table derivatives, then the Brackett profiles with theirs, in FP32
@@ -2740,6 +2771,7 @@ KORG_API int korg_synthesize_batch_dev(korg_ctx* ctx, int32_t nspec, const korg_
     ctx->b_last_line_off = p.line_off;
     ctx->b_last_o_aref = p.o_aref;
     ctx->b_last_o_refwl = p.o_refwl;
+    ctx->b_last_tw = p.geom.tw;
     return KORG_OK;
 }
 
@@ -3018,7 +3050,7 @@ extern "C" KORG_API int korg_line_absorption_noalloc(double* alpha, const double
     ta.tier_ci = tl.ci;
     ta.tier_start = tl.start;
     ta.unsorted = tl.unsorted;
-    ta.far32 = 1;
+    ta.far32 = FAR_NODES;
     ta.math = math;
     return noalloc_tiles(ta, G, kmax, mixed, s);
 }

@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(32 * RT_WARPS) rt_warp_kernel(RtArgs a) {
 
 // alpha[j][l] = continuum interpolant of layer l at wl_j (src/synthesize.jl:226-252)
 __global__ void __launch_bounds__(256) alpha_init_kernel(double* alpha, const double* wls, int64_t nwl, int32_t L,
-                                                         CntmDev cn) {
+                                                         CntmDev cn, TileMarks marks = {}) {
     __shared__ int64_t s_i[64];
     __shared__ double s_t[64], s_u[64];
     const int64_t j0 = int64_t(blockIdx.x) * 64;
@@ -424,6 +424,7 @@ __global__ void __launch_bounds__(256) alpha_init_kernel(double* alpha, const do
     const int64_t n = jn * L;
     for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
         const int jj = int(e / L), l = int(e % L);
+        if (marks.skip(j0 + jj)) continue;
         const double* v = cn.vals + int64_t(l) * cn.nk + s_i[jj];
         alpha[j0 * L + e] = cn.nk == 1 ? v[0] : fma(v[1], s_t[jj], v[0] * s_u[jj]);  // knot_eval, two operations
     }

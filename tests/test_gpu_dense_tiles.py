@@ -61,3 +61,61 @@ def test_sparse_tiles_of_an_unsorted_list(gpu_lib):
     assert n >= 8192 + 40 and np.all(a[:10001].max(axis=0) > 0)
     assert np.array_equal(a[:10001], b[:10001])
     np.testing.assert_allclose(b, a, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("n,hi", [(20000, 5020.0), (9000, 5120.0)])
+@pytest.mark.parametrize("L", [56, 72])
+def test_batch_gradient_of_dense_tiles(gpu_lib, L, n, hi):
+    """Above the limit (20,000 lines on 20 A) and a long list whose tiles are below it: a batch's gradient that
+    reuses its forward equals the recomputed one and the single spectrum's, as for short lists (1e-9), and the
+    mixed gradient lies as near to FP64's as the mixed reverse mode's own comparison asks (2e-3)."""
+    from korg_gb300.api import GRAD_FIELDS, synthesize_vjp
+    from korg_gb300.batch import BatchSynthesis
+    inps = [_inputs(L, 5000, hi, k) for k in (n, 300)]
+    b = BatchSynthesis(inps, precision="mixed", use_graph=False)
+    rng = np.random.default_rng(3)
+    dF, dC = (b.torch.as_tensor(rng.normal(size=(len(inps), b.nwl)), device=b.dev) for _ in range(2))
+    b.run()
+    got = {"reuse": b.vjp(dF, dC, reuse_forward=True)}
+    b.torch.cuda.synchronize()
+    got = {k: [{f: v.cpu().numpy() for f, v in g.items()} for g in gs] for k, gs in got.items()}
+    got["again"] = [{f: v.cpu().numpy() for f, v in g.items()} for g in b.vjp(dF, dC, reuse_forward=True)]
+    got["recompute"] = [{f: v.cpu().numpy() for f, v in g.items()} for g in b.vjp(dF, dC, reuse_forward=False)]
+    for k, inp in enumerate(inps):
+        args = (inp, dF[k].cpu().numpy(), dC[k].cpu().numpy())
+        ref, ref64 = (synthesize_vjp(*args, precision=p, ctx=b.ctx) for p in ("mixed", "fp64"))
+        for f in GRAD_FIELDS:
+            scale = max(float(np.max(np.abs(ref[f]))), 1e-300)
+            for name, g in got.items():
+                assert np.max(np.abs(g[k][f].reshape(ref[f].shape) - ref[f])) <= 1e-9 * scale, (k, f, name)
+            assert np.max(np.abs(ref[f] - ref64[f])) <= 2e-3 * np.max(np.abs(ref64[f])), (k, f)
+
+
+@pytest.mark.parametrize("hydrogen", [True, False])
+@pytest.mark.parametrize("tw", [None, 64, 256])
+def test_gradient_reusing_a_dense_forward(gpu_lib, hydrogen, tw):
+    """The single spectrum's reuse against its recomputation, element by element as for short lists, at the
+    default and other tile widths, and when the width changes between the forward and its reuse."""
+    from korg_gb300.api import rectified_loss, synthesize_prepared, synthesize_vjp
+    ctx = gpu_lib.Context(0)
+    inp = _inputs(56, 5000, 5020, 20000)
+    inp.hydrogen_lines = hydrogen
+    shape = lambda w: ctx.check(ctx.lib.korg_set_tile_config(ctx.h, 56, gpu_lib.KORG_MIXED, w, 0, 1))
+    if tw:
+        shape(tw)
+    r = synthesize_prepared(inp, precision="mixed", ctx=ctx)
+    obs = r.flux / r.cntm * (1 + 0.01 * np.random.default_rng(5).standard_normal(len(r.flux)))
+    _, dF, dC = rectified_loss(r.flux, r.cntm, obs)
+    kw = dict(precision="mixed", ctx=ctx)
+    want = synthesize_vjp(inp, dF, dC, **kw)
+    synthesize_prepared(inp, precision="mixed", ctx=ctx)
+    got = synthesize_vjp(inp, dF, dC, reuse_forward=True, **kw)
+    for k in want:
+        np.testing.assert_allclose(got[k], want[k], rtol=1e-9, atol=1e-14 * np.max(np.abs(want[k])) + 1e-300)
+    if tw:  # another width moves the roundings of single terms, but leaves no far lines behind
+        synthesize_prepared(inp, precision="mixed", ctx=ctx)
+        shape(128)
+        got = synthesize_vjp(inp, dF, dC, reuse_forward=True, **kw)
+        for k in want:
+            np.testing.assert_allclose(got[k], want[k], rtol=1e-9, atol=1e-14 * np.max(np.abs(want[k])) + 1e-300)
+    ctx.close()
