@@ -12,7 +12,6 @@
 //                 registers, then adds to alpha once.
 #pragma once
 #include <cstddef>
-
 #include <type_traits>
 
 #include "physics.cuh"
@@ -216,7 +215,7 @@ __device__ __forceinline__ double brackett_oscillator_strength(int n, int m) {
     return FK * (1 - WT * GINF - (0.222 + GCA / m) * (1 - WT));
 }
 
-// src/line_absorption.jl:169-182 with the table-driven exp and log (expint1_64)
+// Kurucz's E1 (src/line_absorption.jl:169-182) with the table-driven exp and log
 __device__ __forceinline__ double expint1_t(double x, const MathTables& mt) {
     if (x < 0) return 0.0;
     if (x <= 0.01) return -flog64(x, mt) - 0.577215 + x;

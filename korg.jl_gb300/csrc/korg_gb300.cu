@@ -374,27 +374,30 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
     ta.stage = g.stage;
     ta.region = g.region;
     ta.split = g.split;
-    if (MIXED && far_lines) {
-        if (q)
+    if constexpr (MIXED) {
+        if (far_lines && q)
             line_far_batch_kernel<KMAX><<<dim3(unsigned(q->nitems / q->groups), unsigned(q->groups)), FAR_THREADS, 0, s>>>(
                 q->spec, q->nspec, g.tw);
-        else
+        else if (far_lines)
             line_far_kernel<KMAX><<<dim3(unsigned((ta.nwl + g.tw - 1) / g.tw), unsigned(g.G)), FAR_THREADS, 0, s>>>(ta, g.tw);
         KCUDA(cudaGetLastError());
     }
-    if (q) {
-        auto kern = line_tile_queue_kernel<MIXED, KMAX, MAXT, MINB>;
-        KCUDA(allow_smem(kern));
-        int per_sm = 0;
-        KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, g.threads, g.smem));
-        const int64_t grid = std::min<int64_t>(q->nitems, int64_t(ctx->sms) * std::max(per_sm, 1));
-        if (grid > 0) kern<<<unsigned(grid), g.threads, g.smem, s>>>(*q);
-    } else {
-        auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB, SUB>;
-        KCUDA(allow_smem(kern));
-        const int64_t tiles = (ta.nwl + g.tw - 1) / g.tw;
-        kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) * SUB : 1u), g.threads, g.smem, s>>>(ta);
+    if constexpr (SUB == 1) {  // (parts of groups are for short grids only, which no queue holds)
+        if (q) {
+            auto kern = line_tile_queue_kernel<MIXED, KMAX, MAXT, MINB>;
+            KCUDA(allow_smem(kern));
+            int per_sm = 0;
+            KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, g.threads, g.smem));
+            const int64_t grid = std::min<int64_t>(q->nitems, int64_t(ctx->sms) * std::max(per_sm, 1));
+            if (grid > 0) kern<<<unsigned(grid), g.threads, g.smem, s>>>(*q);
+            KCUDA(cudaGetLastError());
+            return KORG_OK;
+        }
     }
+    auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB, SUB>;
+    KCUDA(allow_smem(kern));
+    const int64_t tiles = (ta.nwl + g.tw - 1) / g.tw;
+    kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) * SUB : 1u), g.threads, g.smem, s>>>(ta);
     KCUDA(cudaGetLastError());
     return KORG_OK;
 }

@@ -402,15 +402,4 @@ __device__ __forceinline__ double scaled_vdW_abo(double sigma, double alpha, dou
     return 2 * pow(4 / PI, alpha / 2) * tgamma((4 - alpha) / 2) * v0 * sigma * pow(vbar / v0, 1 - alpha);
 }
 
-// src/line_absorption.jl:169-182
-__device__ __forceinline__ double expint1_64(double x) {
-    if (x < 0) return 0.0;
-    if (x <= 0.01) return -log(x) - 0.577215 + x;
-    if (x <= 1.0)
-        return -log(x) - 0.57721566 +
-               x * (0.99999193 + x * (-0.24991055 + x * (0.05519968 + x * (-0.00976004 + x * 0.00107857))));
-    if (x <= 30.0) return (x * (x + 2.334733) + 0.25062) / (x * (x + 3.330657) + 1.681534) / x * exp(-x);
-    return 0.0;
-}
-
 }  // namespace korg

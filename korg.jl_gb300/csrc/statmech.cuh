@@ -528,6 +528,7 @@ __device__ bool ce_lu32(CeShared& s, float* M, float* uinv) {
 // permutation P (logical -> physical row) and uinv from the factorisation.  Other warps return
 // at once.  Steps in groups of 32 unknowns, so that a step's operand needs no selection and the
 // columns of the steps ahead are loaded early.
+static_assert(CE_N > 64 && CE_N < 96, "three unknowns a lane, the third not on every lane");
 __device__ __forceinline__ float ce_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double ce_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
 template <typename T>
@@ -687,6 +688,7 @@ __device__ bool ce_solve(CeShared& s, bool& refined) {
             long long rl = 0, xl = 0;
             if (tid < CE_N) {
                 // three chains (a dependent FP64 FMA takes ~70 cycles)
+                static_assert(CE_N % 3 == 0, "chains of equal length");
                 double r = s.A[CE_N * CE_LD + tid], ra = 0.0, rb = 0.0;
 #pragma unroll 1
                 for (int c = 0; c < CE_N; c += 3) {
