@@ -2378,6 +2378,19 @@ int rot_args(korg_ctx* ctx, const double* wls, int64_t nwl, const korg_wl_range*
     a->c3 = PI * (1 - eps / 3);
     return KORG_OK;
 }
+// half the longest window in points, and the largest step over the wavelength, of the ranges
+struct RotShape {
+    double points = 0.0, step = 0.0;
+};
+RotShape rot_shape(const RotArgs& a, const korg_wl_range* ranges) {
+    RotShape q;
+    for (int k = 0; k < a.nranges; k++) {
+        const korg_wl_range& r = ranges[k];
+        q.points = std::max(q.points, a.v_over_c * (r.start / r.step + double(r.n - 1)));
+        q.step = std::max(q.step, r.step / r.start);
+    }
+    return q;
+}
 // blocks of ROT_TP points that do not straddle ranges
 unsigned rot_blocks(const RotArgs& a) {
     int64_t n = 0;
@@ -2460,7 +2473,9 @@ KORG_API int korg_apply_rotation_dev(korg_ctx* ctx, const double* wls, int64_t n
     const auto go = [&](auto kern, int ns) {
         kern<<<dim3(rot_blocks(a), unsigned((nspec + ns - 1) / ns)), ROT_TP, 0, s>>>(a, flux, nspec, out);
     };
-    if (nspec > 4) go(rotation_fwd_kernel<16>, 16);
+    if (!(rot_shape(a, ranges).points >= ROT_FWD_MIN))
+        rotation_direct_kernel<<<unsigned((nwl + ROT_TP - 1) / ROT_TP), ROT_TP, 0, s>>>(a, flux, nspec, out);
+    else if (nspec > 4) go(rotation_fwd_kernel<16>, 16);
     else if (nspec > 1) go(rotation_fwd_kernel<4>, 4);
     else go(rotation_fwd_kernel<1>, 1);
     KCUDA(cudaGetLastError());
@@ -2483,7 +2498,11 @@ KORG_API int korg_apply_rotation_vjp_dev(korg_ctx* ctx, const double* wls, int64
         const auto go = [&](auto kern, int ns) {
             kern<<<dim3(rot_blocks(a), unsigned((nspec + ns - 1) / ns)), ROT_TP, 0, s>>>(a, dout, nspec, dflux);
         };
-        if (nspec > 4) go(rotation_vjp_kernel<16>, 16);
+        const RotShape q = rot_shape(a, ranges);
+        if (!(q.points >= ROT_VJP_MIN && q.step <= ROT_VJP_STEP))
+            rotation_scatter_kernel<<<dim3(unsigned((nwl + 127) / 128), unsigned((nspec + ROT_SPEC - 1) / ROT_SPEC)), 128,
+                                      0, s>>>(a, dout, nspec, dflux);
+        else if (nspec > 4) go(rotation_vjp_kernel<16>, 16);
         else if (nspec > 1) go(rotation_vjp_kernel<4>, 4);
         else go(rotation_vjp_kernel<1>, 1);
     }

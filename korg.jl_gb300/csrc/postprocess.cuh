@@ -9,7 +9,8 @@
 //                      for a block of up to LSF_SPEC spectra.
 //   rotation kernels:  one thread per output wavelength (forward) or point (reverse, a gather): a
 //                      walk over the window's offsets, whose kernel integrals are quartics in the
-//                      wavelength over a block, applied to up to 16 spectra at once.
+//                      wavelength over a block, applied to up to 16 spectra at once; short windows, and
+//                      the reverse mode on coarse grids, by their integrals one by one.
 //
 // Everything is FP64, as in the reference (post-processing of the FP64 flux).
 #pragma once
@@ -227,6 +228,94 @@ __device__ __forceinline__ double rot_eval(const RotArgs& a, const RotTable& t, 
     return rot_kernel_integral(a, a.c3 * dl, (double(o) + 0.5) * step, dl);
 }
 
+// Windows that the quartics do not pay for walk their integrals one after the other, a thread per output,
+// two binary searches and one integral per point; the reverse mode scatters with FP64 atomics.  The lines,
+// by m = half the window in points and the step over the wavelength (measured: 1, 4 and 16 spectra of 301
+// to 100,001 points):
+//   forward   m < ROT_FWD_MIN: 2,001 points, m = 1.7: 20 us (quartics 34), m = 3.3: 34 (34), m = 5: 47 (36)
+//   reverse   m < ROT_VJP_MIN: m = 5: 49 us (59), m = 10: 87 (63); or a step above ROT_VJP_STEP of the
+//             wavelength, where the gather's tables, which span three blocks of outputs, have no series for
+//             most offsets and each integral is taken twice: 20,001 points, m = 33: 4e-6 410 us (220),
+//             m = 50: 1e-5 628 (650), m = 25: 2e-5 353 (518).
+constexpr double ROT_FWD_MIN = 3.0, ROT_VJP_MIN = 10.0, ROT_VJP_STEP = 5e-6;
+constexpr int ROT_SPEC = 8;   // spectra per thread of the scatter
+__device__ __forceinline__ const RotRange& rot_range(const RotArgs& a, int64_t i) {  // the range of grid index i
+    int k = 0;
+    while (k + 1 < a.nranges && i >= a.r[k + 1].first) k++;
+    return a.r[k];
+}
+struct RotWindow {
+    const double* w;  // the range's wavelengths
+    int64_t first, ii, lb, ub;  // the range, the output and its window within it
+    double step, dl, c3dl;
+    // integral above point m of the window
+    __device__ __forceinline__ double above(const RotArgs& a, int64_t m) const {
+        return rot_kernel_integral(a, c3dl, m < ub ? (double(m - ii) + 0.5) * step : dl, dl);
+    }
+};
+__device__ __forceinline__ RotWindow rot_window(const RotArgs& a, int64_t i) {
+    const RotRange& rg = rot_range(a, i);
+    RotWindow q;
+    q.w = a.wls + rg.first;
+    q.first = rg.first;
+    q.ii = i - rg.first;
+    q.step = rg.step;
+    const double wl = a.wls[i];
+    q.dl = wl * a.v_over_c;
+    q.c3dl = a.c3 * q.dl;
+    q.lb = search_first(q.w, rg.n, wl - q.dl);
+    q.ub = search_last(q.w, rg.n, wl + q.dl);
+    return q;
+}
+__global__ void __launch_bounds__(128) rotation_scatter_kernel(RotArgs a, const double* dout, int32_t nspec,
+                                                               double* dflux) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= a.nwl) return;
+    const int s0 = blockIdx.y * ROT_SPEC, ns = min(ROT_SPEC, nspec - s0);
+    const RotWindow q = rot_window(a, i);
+    double g[ROT_SPEC];
+#pragma unroll
+    for (int k = 0; k < ROT_SPEC; k++) g[k] = k < ns ? dout[int64_t(s0 + k) * a.nwl + i] : 0.0;
+    double Kp = rot_kernel_integral(a, q.c3dl, -q.dl, q.dl);
+    for (int64_t m = q.lb; m <= q.ub; m++) {
+        const double Kn = q.above(a, m);
+#pragma unroll
+        for (int k = 0; k < ROT_SPEC; k++)
+            if (k < ns) atomicAdd(dflux + int64_t(s0 + k) * a.nwl + q.first + m, g[k] * (Kn - Kp));
+        Kp = Kn;
+    }
+}
+// Forward: a chunk's weights K_{k+1} - K_k in this thread's own column of shared memory, then every spectrum.
+constexpr int ROT_DCH = 8;  // window points per chunk (m < ROT_FWD_MIN: at most 7)
+__global__ void __launch_bounds__(ROT_TP) rotation_direct_kernel(RotArgs a, const double* in, int32_t nspec, double* out) {
+    __shared__ double s_w[ROT_DCH][ROT_TP];
+    const int t = threadIdx.x;
+    const int64_t i = int64_t(blockIdx.x) * ROT_TP + t;
+    if (i >= a.nwl) return;  // no block-wide synchronisation below
+    const RotWindow q = rot_window(a, i);
+    const int64_t nwin = q.ub - q.lb + 1;
+    double Kp = rot_kernel_integral(a, q.c3dl, -q.dl, q.dl);
+    for (int64_t c0 = 0; c0 < nwin; c0 += ROT_DCH) {
+        const int n = int(min(int64_t(ROT_DCH), nwin - c0));
+        for (int e = 0; e < n; e++) {
+            const double Kn = q.above(a, q.lb + c0 + e);
+            s_w[e][t] = Kn - Kp;
+            Kp = Kn;
+        }
+        const double* f0 = in + q.first + q.lb + c0;
+        for (int s = 0; s < nspec; s++) {
+            const double* f = f0 + int64_t(s) * a.nwl;
+            double acc = 0.0;
+            for (int e = 0; e < n; e++) acc += s_w[e][t] * f[e];
+            double* o = out + int64_t(s) * a.nwl + i;
+            *o = c0 == 0 ? acc : *o + acc;
+        }
+    }
+    if (nwin <= 0) {  // empty window (cannot happen for a grid point, which is inside its own window)
+        for (int s = 0; s < nspec; s++) out[int64_t(s) * a.nwl + i] = 0.0;
+    }
+}
+
 // first block of each range in a grid of ROT_TP-point blocks that do not straddle ranges
 __device__ __forceinline__ const RotRange& rot_block(const RotArgs& a, int64_t* i0) {
     int64_t blk = blockIdx.x;
@@ -240,7 +329,7 @@ __device__ __forceinline__ const RotRange& rot_block(const RotArgs& a, int64_t* 
     return a.r[k];
 }
 
-// Forward: one thread per output and up to NS spectra (accumulators in registers), offsets +o and -o
+// Forward of long windows: one thread per output and up to NS spectra (accumulators in registers), offsets +o and -o
 // together.  FP64 pipe bound: 2 NS FMAs and ~8 operations of weights per offset pair.  16 spectra of
 // 100,001 points, vsini 10 km/s (214 window points): 3886 -> 944 us (two asin / sqrt a point and output
 // before).
@@ -300,7 +389,7 @@ __global__ void __launch_bounds__(ROT_TP) rotation_fwd_kernel(RotArgs a, const d
     }
 }
 
-// Reverse mode as a gather: dF_j += sum over the outputs i whose window holds j of dout_i w(i, j), one thread
+// Reverse mode of long windows as a gather: dF_j += sum over the outputs i whose window holds j of dout_i w(i, j), one thread
 // per point j and up to NS spectra, outputs j - o and j + o together (o uniform over the block, so the
 // offsets without a series do not diverge).  The windows of the outputs at hand and their normalised
 // wavelengths go to shared memory; outputs to the left and to the right have a table each where the window
