@@ -638,7 +638,7 @@ int run_rt(korg_ctx* ctx, const double* alpha, const double* S, const double* T,
     RtArgs ra{alpha, S, T, wls, nwl, L, tau_ref, alpha_ref, static_cast<MathTables*>(ctx->math.p), cn, nullptr, flux,
               cntm, unit, int32_t(!S && rt_planck_smem(L) <= RT_SMEM)};
     KCHECK(run_cntm_segments(ctx, &ra, s));
-    if (nwl <= RT_WARP_COLS && rt_smem(L) + E2_BYTES <= RT_SMEM)
+    if (rt_by_warp(nwl, L, S != nullptr) && rt_smem(L) + E2_BYTES <= RT_SMEM)
         rt_warp_kernel<<<unsigned((nwl + RT_WARPS - 1) / RT_WARPS), 32 * RT_WARPS, rt_smem(L), s>>>(ra);
     else
         rt_kernel<<<unsigned((nwl + RT_BLK - 1) / RT_BLK), RT_BLK, ra.planck ? rt_planck_smem(L) : rt_smem(L), s>>>(ra);

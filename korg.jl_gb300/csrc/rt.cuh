@@ -371,9 +371,14 @@ __global__ void __launch_bounds__(RT_BLK) rt_kernel(RtArgs a) {
     if (each) a.cntm[j] = 2 * PI * (cont.I * 1.0) * a.unit;
 }
 
-// One warp per column: grids of at most RT_WARP_COLS columns, where one thread per column is bound by its
-// serial chain (180 us for 56 layers at any size; 2,001 columns 46 us here).
-constexpr int64_t RT_WARP_COLS = 16384;
+// One warp per column, for short grids.  A thread per column takes its serial chain at any size up to 19,456
+// columns (a block per SM): 3.05 us a layer (S given), 3.3 to 5 with the Planck function and the continuum.  Warps
+// take 3.0 + 4.1 c ns a column, c = ceil(L / 32) (7.0 + 5.8 c), and 20 us.  They meet at n (c + 0.9) = 730 L (500
+// to 600 L), measured at S given: 3 layers 1,001 columns, 12: 4,500, 32: 12,600, 33: 9,000, 56: 14,200, 80:
+// 15,100, 128: 19,000; in a synthesis: 12 layers 3,800, 24: 6,500, 56: 9,600, 80 and 128: 10,000 to 17,000.
+inline bool rt_by_warp(int64_t nwl, int L, bool source_given) {
+    return nwl * (10 * ((L + 31) / 32) + 9) <= (source_given ? 7300 : 5000) * int64_t(L);
+}
 constexpr int RT_WARPS = 4;
 __global__ void __launch_bounds__(32 * RT_WARPS) rt_warp_kernel(RtArgs a) {
     extern __shared__ double s_rt[];
