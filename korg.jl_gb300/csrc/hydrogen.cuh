@@ -399,11 +399,13 @@ struct HTileArgs {
 };
 
 // A block takes TW wavelengths; its thread groups and the grid's second dimension share the layers
-// (layer l = slice + slices k).  Long grids: 128 wavelengths x 4 groups (64 x 8 above 64 layers: at 56
-// layers the same time in the infrared, a fifth more in the optical).  Short grids (at most HT_SHORT
-// wavelengths): 32 x 4 and two blocks in y, so that they reach all SMs.  In the infrared the
-// Brackett interpolation's FP64 operations bound it, elsewhere latency.  100,001 points of the H band:
-// 809 -> 740 us; 2,001 points at 5100 A: 139 -> 81 us.
+// (layer l = slice + slices k).  Long grids: 128 wavelengths x 4 groups up to 64 layers; above, 64 x 8 in FP64,
+// and in mixed precision 64 x as many groups as 16 layers a thread ask for: 200,001 points and 80 layers 1.55 ms
+// in the optical and 2.33 in the infrared, with 8 groups 1.87 and 2.77 (their registers hold 16 layers whether
+// used or not); 96 layers 2.70 and 3.49 (2.63 and 3.46).  Short grids (at most HT_SHORT wavelengths): 32 x 4 and two
+// blocks in y, so that they reach all SMs (56 layers, 32,001 points: 357 us, long form from 33,001: 375 us; 72
+// layers 437 and 501).  In the infrared the Brackett interpolation's FP64 operations bound it, elsewhere
+// latency.  100,001 points of the H band: 809 -> 740 us; 2,001 points at 5100 A: 139 -> 81 us.
 constexpr int64_t HT_SHORT = 32768;
 template <bool MIXED, int KMAX>
 __global__ void __launch_bounds__(512, (MIXED && KMAX <= 16) ? 2 : 1) hline_tile_kernel(HTileArgs a) {

@@ -573,7 +573,8 @@ int run_hydrogen(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, c
     if (L > 256) return set_err(ctx, KORG_EINVAL, "at most 256 layers are supported (got %d)", L);
     // layer slices (slice g owns layers g, g + slices, ...): thread groups of a block x blocks in y
     const bool shrt = nwl <= HT_SHORT;
-    const int TW = shrt ? 32 : (L <= 64 ? 128 : 64), groups = shrt || L <= 64 ? 4 : 8, gy = shrt ? 2 : 1;
+    const int TW = shrt ? 32 : (L <= 64 ? 128 : 64), gy = shrt ? 2 : 1;
+    const int groups = shrt || L <= 64 ? 4 : (mixed && L <= 128 ? (L + 15) / 16 : 8);
     const int kmax = (L + groups * gy - 1) / (groups * gy);  // layers per thread
     HOut ho;
     if (prep) ho = *prep;
