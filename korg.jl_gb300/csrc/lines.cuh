@@ -509,10 +509,13 @@ __global__ void __launch_bounds__(32 * PREP_WARPS) line_prep_mixed_kernel(LinesD
     }
 }
 
-// Launch geometry of the prologue kernels.  Up to about two warps per SM the FP64 work of a short list
+// Launch geometry of the prologue kernels.  Up to about two warps per SM (of 152) the FP64 work of a short list
 // is spread thin: fewer lines per warp (mixed), then fewer warps per block.  300 lines, mixed: 196 -> 55 us; lists
-// of 10,000 lines and more launch as before.
+// of 10,000 lines and more launch as before.  In FP64 a line is a warp: up to 16 warps per SM (2,432 lines) in
+// blocks of their own, which spread evenly, above in blocks of 8.  56 layers, 1,000 / 2,000 / 2,300 lines: 66 / 100
+// / 109 us; blocks of 8: 70 / 110 / 110, of as many as keep two blocks per SM (3 / 6 / 7): 74 / 119 / 166.
 constexpr int64_t PREP_SPREAD_WARPS = 304;
+constexpr int64_t PREP64_SPREAD = 16 * 152;
 inline int prep_block_warps(int64_t warps) {
     return int(std::min<int64_t>(std::max<int64_t>(warps / PREP_SPREAD_WARPS, 1), PREP_WARPS));
 }
@@ -524,7 +527,7 @@ inline PrepGeom prep_geom(int64_t n, bool mixed) {
     PrepGeom g{mixed ? 4 : 1, 1, 0};
     while (mixed && g.lpw < 32 && n > g.lpw * PREP_SPREAD_WARPS) g.lpw *= 2;
     const int64_t w = (n + g.lpw - 1) / g.lpw;
-    g.warps = prep_block_warps(w);
+    g.warps = mixed ? prep_block_warps(w) : (w <= PREP64_SPREAD ? 1 : PREP_WARPS);
     g.blocks = unsigned((w + g.warps - 1) / g.warps);
     return g;
 }
