@@ -299,7 +299,7 @@ TileArgs make_tile_args(const korg_ctx* ctx, const LineScratch& sc, double* alph
     ta.tier_ci = sc.tier_ci;
     ta.tier_start = sc.tier_meta;                 // [start: NTIER+1][unsorted][block counts]
     ta.unsorted = sc.tier_meta + NTIER + 1;
-    ta.far32 = FAR_NODES;
+    ta.far32 = 1;
     return ta;
 }
 
@@ -433,7 +433,7 @@ int dispatch_tile(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g
 // nlines: lines of the (largest) list.
 int run_tiles(korg_ctx* ctx, const TileArgs& ta, int kmax, const TileGeom& g, const TileQueue* q, bool mixed,
               int64_t nlines, cudaStream_t s) {
-    const bool far_lines = nlines >= FAR_MIN_CAND32 && (q || ta.far32 == FAR_NODES);
+    const bool far_lines = nlines >= FAR_MIN_CAND32 && (q || ta.far32);
     return mixed ? dispatch_tile<true>(ctx, ta, kmax, g, q, far_lines, s)
                  : dispatch_tile<false>(ctx, ta, kmax, g, q, far_lines, s);
 }
@@ -486,7 +486,7 @@ bool worth_tuning(int64_t nwl, int64_t nlines) { return nwl >= 100000 && nlines 
 
 int run_line_absorption(korg_ctx* ctx, double* alpha, const double* wls, int64_t nwl, const LinesDev& ln,
                         const LayersDev& lay, const CntmDev& cn, double cutoff, bool mixed,
-                        cudaStream_t s, int far32 = FAR_NODES) {
+                        cudaStream_t s, bool far32 = true) {
     if (ln.n == 0) return KORG_OK;  // src/line_absorption.jl:35-37
     const int L = lay.L;
     int kmax = 0;
@@ -935,7 +935,7 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         KCHECK(run_ref_lines(ctx, aref, ref_wl_dev, ln5, lay, cref, in->cutoff_threshold, s));
         if (in->hydrogen_lines)
             KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s));
-        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s, FAR_DIRECT));
+        KCHECK(run_line_absorption(ctx, alpha, wls, nwl, ln, lay, cn, in->cutoff_threshold, mixed, s, false));
     }
     // the metal-line prologue: the batch's for this spectrum, else the context's line scratch (read
     // after step 1, which may have grown it)
@@ -951,14 +951,13 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         LineScratch sc;
         line_scratch(line_base, ln.n, L, Lp, G, mixed, &sc);
         TileArgs ta = make_tile_args(ctx, sc, alpha, wls, nwl, ln, L, Lp, G);
-        ta.far32 = FAR_REDO;
         TileCfg cfg = tile_cfg(ctx, L, mixed);
         cfg.tw = op ? ctx->b_last_tw : ctx->last_tw;
         TileGeom g;
         if (!tile_geom(mixed, Lp, G, cfg, &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
         const TileMarks marks{on, g.tw};
         const int64_t tiles = (nwl + g.tw - 1) / g.tw;
-        dense_tiles_kernel<<<unsigned((tiles + 127) / 128), 128, 0, s>>>(ta, g.tw, on);
+        far_tiles_kernel<<<unsigned((tiles + 127) / 128), 128, 0, s>>>(ta, g.tw, on);
         KCUDA(cudaGetLastError());
         alpha_init_kernel<<<unsigned((nwl + 63) / 64), 256, 0, s>>>(alpha, wls, nwl, L, cn, marks);
         KCUDA(cudaGetLastError());
@@ -967,6 +966,8 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
             have_prep = true;
             KCHECK(run_hydrogen(ctx, alpha, wls, nwl, hl, in->hydrogen_window, in->use_MHD, mixed, s, &ho, marks));
         }
+        ta.far32 = 0;
+        ta.on = on;
         KCHECK(run_tiles(ctx, ta, kmax, g, nullptr, mixed, ln.n, s));
     }
     record(ctx, 9, s);
@@ -3073,7 +3074,7 @@ extern "C" KORG_API int korg_line_absorption_noalloc(double* alpha, const double
     ta.tier_ci = tl.ci;
     ta.tier_start = tl.start;
     ta.unsorted = tl.unsorted;
-    ta.far32 = FAR_NODES;
+    ta.far32 = 1;
     ta.math = math;
     return noalloc_tiles(ta, G, kmax, mixed, s);
 }

@@ -634,10 +634,6 @@ __global__ void __launch_bounds__(PART_THREADS) tier_scatter_kernel(const int32_
     }
 }
 
-// TileArgs::far32.  FAR_NODES: line_far_kernel takes them (the forward).  FAR_DIRECT: they are evaluated at
-// every wavelength like the others.  FAR_REDO: the same, and tiles with fewer candidates are left alone.
-enum { FAR_DIRECT = 0, FAR_NODES = 1, FAR_REDO = 2 };
-
 // Wavelengths that a pass is limited to: those of the marked tiles (tw wavelengths each, a multiple of 32),
 // or all of them where there are no marks.
 struct TileMarks {
@@ -660,7 +656,8 @@ struct TileArgs {
     const uint32_t* amask;
     const int32_t *lb, *ub;
     const int32_t *tier_idx, *tier_ci, *tier_start, *unsorted;
-    int32_t far32;            // mixed: what becomes of the far lines of tiles with FAR_MIN_CAND32 candidates
+    int32_t far32;            // mixed: line_far_kernel takes the far lines of dense tiles, else they are as the others
+    const unsigned char* on;  // tiles to evaluate (line_tile_kernel), or null: all
     const float4* params_w;   // mixed, or null: wing cubics (see PrepOut)
     const float* xcub;        // mixed, or null: cubic boundaries (see PrepOut)
     const MathTables* math;   // FP64: tables of the table-driven exp
@@ -1038,10 +1035,10 @@ struct LineStage32 {
 };
 static_assert(sizeof(LineStage32) == 32, "LineStage32 is two 16-byte loads");
 
-// Whether a mixed tile is dense enough for line_far_kernel (see FAR_MIN_CAND32).  Not with an unsorted list:
+// Whether the mixed tile's far lines go to line_far_kernel (see FAR_MIN_CAND32).  Not with an unsorted list:
 // its runs are whole tiers, whose length says nothing about the tile.
-__device__ __forceinline__ bool dense_tile32(const TileArgs& a, const int64_t (&run)[NTIER][2], int64_t npoints) {
-    if (*a.unsorted || npoints < FAR_MIN_POINTS) return false;
+__device__ __forceinline__ bool far_tile32(const TileArgs& a, const int64_t (&run)[NTIER][2], int64_t npoints) {
+    if (!a.far32 || *a.unsorted || npoints < FAR_MIN_POINTS) return false;
     int64_t n = 0;
     for (int t = 0; t < NTIER; t++) n += max(run[t][1] - run[t][0], int64_t(0));
     return n >= FAR_MIN_CAND32;
@@ -1084,7 +1081,7 @@ __device__ __forceinline__ void line_far_body(const TileArgs& a, int64_t tile, i
     const float span32 = float(span);
     if (tid < NTIER) tier_run(a, tid, j0, jlast, sh.tier[tid]);
     __syncthreads();
-    if (a.far32 != FAR_NODES || !dense_tile32(a, sh.tier, jlast - j0 + 1)) return;  // uniform
+    if (!far_tile32(a, sh.tier, jlast - j0 + 1)) return;  // uniform
     const float kspan = FAR_KAPPA32 * span32;
     for (int e = tid; e < FAR_WARPS * FAR_P * K; e += FAR_THREADS) (&sh.node[0][0][0])[e] = 0.0;
     __syncthreads();
@@ -1223,14 +1220,14 @@ __global__ void __launch_bounds__(FAR_THREADS) line_far_kernel(TileArgs a, int t
     line_far_body<K>(a, blockIdx.x, tw, int(blockIdx.y), sh);
 }
 
-// on[t] = whether tile t (tw wavelengths) is dense, one thread per tile.
-__global__ void dense_tiles_kernel(TileArgs a, int tw, unsigned char* on) {
+// on[t] = whether line_far_kernel takes lines of tile t (tw wavelengths), one thread per tile.
+__global__ void far_tiles_kernel(TileArgs a, int tw, unsigned char* on) {
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, j0 = t * tw;
     if (j0 >= a.nwl) return;
     const int64_t jlast = min(j0 + tw, a.nwl) - 1;
     int64_t run[NTIER][2];
     for (int k = 0; k < NTIER; k++) tier_run(a, k, j0, jlast, run[k]);
-    on[t] = dense_tile32(a, run, jlast - j0 + 1);
+    on[t] = far_tile32(a, run, jlast - j0 + 1);
 }
 
 // Mixed-precision tile: TW = blockDim.x wavelengths x the K layers of group g.  Thread t owns
@@ -1269,9 +1266,7 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
     if (tid < NTIER) tier_run(a, tid, j0, jlast, s_tier[tid]);  // candidate runs of the width tiers
     __syncthreads();
 
-    const bool dense = a.far32 != FAR_DIRECT && dense_tile32(a, s_tier, jlast - j0 + 1);
-    if (a.far32 == FAR_REDO && !dense) return;  // uniform
-    const float kspan = a.far32 == FAR_NODES && dense ? FAR_KAPPA32 * span32 : INFINITY;
+    const float kspan = far_tile32(a, s_tier, jlast - j0 + 1) ? FAR_KAPPA32 * span32 : INFINITY;
     // accumulators of layer pairs (packed FP32 arithmetic on the wing cubics)
     constexpr int KP = K / 2, QB = wing_quads(K);
     float acc[K], comp[K];
@@ -1430,6 +1425,7 @@ __device__ __forceinline__ void line_tile_body_mixed(const TileArgs& a, int64_t 
 template <bool MIXED, int K, int MAXT, int MINB, int SUB = 1>
 __global__ void __launch_bounds__(MAXT, MINB) line_tile_kernel(TileArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (MIXED && a.on && !a.on[blockIdx.x]) return;
     if constexpr (MIXED)
         line_tile_body_mixed<K>(a, blockIdx.x, int(blockIdx.y), smem);
     else
