@@ -636,7 +636,8 @@ __global__ void __launch_bounds__(32 * RAY_WARPS) rt_rays_kernel(RtGenArgs a) {
             const double d = (ib + ibp) * s_hd[k];
             const double m = (S - Sp) * recip64(a.I_scheme == 1 && d == 0 ? 1.0 : d);
             const double e = fexp64(-d, s_math);
-            if (open) Iout = fma(T, fma(-e, S + m, Sp + m), Iout);
+            const double with = fma(T, fma(-e, S + m, Sp + m), Iout);
+            Iout = open ? with : Iout;
             if (inward) Iin = fma(e, Iin - (Sp - m), S - m);
             T *= e;
             open = open && T >= RAY_STOP;
