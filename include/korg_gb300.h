@@ -18,8 +18,10 @@
  *   - `_dev` calls take device pointers (including the arrays inside the structs) and a
  *     CUDA stream, enqueue the work and return without synchronising.
  *
- * Precision: KORG_FP64 evaluates everything in FP64 (the plain form).  KORG_MIXED evaluates
- * line profiles in FP32 with Kahan-compensated accumulation, and keeps FP64 for the
+ * Precision: KORG_FP64 evaluates everything in FP64 (the plain form; lines far from a tile of
+ * wavelengths at 16 Chebyshev nodes of it, to FP64 rounding).  KORG_MIXED evaluates
+ * line profiles in FP32 with Kahan-compensated accumulation (in tiles of 8,192 candidate lines
+ * and more the far ones at nodes, at most 64 lines added in FP32, then FP64), and keeps FP64 for the
  * wavelength offsets from line centres (rounded to FP32 afterwards), the per-layer line
  * strengths (Boltzmann factors, n/U), the reference-wavelength line opacity (one wavelength,
  * which anchors the optical depths), the optical-depth integration and the formal solution.

@@ -2958,8 +2958,9 @@ int noalloc_setup(unsigned char** out) {
     return KORG_OK;
 }
 
-// The context's default tile shape and the same kernel instances as korg_line_absorption_dev,
-// so results are bitwise equal.  (No context: the tile kernel is launched directly.)
+// The context's default tile width and evaluations as korg_line_absorption_dev, so results are bitwise equal
+// (that call may take parts of layer groups per CTA on short FP64 grids, of the same bits).  No context: the
+// tile kernel is launched directly.
 int noalloc_tiles(const TileArgs& ta, int G, int kmax, bool mixed, cudaStream_t s) {
     TileGeom g;
     if (!tile_geom(mixed, ta.Lp, G, default_tile(mixed), &g)) return KORG_EINVAL;

@@ -766,8 +766,9 @@ constexpr double FAR_KAPPA64 = 2.5;
 constexpr int FAR_MIN_POINTS = 64;  // shorter tiles: 16 nodes would save less than 3 of 4 evaluations
 // Mixed tiles with fewer candidates evaluate every line at every wavelength: there a few lines carry
 // the far opacity, and the FP32 rounding of their evaluations (1e-7 each, averaged differently at the
-// nodes) would move the flux by up to 6e-9 of itself (7e-11 and less above the limit), for a gain of
-// a tenth (full optical synthesis, 4,000 candidates a tile) or none (sparser lists).
+// nodes) would move the flux by up to 6e-9 of itself (above the limit by 2e-9 at single wavelengths and
+// 2e-11 in the norm, measured on a cool giant), for a gain of a tenth (full optical synthesis, 4,000
+// candidates a tile) or none (sparser lists).
 constexpr int64_t FAR_MIN_CAND32 = 8192;
 
 // cos(pi i / 32), i = 0..16; the other angles by symmetry

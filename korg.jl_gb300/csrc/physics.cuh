@@ -152,7 +152,8 @@ __device__ __forceinline__ double voigt64(double a, double v) {
 // of them, and one reciprocal instead of two quotients in the far-Lorentz branch.  line_absorption! of 2,000
 // lines x 10,001 wavelengths: error against 64 bits 5.4e-16 as before, 4.80 -> 4.52 ms; the cross
 // section table of 1,000 molecular lines (11 x 51 x 10,001) 83.9 -> 77.2 ms.
-// Every rounding is written out (fma, __dmul_rn, __dadd_rn): tiles of other shapes give the same bits.
+// Every rounding is written out (fma, __dmul_rn, __dadd_rn): tiles of the same width give the same bits in every
+// other respect of their shape.
 __device__ __forceinline__ void harris64t(double v, double v2, double& H0, double& H1, double& H2, const double* exp2j) {
     H0 = fexp64(-v2, exp2j);
     if (v < 1.3)

@@ -2,9 +2,9 @@
 // Restates RadiativeTransfer.jl:62-139 for the default planar path (tau_scheme "anchored",
 // I_scheme "linear_flux_only" -> "linear_flux_only_expint", mu = [1], weights = [1]).
 //
-// One thread per wavelength column (on short grids a warp, lanes over layers); the layer recursion (the
-// tau prefix integral of :244-253 and the segment sum of :379-388) is sequential per column and
-// entirely FP64.  E2(tau) and exp(-tau) are evaluated once per layer and shared by the two segments
+// One thread per wavelength column (a warp, lanes over layers, on grids short for their layers:
+// rt_by_warp); the layer recursion (the tau prefix integral of :244-253 and the segment sum of
+// :379-388) is sequential per column and entirely FP64.  E2(tau) and exp(-tau) are evaluated once per layer and shared by the two segments
 // meeting there.  When a continuum interpolant is given, the continuum-only transfer of synthesize
 // (src/synthesize.jl:287-291) runs once per continuum knot interval where its flux is a series in
 // wavelength there, else in the same loop.
