@@ -954,7 +954,10 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         TileCfg cfg = tile_cfg(ctx, L, mixed);
         cfg.tw = op ? ctx->b_last_tw : ctx->last_tw;
         TileGeom g;
-        if (!tile_geom(mixed, Lp, G, cfg, &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
+        if (!tile_geom(mixed, Lp, G, cfg, &g)) {  // a batch size set since then, for another width
+            cfg.stage = 0;
+            if (!tile_geom(mixed, Lp, G, cfg, &g)) return set_err(ctx, KORG_EINVAL, "bad tile shape");
+        }
         const TileMarks marks{on, g.tw};
         const int64_t tiles = (nwl + g.tw - 1) / g.tw;
         far_tiles_kernel<<<unsigned((tiles + 127) / 128), 128, 0, s>>>(ta, g.tw, on);

@@ -119,3 +119,23 @@ def test_gradient_reusing_a_dense_forward(gpu_lib, hydrogen, tw):
         for k in want:
             np.testing.assert_allclose(got[k], want[k], rtol=1e-9, atol=1e-14 * np.max(np.abs(want[k])) + 1e-300)
     ctx.close()
+
+
+def test_reuse_after_a_batch_size_that_only_the_new_width_takes(gpu_lib):
+    """Forward at 256 wavelengths a tile, then a shape of 64 whose batches of 510 lines would not fit 256: the
+    reuse goes by the forward's width and the default batches, as the forward did."""
+    from korg_gb300.api import synthesize_prepared, synthesize_vjp
+    ctx = gpu_lib.Context(0)
+    inp = _inputs(56, 5000, 5010, 12000)
+    inp.hydrogen_lines = False
+    shape = lambda *s: ctx.check(ctx.lib.korg_set_tile_config(ctx.h, 56, gpu_lib.KORG_MIXED, *s))
+    shape(256, 0, 1)
+    dF = np.random.default_rng(1).standard_normal(len(inp.wls))
+    want = synthesize_vjp(inp, dF, precision="mixed", ctx=ctx)
+    synthesize_prepared(inp, precision="mixed", ctx=ctx)
+    assert ctx.lib.korg_set_tile_config(ctx.h, 56, gpu_lib.KORG_MIXED, 256, 510, 1) == 1
+    shape(64, 510, 1)
+    got = synthesize_vjp(inp, dF, precision="mixed", reuse_forward=True, ctx=ctx)
+    ctx.close()
+    for k in want:
+        np.testing.assert_allclose(got[k], want[k], rtol=1e-9, atol=1e-14 * np.max(np.abs(want[k])) + 1e-300)
