@@ -313,10 +313,12 @@ int prep_lines(korg_ctx* ctx, const LineScratch& sc, const double* wls, int64_t 
     PrepOut po{sc.params, sc.lb, sc.ub, sc.ci, sc.xfar, sc.amask, Lp, kmax, G, ctr, ctr + 1, sc.params_w, sc.xcub};
     const PrepGeom pg = prep_geom(ln.n, mixed);
     auto* math = static_cast<MathTables*>(ctx->math.p);
-    if (mixed)
+    if (mixed) {
+        // (26 KB of tables and lines of its own: 8 warps of more than 224 padded layers go above 48 KB)
+        if (Lp > 224) KCUDA(allow_smem(line_prep_mixed_kernel));
         line_prep_mixed_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, true), s>>>(
             ln, lay, sc.lc, cn, wls, nwl, cutoff, po, math, pg.lpw);
-    else
+    } else
         line_prep64_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, false), s>>>(ln, lay, sc.lc, cn, wls, nwl,
                                                                                       cutoff, po, math);
     KCUDA(cudaGetLastError());
