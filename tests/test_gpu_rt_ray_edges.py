@@ -91,3 +91,43 @@ def test_columns_do_not_depend_on_each_other(gpu_lib, inward):
     F, I = _rays(gpu_lib, alpha, S, 7e10 + z, True, tau, ref, MU[9], inward, 0)
     F1, I1 = _rays(gpu_lib, alpha[7:8], S[7:8], 7e10 + z, True, tau, ref, MU[9], inward, 0)
     assert F[7] == F1[0] and np.array_equal(I[:, 7], I1[:, 0])
+
+
+def _long_double(alpha, S, z, shell, tau, ref, mu, inward, scheme):
+    """Surface intensities by the same formulas in extended precision (RadiativeTransfer.jl:92-139, 244-324)."""
+    LD, out = np.longdouble, []
+    for u in mu:
+        n, ds = len(z), np.full(len(z), 1 / u)
+        if shell:
+            b = z[0] * np.sqrt(1 - u * u)
+            if b >= z[-1]:
+                n = int(np.argmin(np.abs(z - b)))
+                n = n if z[n] < b else n + 1
+            ds = z[:n] / np.sqrt(z[:n] ** 2 - b * b)
+        ib = alpha[:, :n].astype(LD) * (tau[:n] / ref[:n] * ds).astype(LD)
+        d = LD(0.5) * (ib[:, 1:] + ib[:, :-1]) * np.diff(np.log(tau[:n])).astype(LD)
+        e, Sx = np.exp(-d), S[:, :n].astype(LD)
+        m = np.diff(Sx, axis=1) / d
+        T, up, down = np.ones(len(S), LD), np.zeros(len(S), LD), np.zeros(len(S), LD)
+        for k in range(n - 1):
+            up += T * (Sx[:, k] + m[:, k] - e[:, k] * (Sx[:, k + 1] + m[:, k]))
+            down = e[:, k] * down + Sx[:, k + 1] - m[:, k] - e[:, k] * (Sx[:, k] - m[:, k])
+            T = T * e[:, k]
+        out.append(up + T * down if inward or n < len(z) else up)
+    return np.array(out, np.float64)
+
+
+@pytest.mark.parametrize("seed", range(8))
+@pytest.mark.parametrize("shell", [False, True])
+@pytest.mark.parametrize("scheme", [0, 1])
+def test_intensities_where_slopes_cancel(gpu_lib, seed, shell, scheme):
+    """Thin segments with source slopes of 1e6 and more, and rays through a shell that leave on the other side:
+    each ray's intensity to 1e-9 of an evaluation in extended precision, as the schemes' own comparison asks."""
+    L = (20, 56, 100)[seed % 3]
+    alpha, S, z, tau, ref = _atmosphere(L, 32, seed)
+    mu, w = np.polynomial.legendre.leggauss(8)
+    mu, w = mu / 2 + 0.5, w / 2
+    z = z + 7e10 * shell
+    inward = bool(seed % 2)
+    _, I = _rays(gpu_lib, alpha, S, z, shell, tau, ref, (mu, w), inward, scheme)
+    np.testing.assert_allclose(I, _long_double(alpha, S, z, shell, tau, ref, mu, inward, scheme), rtol=1e-9, atol=0)
