@@ -186,12 +186,14 @@ int reset_counters(korg_ctx* ctx, cudaStream_t s) {
     return KORG_OK;
 }
 
-// Lets `kern` take all the dynamic shared memory that an SM gives a block, whatever this call needs: the
-// attribute belongs to the process, and set to one call's size, a smaller call of another context's thread
-// in between would have the launch refused.
-constexpr size_t SMEM_BLOCK = 227 * 1024;
+// Lets `kern` be launched with `bytes` of dynamic shared memory: all that an SM gives a block, whatever this
+// call needs, as the attribute belongs to the process, and set to one call's size, a smaller call of another
+// context's thread in between would have the launch refused.  Up to 32 KB (beside at most 16 KB that a kernel
+// declares) need no attribute.
+constexpr size_t SMEM_BLOCK = 227 * 1024, SMEM_PLAIN = 32 * 1024;
 template <class... Args>
-cudaError_t allow_smem(void (*kern)(Args...)) {
+cudaError_t allow_smem(void (*kern)(Args...), size_t bytes) {
+    if (bytes <= SMEM_PLAIN) return cudaSuccess;
     cudaFuncAttributes fa;
     const cudaError_t e = cudaFuncGetAttributes(&fa, kern);
     if (e != cudaSuccess) return e;
@@ -315,7 +317,7 @@ int prep_lines(korg_ctx* ctx, const LineScratch& sc, const double* wls, int64_t 
     auto* math = static_cast<MathTables*>(ctx->math.p);
     if (mixed) {
         // (26 KB of tables and lines of its own: 8 warps of more than 224 padded layers go above 48 KB)
-        if (Lp > 224) KCUDA(allow_smem(line_prep_mixed_kernel));
+        if (Lp > 224) KCUDA(allow_smem(line_prep_mixed_kernel, SMEM_BLOCK));
         line_prep_mixed_kernel<<<pg.blocks, 32 * pg.warps, prep_smem(pg, Lp, true), s>>>(
             ln, lay, sc.lc, cn, wls, nwl, cutoff, po, math, pg.lpw);
     } else
@@ -387,7 +389,7 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
     if constexpr (SUB == 1) {  // (parts of groups are for short grids only, which no queue holds)
         if (q) {
             auto kern = line_tile_queue_kernel<MIXED, KMAX, MAXT, MINB>;
-            KCUDA(allow_smem(kern));
+            KCUDA(allow_smem(kern, g.smem));
             int per_sm = 0;
             KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, g.threads, g.smem));
             const int64_t grid = std::min<int64_t>(q->nitems, int64_t(ctx->sms) * std::max(per_sm, 1));
@@ -397,7 +399,7 @@ int launch_tile(korg_ctx* ctx, TileArgs ta, const TileGeom& g, const TileQueue* 
         }
     }
     auto kern = line_tile_kernel<MIXED, KMAX, MAXT, MINB, SUB>;
-    KCUDA(allow_smem(kern));
+    KCUDA(allow_smem(kern, g.smem));
     const int64_t tiles = (ta.nwl + g.tw - 1) / g.tw;
     kern<<<dim3(unsigned(tiles), g.split ? unsigned(g.G) * SUB : 1u), g.threads, g.smem, s>>>(ta);
     KCUDA(cudaGetLastError());
@@ -982,7 +984,7 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
                  dcntm, 1e-8, ctx->vjp_g.p, int32_t(mixed), dT, daref, gr.cntm_vals};
     {
         const size_t smem = size_t(RTA_WARPS) * RTA_ARRAYS * (L + 1) * sizeof(double);
-        KCUDA(allow_smem(rt_adjoint_kernel));
+        KCUDA(allow_smem(rt_adjoint_kernel, smem));
         const int64_t blocks = std::min<int64_t>((nwl + RTA_WARPS - 1) / RTA_WARPS, int64_t(ctx->sms) * 8);
         rt_adjoint_kernel<<<unsigned(blocks), 32 * RTA_WARPS, smem, s>>>(ra);
         KCUDA(cudaGetLastError());
@@ -1088,17 +1090,17 @@ int run_vjp(korg_ctx* ctx, const korg_synth_inputs* in, const LinesDev& ln, cons
         const size_t smem = adj_smem(sh, mixed);
         int per_sm = 0;
         if (mixed) {
-            KCUDA(allow_smem(line_adj_kernel<true>));
+            KCUDA(allow_smem(line_adj_kernel<true>, smem));
             KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_adj_kernel<true>, threads, smem));
             line_adj_kernel<true><<<ctx->sms * std::max(per_sm, 1), threads, smem, s>>>(la);
         } else {
-            KCUDA(allow_smem(line_adj_kernel<false>));
+            KCUDA(allow_smem(line_adj_kernel<false>, smem));
             KCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, line_adj_kernel<false>, threads, smem));
             line_adj_kernel<false><<<ctx->sms * std::max(per_sm, 1), threads, smem, s>>>(la);
         }
         KCUDA(cudaGetLastError());
         const size_t psmem = sizeof(double) * size_t(4 + S) * L;
-        KCUDA(allow_smem(line_adj_prologue_kernel));
+        KCUDA(allow_smem(line_adj_prologue_kernel, psmem));
         line_adj_prologue_kernel<<<unsigned((lns.n * 32 + 255) / 256), 256, psmem, s>>>(
             lns, lay, sc.lc, dpar, Lp, out, static_cast<MathTables*>(ctx->math.p));
         KCUDA(cudaGetLastError());
@@ -2140,7 +2142,7 @@ KORG_API int korg_radiative_transfer_general(korg_ctx* ctx, const double* alpha,
     for (int r = 0; r < n_in; r++) paired = paired && in_idx[r] == r;
     if (paired) {
         const size_t smem = rt_rays_smem(L, n_mu);
-        KCUDA(allow_smem(rt_rays_kernel));
+        KCUDA(allow_smem(rt_rays_kernel, smem));
         rt_rays_kernel<<<unsigned((nwl + 31) / 32), 32 * RAY_WARPS, smem, ctx->stream>>>(ra);
     } else {
         rt_general_kernel<<<unsigned((nwl + 127) / 128), 128, 0, ctx->stream>>>(ra);
@@ -2976,7 +2978,7 @@ int noalloc_tiles(const TileArgs& ta, int G, int kmax, bool mixed, cudaStream_t 
     t.G = G;
     const dim3 grid(unsigned((ta.nwl + g.tw - 1) / g.tw), unsigned(G));
     auto go = [&](auto kern) {
-        if (allow_smem(kern) != cudaSuccess)
+        if (allow_smem(kern, g.smem) != cudaSuccess)
             return KORG_ECUDA;
         kern<<<grid, g.threads, g.smem, s>>>(t);
         return cudaGetLastError() == cudaSuccess ? KORG_OK : KORG_ECUDA;
